@@ -181,18 +181,42 @@ __device__ __forceinline__ double div_sqrt2(double num, double d1, double d2)
 // FP32 here adds an error of the same order (~1e-7 in r), and this GPU's
 // FP64 pipe is narrow (FP64 arithmetic bounded the lag kernel).  The
 // flat-overlap guard d1 d2 < n^2 1e-9 is evaluated in FP32 too.
-__device__ __forceinline__ double r_int(const PairDev &p, long long n, float cs, long long s1,
-                                        long long q1, long long s2, long long q2)
+//
+// Nothing here touches a 64-bit floating-point or conversion instruction:
+// those run two lanes per clock and SM on this GPU, and the five 64-bit
+// integer to FP32 conversions, the FP64 result and its FP64 comparisons had
+// bounded the lag scan (971 of 1703 us for 48 pairs of 512^2 over all lags).
+__device__ __forceinline__ float u64_to_float(unsigned long long v)
+{
+    // the leading 32 bits with the rest folded into the last one round as v
+    // does; the scale is a power of two
+    const int s = __clzll((long long)v) & 63;   // (v = 0: 0, and the product is 0)
+    const unsigned long long t = v << s;
+    const unsigned top = (unsigned)(t >> 32) | ((unsigned)t != 0u);
+    return __uint2float_rn(top) * __uint_as_float((unsigned)(127 + 32 - s) << 23);
+}
+
+__device__ __forceinline__ float i64_to_float(long long v)
+{
+    const float f = u64_to_float((unsigned long long)(v < 0 ? -v : v));
+    return v < 0 ? -f : f;
+}
+
+// n: the overlap's pixels (a box of an FFT raster: < 2^26); m1, m2: the
+// integer mean shifts
+__device__ __forceinline__ float r_int(int n, float cs, long long s1, long long q1, long long s2,
+                                       long long q2, int m1, int m2)
 {
     typedef unsigned long long u64;
     const u64 un = (u64)n;
     const u64 d1 = un * (u64)q1 - (u64)s1 * (u64)s1, d2 = un * (u64)q2 - (u64)s2 * (u64)s2;
-    const float f1 = __ull2float_rn(d1), f2 = __ull2float_rn(d2), fn = __ll2float_rn(n);
+    const float f1 = u64_to_float(d1), f2 = u64_to_float(d2), fn = __int2float_rn(n);
     if (f1 * f2 < fn * fn * 1.0e-9f)
-        return 0.0;
-    const long long m1 = (long long)p.mu[0], m2 = (long long)p.mu[1];
-    const float num = fmaf(fn, cs, -(__ll2float_rn(s1 - n * m1) * __ll2float_rn(s2 - n * m2)));
-    return (double)(num * (rsqrtf(f1) * rsqrtf(f2)));
+        return 0.0f;
+    const float num = fmaf(fn, cs,
+                           -(i64_to_float(s1 - (long long)n * m1) *
+                             i64_to_float(s2 - (long long)n * m2)));
+    return num * (rsqrtf(f1) * rsqrtf(f2));
 }
 
 // the overlap sizes for which r_int is exact on this pair's pixel types
@@ -204,51 +228,102 @@ __device__ __forceinline__ bool r_int_ok(const PairDev &p, long long n)
     return u8 || n < (1ll << 20);
 }
 
-// cs: the cross sum at this lag (the inverse transform's value over Nx Ny)
-__device__ __forceinline__ bool lag_r(const PairDev &p, int x, int y, float cs, double &r)
+// The summed-area rows that the overlap boxes of one lag row read, per image:
+// row T of the box and, when the box starts above row 0, row B - 1 (element
+// offsets into the tables).  The same for every lag of the row, so a scan
+// over a row computes them once.
+struct LagRow {
+    int olh;           // box height
+    int oT[2], oB[2];  // oB < 0: the box starts at row 0
+};
+
+__device__ __forceinline__ LagRow lag_row(const PairDev &p, int y)
 {
-    const int w1 = p.w[0], h1 = p.h[0], w2 = p.w[1], h2 = p.h[1];
-    // BoxesFromShifts, 0_GEN/Geometry.cpp:150-176
-    int L2 = max(0, x), R2 = min(w2 - 1, x + w1 - 1);
-    int B2 = max(0, y), T2 = min(h2 - 1, y + h1 - 1);
-    R2 = max(R2, L2);
-    T2 = max(T2, B2);
-    const int L1 = L2 - x, R1 = R2 - x, B1 = B2 - y, T1 = T2 - y;
-    const int olw = R1 - L1 + 1, olh = T1 - B1 + 1;
-    r = 0.0;
+    LagRow q;
+    const int B2 = max(0, y), T2 = max(min(p.h[1] - 1, y + p.h[0] - 1), B2);
+    const int B[2] = {B2 - y, B2}, T[2] = {T2 - y, T2};
+    q.olh = T2 - B2 + 1;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        q.oT[i] = sat_slot(p, i, T[i]) * p.w[i];
+        q.oB[i] = B[i] > 0 ? sat_slot(p, i, B[i] - 1) * p.w[i] : -1;
+    }
+    return q;
+}
+
+// IntegralTable (0_GEN/Correlation.cpp:112-150) on a lag row's table rows,
+// columns L..R; int64 sums are exact, FP64 ones in the reference's order
+template <typename TA>
+__device__ __forceinline__ TA row_box(const TA *__restrict__ t, int oT, int oB, int L, int R)
+{
+    TA r = __ldg(t + oT + R);
+    if (L > 0)
+        r -= __ldg(t + oT + L - 1);
+    if (oB >= 0) {
+        r -= __ldg(t + oB + R);
+        if (L > 0)
+            r += __ldg(t + oB + L - 1);
+    }
+    return r;
+}
+
+// legality of lag (x, y) by box size and counts, q = lag_row(p, y); L2..R2:
+// the box's columns in image 2 (BoxesFromShifts, 0_GEN/Geometry.cpp:150-176)
+__device__ __forceinline__ bool lag_row_legal(const PairDev &p, const LagRow &q, int x, int &L2,
+                                              int &R2)
+{
+    L2 = max(0, x);
+    R2 = max(min(p.w[1] - 1, x + p.w[0] - 1), L2);
+    const int L1 = L2 - x, R1 = R2 - x;
+    const int olw = R1 - L1 + 1, olh = q.olh;
     // a transposed job evaluates LegalRgn on the caller's (untransposed) box
     if (p.rgn_kind != ALN_RGN_NONE &&
         !(p.transposed ? rgn_ok(p, olh, olw) : rgn_ok(p, olw, olh)))
         return false;
     if (p.cnt_kind == ALN_CNT_GT) {
-        const int c1 = sat_box_n(p.satN[0], p, 0, L1, R1, B1, T1);
-        const int c2 = sat_box_n(p.satN[1], p, 1, L2, R2, B2, T2);
+        const int c1 = row_box(p.satN[0], q.oT[0], q.oB[0], L1, R1);
+        const int c2 = row_box(p.satN[1], q.oT[1], q.oB[1], L2, R2);
         if (!(c1 > p.cnt_n && c2 > p.cnt_n))
             return false;
     }
+    return true;
+}
+
+// r of lag (x, y), q = lag_row(p, y); cs: the cross sum at this lag (the
+// inverse transform's value over Nx Ny)
+__device__ __forceinline__ bool lag_row_r(const PairDev &p, const LagRow &q, int x, float cs,
+                                          double &r)
+{
+    int L2, R2;
+    r = 0.0;
+    if (!lag_row_legal(p, q, x, L2, R2))
+        return false;
+    const int L1 = L2 - x, R1 = R2 - x;
+    const int olw = R1 - L1 + 1, olh = q.olh;
+    const long long *iS1 = (const long long *)p.satS[0], *iQ1 = (const long long *)p.satQ[0];
+    const long long *iS2 = (const long long *)p.satS[1], *iQ2 = (const long long *)p.satQ[1];
     if (r_int_ok(p, (long long)olw * olh)) {
-        r = r_int(p, (long long)olw * olh, cs,
-                 sat_box_i64((const long long *)p.satS[0], p, 0, L1, R1, B1, T1),
-                 sat_box_i64((const long long *)p.satQ[0], p, 0, L1, R1, B1, T1),
-                 sat_box_i64((const long long *)p.satS[1], p, 1, L2, R2, B2, T2),
-                 sat_box_i64((const long long *)p.satQ[1], p, 1, L2, R2, B2, T2));
+        r = (double)r_int(olw * olh, cs, row_box(iS1, q.oT[0], q.oB[0], L1, R1),
+                          row_box(iQ1, q.oT[0], q.oB[0], L1, R1),
+                          row_box(iS2, q.oT[1], q.oB[1], L2, R2),
+                          row_box(iQ2, q.oT[1], q.oB[1], L2, R2), (int)p.mu[0], (int)p.mu[1]);
         return true;
     }
     const double n = (double)(olw * olh);
     double s1, q1, s2, q2;
     if (p.sat_int & 1) {
-        s1 = (double)sat_box_i64((const long long *)p.satS[0], p, 0, L1, R1, B1, T1);
-        q1 = (double)sat_box_i64((const long long *)p.satQ[0], p, 0, L1, R1, B1, T1);
+        s1 = (double)row_box(iS1, q.oT[0], q.oB[0], L1, R1);
+        q1 = (double)row_box(iQ1, q.oT[0], q.oB[0], L1, R1);
     } else {
-        s1 = sat_box(p.satS[0], p, 0, L1, R1, B1, T1);
-        q1 = sat_box(p.satQ[0], p, 0, L1, R1, B1, T1);
+        s1 = row_box(p.satS[0], q.oT[0], q.oB[0], L1, R1);
+        q1 = row_box(p.satQ[0], q.oT[0], q.oB[0], L1, R1);
     }
     if (p.sat_int & 2) {
-        s2 = (double)sat_box_i64((const long long *)p.satS[1], p, 1, L2, R2, B2, T2);
-        q2 = (double)sat_box_i64((const long long *)p.satQ[1], p, 1, L2, R2, B2, T2);
+        s2 = (double)row_box(iS2, q.oT[1], q.oB[1], L2, R2);
+        q2 = (double)row_box(iQ2, q.oT[1], q.oB[1], L2, R2);
     } else {
-        s2 = sat_box(p.satS[1], p, 1, L2, R2, B2, T2);
-        q2 = sat_box(p.satQ[1], p, 1, L2, R2, B2, T2);
+        s2 = row_box(p.satS[1], q.oT[1], q.oB[1], L2, R2);
+        q2 = row_box(p.satQ[1], q.oT[1], q.oB[1], L2, R2);
     }
     const double num = n * (double)cs - (s1 - n * p.mu[0]) * (s2 - n * p.mu[1]);
     const double d1 = n * q1 - s1 * s1;
@@ -699,9 +774,22 @@ __global__ void k_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int CG)
 // lag rows: inverse real FFT, normalisation, legality, disc, row argmax
 // ---------------------------------------------------------------------------
 
+// A double as an integer that orders the same way (-0 as 0, NaN below
+// everything, so that it never wins): FP64 comparisons run two lanes per
+// clock and SM on this GPU.
+__device__ __forceinline__ long long ord_bits(double v)
+{
+    long long b = __double_as_longlong(v);
+    const unsigned long long mag = (unsigned long long)b << 1;
+    if (mag == 0 || mag > 0x7ff0000000000000ull << 1)
+        b = mag == 0 ? 0 : -1;   // (-1: the least value below)
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
 __device__ __forceinline__ void best_merge(double &r, long long &k, double r2, long long k2)
 {
-    if (r2 > r || (r2 == r && k2 < k)) {
+    const long long a = ord_bits(r), b = ord_bits(r2);
+    if (b > a || (b == a && k2 < k)) {
         r = r2;
         k = k2;
     }
@@ -745,6 +833,7 @@ __global__ void k_lagrow(PairDev *pairs, const float2 *__restrict__ tw, int RBL)
         const int xa = xr < 0 ? 1 : max(p.xlo, p.ox - xr);
         const int xb = xr < 0 ? 0 : min(p.xhi, p.ox + xr);
         const int ys = y < 0 ? y + Ny : y;
+        const LagRow lr = lag_row(p, y);
         double br = -1.0e30;
         long long bk = 0x7fffffffffffffffLL;
         const float *row = (const float *)(res + r * pitch);
@@ -752,7 +841,7 @@ __global__ void k_lagrow(PairDev *pairs, const float2 *__restrict__ tw, int RBL)
             double rv = 0.0;
             if (x >= xa && x <= xb) {
                 const int xs = x < 0 ? x + Nx : x;
-                if (lag_r(p, x, y, row[xs] * inv, rv))
+                if (lag_row_r(p, lr, x, row[xs] * inv, rv))
                     best_merge(br, bk, rv, (long long)ys * Nx + xs);
             }
             p.rr[(long long)j * Wx + (x - p.xlo)] = rv;
@@ -779,8 +868,10 @@ __global__ void k_lagrow(PairDev *pairs, const float2 *__restrict__ tw, int RBL)
 
 // value at FFT storage index (xs, ys) after the reference's lag loop:
 // r for a legal lag in the disc, 0 otherwise (dead zone, outside the disc,
-// illegal) -- the rslt array ParabPeakFFT reads.
-__device__ double stored_value(const PairDev &p, int xs, int ys)
+// illegal) -- the rslt array ParabPeakFFT reads.  raw: rr holds the window's
+// inverse-transform values (k2_lagrow), and r is computed from them as
+// k2_lagscan does; else rr holds r itself (k_lagrow).
+__device__ double stored_value(const PairDev &p, int xs, int ys, bool raw)
 {
     const int nnegx = p.w[0] - 1, nposx = p.w[1];
     const int nnegy = p.h[0] - 1, nposy = p.h[1];
@@ -800,14 +891,24 @@ __device__ double stored_value(const PairDev &p, int xs, int ys)
     if (x < p.xlo || x > p.xhi || y < p.ylo || y > p.yhi)
         return 0.0;
     const int Wx = p.xhi - p.xlo + 1;
-    return p.rr[(long long)(y - p.ylo) * Wx + (x - p.xlo)];
+    const long long o = (long long)(y - p.ylo) * Wx + (x - p.xlo);
+    if (!raw)
+        return p.rr[o];
+    const long long dx = x - p.ox, dy = y - p.oy;
+    double r = 0.0;
+    if (dx * dx + dy * dy <= p.rsqr)
+        lag_row_r(p, lag_row(p, y), x,
+                  ((const float *)p.rr)[o] * (1.0f / ((float)p.Nx * (float)p.Ny)), r);
+    return r;
 }
 
-// grid (npairs), block 256
-__global__ void k_final(PairDev *pairs, ResultDev *res, int nreal_x_is_one, int nreal_y_is_one)
+// grid (npairs), block 256; raw: see stored_value
+__global__ void k_final(PairDev *pairs, ResultDev *res, int nreal_x_is_one, int nreal_y_is_one,
+                        int raw)
 {
     __shared__ double red_r[32];
     __shared__ long long red_k[32];
+    __shared__ double near[4];
     PairDev &p = pairs[blockIdx.x];
     if (p.status != 0)
         return;
@@ -827,18 +928,23 @@ __global__ void k_final(PairDev *pairs, ResultDev *res, int nreal_x_is_one, int 
         red_k[wid] = bk;
     }
     __syncthreads();
-    if (threadIdx.x != 0)
+    if (threadIdx.x >= 4)
         return;
+    // four threads: each finds the peak and fetches one of its neighbours
+    br = red_r[0];
+    bk = red_k[0];
     for (int q = 1; q < (int)(blockDim.x >> 5); ++q)
         best_merge(br, bk, red_r[q], red_k[q]);
     ResultDev &o = res[blockIdx.x];
     if (br < -2.0) {
-        p.status = ALN_NO_PEAK;
-        p.r = p.dx = p.dy = 0.0;
-        p.px = p.py = 0;
-        o.r = o.dx = o.dy = 0.0;
-        o.status = ALN_NO_PEAK;
-        o.px = o.py = 0;
+        if (threadIdx.x == 0) {
+            p.status = ALN_NO_PEAK;
+            p.r = p.dx = p.dy = 0.0;
+            p.px = p.py = 0;
+            o.r = o.dx = o.dy = 0.0;
+            o.status = ALN_NO_PEAK;
+            o.px = o.py = 0;
+        }
         return;
     }
     const int Nx = p.Nx, Ny = p.Ny;
@@ -853,18 +959,24 @@ __global__ void k_final(PairDev *pairs, ResultDev *res, int nreal_x_is_one, int 
     // reference's, which may be larger than the transform grid).
     const int xs = bigx < 0 ? bigx + p.rnx : bigx, ys = bigy < 0 ? bigy + p.rny : bigy;
     const int nx = nreal_x_is_one ? 1 : p.rnx, ny = nreal_y_is_one ? 1 : p.rny;
-    double xpk = bigx, ypk = bigy;
     const int ix = bigx, iy = bigy;
+    const bool inx = ix - 1 >= 0 && ix + 1 < nx, iny = iy - 1 >= 0 && iy + 1 < ny;
+    const int way = (threadIdx.x & 1) ? 1 : -1;
+    if (threadIdx.x < 2 ? inx : iny)
+        near[threadIdx.x] = threadIdx.x < 2 ? stored_value(p, ix + way, ys, raw != 0)
+                                            : stored_value(p, xs, iy + way, raw != 0);
+    __syncwarp(0xf);
+    if (threadIdx.x != 0)
+        return;
+    double xpk = bigx, ypk = bigy;
     const double z1 = br;
     double z0, z2;
-    if (ix - 1 >= 0 && ix + 1 < nx && (z0 = stored_value(p, ix - 1, ys)) != 0.0 &&
-        (z2 = stored_value(p, ix + 1, ys)) != 0.0) {
+    if (inx && (z0 = near[0]) != 0.0 && (z2 = near[1]) != 0.0) {
         z0 = 1 * (z0 - z2) / (2 * (z0 + z2 - z1 - z1));
         if (fabs(z0) <= 8 * 1)
             xpk += z0;
     }
-    if (iy - 1 >= 0 && iy + 1 < ny && (z0 = stored_value(p, xs, iy - 1)) != 0.0 &&
-        (z2 = stored_value(p, xs, iy + 1)) != 0.0) {
+    if (iny && (z0 = near[2]) != 0.0 && (z2 = near[3]) != 0.0) {
         z0 = 1 * (z0 - z2) / (2 * (z0 + z2 - z1 - z1));
         if (fabs(z0) <= 8 * 1)
             ypk += z0;
@@ -2143,6 +2255,8 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
 #undef X
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "row length %d", L);
         }
+        LAUNCH(ctx, "k2_lagscan", k2_lagscan, dim3((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n),
+               32 * LAGSCAN_ROWS, 0, ctx->dpairs);
     } else if (mode == JOB_P2I) {
         switch (L) {
 #define X(v) case v: launch_lagp2i<v>(ctx, n, maxWy); break;
@@ -2294,7 +2408,8 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "column length %d", Ny);
         }
     }
-    if (L >= 8 && L <= 4096 && Ny >= 8 && Ny <= 8192) {
+    const bool reg_path = L >= 8 && L <= 4096 && Ny >= 8 && Ny <= 8192;
+    if (reg_path) {
         if (int rc = launch_fft_pipeline(ctx, L, Ny, n, cl.maxh, cl.maxWy, mode, cl.both != 0,
                                          cl.sonly != 0, cl.seg != 0))
             return rc;
@@ -2323,7 +2438,7 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
     }
     if (mode == JOB_PATCHES)
         LAUNCH(ctx, "k_final", k_final, n, 256, 0, ctx->dpairs, ctx->dres, cl.frame_nx1,
-               cl.frame_ny1);
+               cl.frame_ny1, (int)reg_path);
     else if (mode == JOB_P2I)
         LAUNCH(ctx, "k_final_p2i", k_final_p2i, n, 256, 0, ctx->dpairs, ctx->dres);
     else if (mode == JOB_IMAGES_F) {
@@ -3442,7 +3557,7 @@ extern "C" int aln_corr_patches_noalloc(const aln_image *a, const aln_image *b, 
         const size_t sm = 2 * (size_t)RBL * (L + 1) * sizeof(float2);
         k_lagrow<<<dim3((Wy + RBL - 1) / RBL, 1), 256, sm, st>>>(dpair, tw, RBL);
     }
-    k_final<<<1, 256, 0, st>>>(dpair, dres, pl.orig_nx == 1, pl.orig_ny == 1);
+    k_final<<<1, 256, 0, st>>>(dpair, dres, pl.orig_nx == 1, pl.orig_ny == 1, 0);
     CK(cudaGetLastError());
     ResultDev hr;
     CK(cudaMemcpyAsync(&hr, dres, sizeof hr, cudaMemcpyDeviceToHost, st));

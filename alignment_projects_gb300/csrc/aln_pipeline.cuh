@@ -13,7 +13,8 @@
 //   k2_corrseg<NS> the same with the column cut into segments of a's rows
 //             (CorrPatches): per segment two NS-point FFTs and the product,
 //             summed per column, one inverse
-//   k2_lagrow<L>   per lag row: inverse real FFT, r per lag, row argmax
+//   k2_lagrow<L>   per lag row: inverse real FFT -> the lag image
+//   k2_lagscan     per lag row: r per lag, row argmax
 //   k2_lagimg / k2_lagp2i, k_final_img / k_makef / k_fpeak / k_final_p2i:
 //             the CorrImages and CorrPatchToImage ends of the pipeline
 #pragma once
@@ -1003,15 +1004,12 @@ k2_lagrow(PairDev *pairs, const float2 *__restrict__ tw)
     using F = FFTOf<L, +1>;   // RegFFT, or MixFFT for L = 3 * 2^k, 5 * 2^k
     static_assert(F::SMEM <= lag_pitch<L>(), "the exchange buffer fits the team's row region");
     constexpr int V = F::V, T = F::T;
-    constexpr int PITCH = lag_pitch<L>();   // holds L+1 bins, then 2L reals
+    constexpr int PITCH = lag_pitch<L>();   // holds the L+1 bins
     extern __shared__ float2 smem[];
-    __shared__ double red_r[32];
-    __shared__ long long red_k[32];
-    __shared__ PairDev sp;
-    const PairDev &p = stage_job(pairs, blockIdx.y, sp);
+    const PairDev &p = pairs[blockIdx.y];
     if (p.status != 0)
         return;
-    const int Wy = p.yhi - p.ylo + 1, Wx = p.xhi - p.xlo + 1;
+    const int xlo = p.xlo, xhi = p.xhi, Wx = xhi - xlo + 1, Wy = p.yhi - p.ylo + 1;
     const int G = blockDim.x / T;
     const int team = threadIdx.x / T, t = threadIdx.x - team * T;
     const int j0 = blockIdx.x * G;
@@ -1020,7 +1018,6 @@ k2_lagrow(PairDev *pairs, const float2 *__restrict__ tw)
     const int j = j0 + team;
     const bool live = j < Wy;
     float2 *sm = smem + team * PITCH;
-    const int Nx = p.Nx, Ny = p.Ny;
     // spectrum bins of the CTA's lag rows
     load_lag_rows<L, T, lagrow_threads(T) / T>(smem, PITCH, p.Q, Wy, j0);
     __syncthreads();
@@ -1042,61 +1039,107 @@ k2_lagrow(PairDev *pairs, const float2 *__restrict__ tw)
     }
     // the teams' rows are their own from here on: team barriers only
     F::run_team(v, sm, t, tw, team);
-    __syncthreads();
-    float *C = (float *)sm;   // 2L reals, unpadded
+    if (!live)
+        return;
+    // storage index xs holds lag xs (xs <= xhi) or xs - Nx; the window's lags
+    // go to the row of the lag image
+    float *row = (float *)p.rr + (long long)j * Wx - xlo;
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-        const int n = F::out_idx(t, q);
-        C[2 * n] = v[q].x;
-        C[2 * n + 1] = v[q].y;
+        const int xs = 2 * F::out_idx(t, q);
+        const int xa = xs > xhi ? xs - 2 * L : xs, xb = xs + 1 > xhi ? xs + 1 - 2 * L : xs + 1;
+        if (xa >= xlo && xa <= xhi)
+            row[xa] = v[q].x;
+        if (xb >= xlo && xb <= xhi)
+            row[xb] = v[q].y;
     }
-    __syncthreads();
+}
+
+// r per lag and each lag row's best, from the lag image k2_lagrow wrote: one
+// warp per lag row, lanes on consecutive lags.  Apart from the transforms,
+// because a row's transform has few threads (8 for the 160- and 192-point
+// rows), and its lags then ran one after another on them: 16 per thread on
+// a 129-lag row, each a chain of table loads.  The row's table rows, box
+// height and disc span are set once per warp (LagRow); r itself is not
+// stored, k_final computes the four it needs again.  Transform and scan
+// together, before (one kernel) and now: one 235 x 2048 pair 45 -> 22 us, 3000
+// uneven pairs 7.3 -> 4.7 ms, 48 pairs of 512^2 over all lags 1120 -> 752 us.
+#define LAGSCAN_ROWS 8
+
+// grid (ceil(max Wy / LAGSCAN_ROWS), npairs), block 32 * LAGSCAN_ROWS
+__global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
+{
+    const PairDev &p = pairs[blockIdx.y];
+    if (p.status != 0)
+        return;
+    const int j = blockIdx.x * LAGSCAN_ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (j >= p.yhi - p.ylo + 1)
+        return;
+    const int Nx = p.Nx, Ny = p.Ny;
+    const int y = p.ylo + j, ox = p.ox;
+    const long long dy = y - p.oy, in = p.rsqr - dy * dy;   // disc: dx^2 <= in
+    // the row's span of the disc, a little wide; the lag's own test is exact
+    // (an FP64 square root per row cost more than the test)
+    const int xr = in < 0 ? -1 : (int)sqrtf(__uint2float_rn((unsigned)min(in, 1ll << 30))) + 2;
+    const int xa = max(p.xlo, ox - xr), xb = xr < 0 ? xa - 1 : min(p.xhi, ox + xr);
+    const float *__restrict__ row =
+        (const float *)p.rr + (long long)j * (p.xhi - p.xlo + 1) - p.xlo;
     // 1 / (Nx Ny): exact for power-of-two grids; on the split lengths one
     // more FP32 rounding, below the transform's own error
     const float invf = 1.0f / ((float)Nx * (float)Ny);
-    double br = -1.0e30;
-    long long bk = 0x7fffffffffffffffLL;
-    if (live) {
-        const int y = p.ylo + j;
-        const long long dy = y - p.oy;
-        const int xr = isqrt_ll(p.rsqr - dy * dy);
-        const int xa = xr < 0 ? 1 : max(p.xlo, p.ox - xr);
-        const int xb = xr < 0 ? 0 : min(p.xhi, p.ox + xr);
-        const int ys = y < 0 ? y + Ny : y;
-        for (int x = p.xlo + t; x <= p.xhi; x += T) {
-            double rv = 0.0;
-            if (x >= xa && x <= xb) {
-                const int xs = x < 0 ? x + Nx : x;
-                if (lag_r(p, x, y, C[xs] * invf, rv))
-                    best_merge(br, bk, rv, (long long)ys * Nx + xs);
+    const LagRow q = lag_row(p, y);
+    const int key0 = (y < 0 ? y + Ny : y) * Nx;   // storage indices are < 2^26
+    if (r_int_ok(p, (long long)min(p.w[0], p.w[1]) * q.olh)) {
+        // every lag of the row takes r_int: FP32 keys
+        const long long *S1 = (const long long *)p.satS[0], *Q1 = (const long long *)p.satQ[0];
+        const long long *S2 = (const long long *)p.satS[1], *Q2 = (const long long *)p.satQ[1];
+        const int m1 = (int)p.mu[0], m2 = (int)p.mu[1];
+        float br = -1.0e30f;
+        int bk = 0x7fffffff;
+        for (int x = xa + lane; x <= xb; x += 32) {
+            const long long dx = x - ox;
+            int L2, R2;
+            if (dx * dx > in || !lag_row_legal(p, q, x, L2, R2))
+                continue;
+            const float r = r_int((R2 - L2 + 1) * q.olh, __ldg(row + x) * invf,
+                                  row_box(S1, q.oT[0], q.oB[0], L2 - x, R2 - x),
+                                  row_box(Q1, q.oT[0], q.oB[0], L2 - x, R2 - x),
+                                  row_box(S2, q.oT[1], q.oB[1], L2, R2),
+                                  row_box(Q2, q.oT[1], q.oB[1], L2, R2), m1, m2);
+            const int k = key0 + (x < 0 ? x + Nx : x);
+            if (r > br || (r == br && k < bk)) {
+                br = r;
+                bk = k;
             }
-            p.rr[(long long)j * Wx + (x - p.xlo)] = rv;
         }
-    }
-    // team reduction
-    for (int o = 16; o > 0; o >>= 1) {
-        const double r2 = __shfl_down_sync(0xffffffff, br, o);
-        const long long k2 = __shfl_down_sync(0xffffffff, bk, o);
-        if ((threadIdx.x & 31) + o < 32 && ((threadIdx.x & 31) + o) / T == (threadIdx.x & 31) / T)
-            best_merge(br, bk, r2, k2);
-    }
-    if (T <= 32) {
-        if (live && t == 0) {
-            p.rb[j].r = br;
+        for (int o = 16; o > 0; o >>= 1) {
+            const float r2 = __shfl_down_sync(0xffffffff, br, o);
+            const int k2 = __shfl_down_sync(0xffffffff, bk, o);
+            if (r2 > br || (r2 == br && k2 < bk)) {
+                br = r2;
+                bk = k2;
+            }
+        }
+        if (lane == 0) {
+            p.rb[j].r = (double)br;
             p.rb[j].key = bk;
         }
         return;
     }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        red_r[wid] = br;
-        red_k[wid] = bk;
+    double br = -1.0e30;
+    long long bk = 0x7fffffffffffffffLL;
+    for (int x = xa + lane; x <= xb; x += 32) {
+        const long long dx = x - ox;
+        double rv;
+        if (dx * dx <= in && lag_row_r(p, q, x, __ldg(row + x) * invf, rv))
+            best_merge(br, bk, rv, key0 + (x < 0 ? x + Nx : x));
     }
-    __syncthreads();
-    if (live && t == 0) {
-        const int w0 = team * (T / 32);
-        for (int q = 1; q < T / 32; ++q)
-            best_merge(br, bk, red_r[w0 + q], red_k[w0 + q]);
+    for (int o = 16; o > 0; o >>= 1) {
+        const double r2 = __shfl_down_sync(0xffffffff, br, o);
+        const long long k2 = __shfl_down_sync(0xffffffff, bk, o);
+        best_merge(br, bk, r2, k2);
+    }
+    if (lane == 0) {
         p.rb[j].r = br;
         p.rb[j].key = bk;
     }
