@@ -93,51 +93,6 @@ __device__ __forceinline__ int nslots(const PairDev &p, int i)
     return n;
 }
 
-// IntegralTable, 0_GEN/Correlation.cpp:112-150, on slot-indexed SAT rows
-__device__ __forceinline__ double sat_box(const double *t, const PairDev &p, int i,
-                                          int L, int R, int B, int T)
-{
-    const int w = p.w[i];
-    double r = t[(long long)sat_slot(p, i, T) * w + R];
-    if (L > 0)
-        r -= t[(long long)sat_slot(p, i, T) * w + L - 1];
-    if (B > 0)
-        r -= t[(long long)sat_slot(p, i, B - 1) * w + R];
-    if (L > 0 && B > 0)
-        r += t[(long long)sat_slot(p, i, B - 1) * w + L - 1];
-    return r;
-}
-
-// exact integer box sum; equals the reference's FP64 IntegralTable result
-// whenever the sums are below 2^53 (always, for 8/16-bit pixels)
-__device__ __forceinline__ long long sat_box_i64(const long long *t, const PairDev &p, int i,
-                                                 int L, int R, int B, int T)
-{
-    const int w = p.w[i];
-    long long r = t[(long long)sat_slot(p, i, T) * w + R];
-    if (L > 0)
-        r -= t[(long long)sat_slot(p, i, T) * w + L - 1];
-    if (B > 0)
-        r -= t[(long long)sat_slot(p, i, B - 1) * w + R];
-    if (L > 0 && B > 0)
-        r += t[(long long)sat_slot(p, i, B - 1) * w + L - 1];
-    return r;
-}
-
-__device__ __forceinline__ int sat_box_n(const int *t, const PairDev &p, int i, int L,
-                                         int R, int B, int T)
-{
-    const int w = p.w[i];
-    int r = t[(long long)sat_slot(p, i, T) * w + R];
-    if (L > 0)
-        r -= t[(long long)sat_slot(p, i, T) * w + L - 1];
-    if (B > 0)
-        r -= t[(long long)sat_slot(p, i, B - 1) * w + R];
-    if (L > 0 && B > 0)
-        r += t[(long long)sat_slot(p, i, B - 1) * w + L - 1];
-    return r;
-}
-
 __device__ __forceinline__ bool rgn_ok(const PairDev &p, int sx, int sy)
 {
     switch (p.rgn_kind) {
@@ -203,7 +158,7 @@ __device__ __forceinline__ float i64_to_float(long long v)
 }
 
 // n: the overlap's pixels (a box of an FFT raster: < 2^26); m1, m2: the
-// integer mean shifts
+// integer mean shifts.  (The 32-bit form of the sums is r_int32.)
 __device__ __forceinline__ float r_int(int n, float cs, long long s1, long long q1, long long s2,
                                        long long q2, int m1, int m2)
 {
@@ -216,6 +171,23 @@ __device__ __forceinline__ float r_int(int n, float cs, long long s1, long long 
     const float num = fmaf(fn, cs,
                            -(i64_to_float(s1 - (long long)n * m1) *
                              i64_to_float(s2 - (long long)n * m2)));
+    return num * (rsqrtf(f1) * rsqrtf(f2));
+}
+
+// r_int where the box sums S are below 2^31 (n times the largest pixel value
+// is): they and S - n mu are 32-bit integers, the same numbers with fewer
+// instructions.
+__device__ __forceinline__ float r_int32(int n, float cs, unsigned s1, unsigned long long q1,
+                                         unsigned s2, unsigned long long q2, int m1, int m2)
+{
+    typedef unsigned long long u64;
+    const u64 d1 = (u64)(unsigned)n * q1 - (u64)s1 * s1;
+    const u64 d2 = (u64)(unsigned)n * q2 - (u64)s2 * s2;
+    const float f1 = u64_to_float(d1), f2 = u64_to_float(d2), fn = __int2float_rn(n);
+    if (f1 * f2 < fn * fn * 1.0e-9f)
+        return 0.0f;
+    const float num = fmaf(fn, cs,
+                           -(__int2float_rn((int)s1 - n * m1) * __int2float_rn((int)s2 - n * m2)));
     return num * (rsqrtf(f1) * rsqrtf(f2));
 }
 
@@ -251,12 +223,12 @@ __device__ __forceinline__ LagRow lag_row(const PairDev &p, int y)
     return q;
 }
 
-// IntegralTable (0_GEN/Correlation.cpp:112-150) on a lag row's table rows,
-// columns L..R; int64 sums are exact, FP64 ones in the reference's order
-template <typename TA>
-__device__ __forceinline__ TA row_box(const TA *__restrict__ t, int oT, int oB, int L, int R)
+// Box sums over columns L..R of a lag row's table rows (IntegralTable,
+// 0_GEN/Correlation.cpp:112-150): counts, and the pairs (sum v, sum v^2) as
+// int64 (exact) or FP64 (the reference's order of operations).
+__device__ __forceinline__ int row_box_n(const int *__restrict__ t, int oT, int oB, int L, int R)
 {
-    TA r = __ldg(t + oT + R);
+    int r = __ldg(t + oT + R);
     if (L > 0)
         r -= __ldg(t + oT + L - 1);
     if (oB >= 0) {
@@ -265,6 +237,39 @@ __device__ __forceinline__ TA row_box(const TA *__restrict__ t, int oT, int oB, 
             r += __ldg(t + oB + L - 1);
     }
     return r;
+}
+
+template <typename T2>
+__device__ __forceinline__ T2 row_box2(const T2 *__restrict__ t, int oT, int oB, int L, int R)
+{
+    T2 r = __ldg(t + oT + R);
+    if (L > 0) {
+        const T2 a = __ldg(t + oT + L - 1);
+        r.x -= a.x;
+        r.y -= a.y;
+    }
+    if (oB >= 0) {
+        const T2 b = __ldg(t + oB + R);
+        r.x -= b.x;
+        r.y -= b.y;
+        if (L > 0) {
+            const T2 c = __ldg(t + oB + L - 1);
+            r.x += c.x;
+            r.y += c.y;
+        }
+    }
+    return r;
+}
+
+// the pair as doubles (image i's table holds int64 or FP64 pairs)
+__device__ __forceinline__ double2 row_box_d(const PairDev &p, const LagRow &q, int i, int L, int R)
+{
+    if ((p.sat_int >> i) & 1) {
+        const longlong2 v =
+            row_box2((const longlong2 *)p.sat[i], q.oT[i], q.oB[i], L, R);
+        return make_double2((double)v.x, (double)v.y);
+    }
+    return row_box2((const double2 *)p.sat[i], q.oT[i], q.oB[i], L, R);
 }
 
 // legality of lag (x, y) by box size and counts, q = lag_row(p, y); L2..R2:
@@ -281,8 +286,8 @@ __device__ __forceinline__ bool lag_row_legal(const PairDev &p, const LagRow &q,
         !(p.transposed ? rgn_ok(p, olh, olw) : rgn_ok(p, olw, olh)))
         return false;
     if (p.cnt_kind == ALN_CNT_GT) {
-        const int c1 = row_box(p.satN[0], q.oT[0], q.oB[0], L1, R1);
-        const int c2 = row_box(p.satN[1], q.oT[1], q.oB[1], L2, R2);
+        const int c1 = row_box_n(p.satN[0], q.oT[0], q.oB[0], L1, R1);
+        const int c2 = row_box_n(p.satN[1], q.oT[1], q.oB[1], L2, R2);
         if (!(c1 > p.cnt_n && c2 > p.cnt_n))
             return false;
     }
@@ -300,31 +305,15 @@ __device__ __forceinline__ bool lag_row_r(const PairDev &p, const LagRow &q, int
         return false;
     const int L1 = L2 - x, R1 = R2 - x;
     const int olw = R1 - L1 + 1, olh = q.olh;
-    const long long *iS1 = (const long long *)p.satS[0], *iQ1 = (const long long *)p.satQ[0];
-    const long long *iS2 = (const long long *)p.satS[1], *iQ2 = (const long long *)p.satQ[1];
     if (r_int_ok(p, (long long)olw * olh)) {
-        r = (double)r_int(olw * olh, cs, row_box(iS1, q.oT[0], q.oB[0], L1, R1),
-                          row_box(iQ1, q.oT[0], q.oB[0], L1, R1),
-                          row_box(iS2, q.oT[1], q.oB[1], L2, R2),
-                          row_box(iQ2, q.oT[1], q.oB[1], L2, R2), (int)p.mu[0], (int)p.mu[1]);
+        const longlong2 a = row_box2((const longlong2 *)p.sat[0], q.oT[0], q.oB[0], L1, R1);
+        const longlong2 b = row_box2((const longlong2 *)p.sat[1], q.oT[1], q.oB[1], L2, R2);
+        r = (double)r_int(olw * olh, cs, a.x, a.y, b.x, b.y, (int)p.mu[0], (int)p.mu[1]);
         return true;
     }
     const double n = (double)(olw * olh);
-    double s1, q1, s2, q2;
-    if (p.sat_int & 1) {
-        s1 = (double)row_box(iS1, q.oT[0], q.oB[0], L1, R1);
-        q1 = (double)row_box(iQ1, q.oT[0], q.oB[0], L1, R1);
-    } else {
-        s1 = row_box(p.satS[0], q.oT[0], q.oB[0], L1, R1);
-        q1 = row_box(p.satQ[0], q.oT[0], q.oB[0], L1, R1);
-    }
-    if (p.sat_int & 2) {
-        s2 = (double)row_box(iS2, q.oT[1], q.oB[1], L2, R2);
-        q2 = (double)row_box(iQ2, q.oT[1], q.oB[1], L2, R2);
-    } else {
-        s2 = row_box(p.satS[1], q.oT[1], q.oB[1], L2, R2);
-        q2 = row_box(p.satQ[1], q.oT[1], q.oB[1], L2, R2);
-    }
+    const double2 a = row_box_d(p, q, 0, L1, R1), b = row_box_d(p, q, 1, L2, R2);
+    const double s1 = a.x, q1 = a.y, s2 = b.x, q2 = b.y;
     const double num = n * (double)cs - (s1 - n * p.mu[0]) * (s2 - n * p.mu[1]);
     const double d1 = n * q1 - s1 * s1;
     const double d2 = n * q2 - s2 * s2;
@@ -334,44 +323,18 @@ __device__ __forceinline__ bool lag_row_r(const PairDev &p, const LagRow &q, int
 }
 
 // RCalc::Valid + RCalc::CalcR (0_GEN/Correlation.cpp:1790-1845): legality
-// of lag (x, y) and, when want_r, its Pearson r clamped to (-1, 1) (0 outside).
-__device__ __forceinline__ bool lag_eval(const PairDev &p, int x, int y, double cs, bool want_r,
-                                         double &r)
+// of lag (x, y) and, when want_r, its Pearson r clamped to (-1, 1) (0
+// outside); q = lag_row(p, y).
+__device__ __forceinline__ bool lag_eval(const PairDev &p, const LagRow &q, int x, double cs,
+                                         bool want_r, double &r)
 {
-    const int w1 = p.w[0], h1 = p.h[0], w2 = p.w[1], h2 = p.h[1];
-    int L2 = max(0, x), R2 = min(w2 - 1, x + w1 - 1);
-    int B2 = max(0, y), T2 = min(h2 - 1, y + h1 - 1);
-    R2 = max(R2, L2);
-    T2 = max(T2, B2);
-    const int L1 = L2 - x, R1 = R2 - x, B1 = B2 - y, T1 = T2 - y;
-    const int olw = R1 - L1 + 1, olh = T1 - B1 + 1;
-    bool ok = true;
-    if (p.rgn_kind != ALN_RGN_NONE && !rgn_ok(p, olw, olh))
-        ok = false;
-    if (ok && p.cnt_kind == ALN_CNT_GT) {
-        const int c1 = sat_box_n(p.satN[0], p, 0, L1, R1, B1, T1);
-        const int c2 = sat_box_n(p.satN[1], p, 1, L2, R2, B2, T2);
-        if (!(c1 > p.cnt_n && c2 > p.cnt_n))
-            ok = false;
-    }
+    int L2, R2;
+    const bool ok = lag_row_legal(p, q, x, L2, R2);
     r = 0.0;
     if (want_r) {
-        const double n = (double)(olw * olh);
-        double s1, q1, s2, q2;
-        if (p.sat_int & 1) {
-            s1 = (double)sat_box_i64((const long long *)p.satS[0], p, 0, L1, R1, B1, T1);
-            q1 = (double)sat_box_i64((const long long *)p.satQ[0], p, 0, L1, R1, B1, T1);
-        } else {
-            s1 = sat_box(p.satS[0], p, 0, L1, R1, B1, T1);
-            q1 = sat_box(p.satQ[0], p, 0, L1, R1, B1, T1);
-        }
-        if (p.sat_int & 2) {
-            s2 = (double)sat_box_i64((const long long *)p.satS[1], p, 1, L2, R2, B2, T2);
-            q2 = (double)sat_box_i64((const long long *)p.satQ[1], p, 1, L2, R2, B2, T2);
-        } else {
-            s2 = sat_box(p.satS[1], p, 1, L2, R2, B2, T2);
-            q2 = sat_box(p.satQ[1], p, 1, L2, R2, B2, T2);
-        }
+        const double n = (double)((R2 - L2 + 1) * q.olh);
+        const double2 a = row_box_d(p, q, 0, L2 - x, R2 - x), b = row_box_d(p, q, 1, L2, R2);
+        const double s1 = a.x, q1 = a.y, s2 = b.x, q2 = b.y;
         const double num = n * cs - (s1 - n * p.mu[0]) * (s2 - n * p.mu[1]);
         const double d1 = n * q1 - s1 * s1;
         const double d2 = n * q2 - s2 * s2;
@@ -423,7 +386,7 @@ __global__ void k_colsum(PairDev *pairs)
         return;
     const void *img = p.img[i];
     const long long st = p.stride[i];
-    double *S = p.satS[i], *Q = p.satQ[i];
+    double2 *S = p.sat[i];
     int *N = p.satN[i];
     if (dt == ALN_U8 || dt == ALN_U16) {
         long long s = 0, q = 0;
@@ -436,8 +399,7 @@ __global__ void k_colsum(PairDev *pairs)
             nz += (v != 0);
             if (row_needed(p, i, y)) {
                 const long long o = (long long)sat_slot(p, i, y) * w + c;
-                S[o] = (double)s;
-                Q[o] = (double)q;
+                S[o] = make_double2((double)s, (double)q);
                 N[o] = nz;
             }
         }
@@ -452,8 +414,7 @@ __global__ void k_colsum(PairDev *pairs)
             nz += (v != 0.0);
             if (row_needed(p, i, y)) {
                 const long long o = (long long)sat_slot(p, i, y) * w + c;
-                S[o] = s;
-                Q[o] = q;
+                S[o] = make_double2(s, q);
                 N[o] = nz;
             }
         }
@@ -502,16 +463,15 @@ __global__ void k_rowscan(PairDev *pairs)
     if (p.status != 0 || slot >= nslots(p, i))
         return;
     const int w = p.w[i];
-    double *S = p.satS[i] + (long long)slot * w;
-    double *Q = p.satQ[i] + (long long)slot * w;
+    double2 *S = p.sat[i] + (long long)slot * w;
     int *N = p.satN[i] + (long long)slot * w;
     const int per = (w + blockDim.x - 1) / blockDim.x;
     const int c0 = threadIdx.x * per, c1 = min(w, c0 + per);
     double s = 0.0, q = 0.0;
     int n = 0;
     for (int c = c0; c < c1; ++c) {
-        s += S[c];
-        q += Q[c];
+        s += S[c].x;
+        q += S[c].y;
         n += N[c];
     }
     __shared__ double ss[256], sq[256];
@@ -539,11 +499,10 @@ __global__ void k_rowscan(PairDev *pairs)
     q = sq[threadIdx.x];
     n = sn[threadIdx.x];
     for (int c = c0; c < c1; ++c) {
-        s += S[c];
-        q += Q[c];
+        s += S[c].x;
+        q += S[c].y;
         n += N[c];
-        S[c] = s;
-        Q[c] = q;
+        S[c] = make_double2(s, q);
         N[c] = n;
     }
 }
@@ -1962,9 +1921,9 @@ static int plan_pair(aln_ctx *ctx, const aln_pair &P, PairPlan &pl, bool allow_t
         for (int k = 0; k < 2; ++k)
             if (d.need_hi[i][k] >= d.need_lo[i][k])
                 ns += d.need_hi[i][k] - d.need_lo[i][k] + 1;
-        b += 2 * al256((size_t)ns * d.w[i] * sizeof(double)) + al256((size_t)ns * d.w[i] * sizeof(int));
+        b += al256((size_t)ns * d.w[i] * sizeof(double2)) + al256((size_t)ns * d.w[i] * sizeof(int));
         b += al256((size_t)d.w[i] * sizeof(double));
-        b += 2 * al256((size_t)SAT_WARPS * d.w[i] * sizeof(double)) +
+        b += al256((size_t)SAT_WARPS * d.w[i] * sizeof(double2)) +
              al256((size_t)SAT_WARPS * d.w[i] * sizeof(int));
     }
     b += al256((size_t)L1 * d.Ny * sizeof(float2));
@@ -2035,18 +1994,14 @@ static size_t carve(PairPlan &pl, char *base, const aln_pair &P)
         for (int k = 0; k < 2; ++k)
             if (d.need_hi[i][k] >= d.need_lo[i][k])
                 ns += d.need_hi[i][k] - d.need_lo[i][k] + 1;
-        d.satS[i] = (double *)p;
-        p += al256((size_t)ns * d.w[i] * sizeof(double));
-        d.satQ[i] = (double *)p;
-        p += al256((size_t)ns * d.w[i] * sizeof(double));
+        d.sat[i] = (double2 *)p;
+        p += al256((size_t)ns * d.w[i] * sizeof(double2));
         d.satN[i] = (int *)p;
         p += al256((size_t)ns * d.w[i] * sizeof(int));
         d.colsum[i] = (double *)p;
         p += al256((size_t)d.w[i] * sizeof(double));
-        d.segS[i] = (double *)p;
-        p += al256((size_t)SAT_WARPS * d.w[i] * sizeof(double));
-        d.segQ[i] = (double *)p;
-        p += al256((size_t)SAT_WARPS * d.w[i] * sizeof(double));
+        d.seg[i] = (double2 *)p;
+        p += al256((size_t)SAT_WARPS * d.w[i] * sizeof(double2));
         d.segN[i] = (int *)p;
         p += al256((size_t)SAT_WARPS * d.w[i] * sizeof(int));
     }

@@ -120,6 +120,23 @@ __device__ __forceinline__ int sat_seg_start(const PairDev &p, int i, int g)
 // Accumulator of a warp's segment-local sums: 32-bit for uint8 pixels (a
 // segment is at most 1536 rows -- h <= 8192 -- so the sums of v and v^2 stay
 // below 2^27), the table type otherwise.
+// a table entry: (sum v, sum v^2)
+template <typename TA>
+struct SatPair;
+template <>
+struct SatPair<long long> {
+    typedef longlong2 type;
+    __device__ __forceinline__ static longlong2 of(long long s, long long q)
+    {
+        return make_longlong2(s, q);
+    }
+};
+template <>
+struct SatPair<double> {
+    typedef double2 type;
+    __device__ __forceinline__ static double2 of(double s, double q) { return make_double2(s, q); }
+};
+
 template <typename TA, typename PIX>
 struct SatAcc {
     typedef TA type;
@@ -144,8 +161,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
     const int lo1 = p.need_lo[i][1], hi1 = p.need_hi[i][1];
     const int len0 = hi0 - lo0 + 1;
     const bool want_n = p.cnt_kind == ALN_CNT_GT;
-    TA *__restrict__ S = (TA *)p.satS[i];
-    TA *__restrict__ Q = (TA *)p.satQ[i];
+    typename SatPair<TA>::type *__restrict__ S = (typename SatPair<TA>::type *)p.sat[i];
     int *__restrict__ N = p.satN[i];
     AC s = 0, q = 0;
     int n = 0;
@@ -181,8 +197,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
                 if (SQ) {
                     s += v;
                     q += v * v;
-                    S[o] = (TA)s;
-                    Q[o] = (TA)q;
+                    S[o] = SatPair<TA>::of((TA)s, (TA)q);
                 }
                 if (want_n)
                     n += (v != 0);
@@ -204,8 +219,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
         on += shN[g * 32 + tx];
     }
     if (SQ) {
-        ((TA *)p.segS[i])[ty * w + c] = os;
-        ((TA *)p.segQ[i])[ty * w + c] = oq;
+        ((typename SatPair<TA>::type *)p.seg[i])[ty * w + c] = SatPair<TA>::of(os, oq);
         if (ty == SAT_WARPS - 1)
             p.colsum[i][c] = (double)(os + (TA)s);
     }
@@ -367,11 +381,10 @@ __global__ void k_transpose(PairDev *pairs)
 // The row pass of the summed-area tables: per needed row, add the warp
 // segment offsets of k3_sat and take the x-prefix.  One warp per row (no
 // block-wide synchronisation, so a CTA carries eight rows and small images
-// do not pay one CTA per row); the warp walks the row 32 columns at a time,
-// lane l on column c0 + l: coalesced loads and stores, an inclusive shuffle
-// scan per 32 columns and a carry between them.  (On the uneven uint16 batch
-// this took 16 ms per 20000 pairs where a CTA-per-row scan on the rows wider
-// than 512 columns took 29 ms.)
+// do not pay one CTA per row); the warp walks the row a few columns per lane
+// at a time, with an inclusive shuffle scan per step and a carry between them.
+// (On the uneven uint16 batch a CTA-per-row scan on the rows wider than 512
+// columns took nearly twice as long.)
 
 template <typename TA>
 __device__ __forceinline__ TA warp_incl_scan(TA v, int lane)
@@ -385,55 +398,48 @@ __device__ __forceinline__ TA warp_incl_scan(TA v, int lane)
     return v;
 }
 
-template <typename TA, bool SQ>
-__device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, int y, TA *S,
-                                             TA *Q, int lane)
+// Four consecutive columns per lane: three additions, then one scan of the
+// lanes' totals per 128 columns (a scan is ten 64-bit shuffles, and on FP64
+// tables ten additions on the narrow FP64 pipe: 199 -> 148 us for 24 pairs of
+// FP64 images, where one column per lane took a scan per 32 columns).
+template <typename TA>
+__device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, int y, int lane)
 {
+    typedef SatPair<TA> SP;
+    constexpr int K = 4;
     const int w = p.w[i];
     const int seg = sat_seg_of(p, i, y);
-    const TA *__restrict__ oS = (const TA *)p.segS[i] + (long long)seg * w;
-    const TA *__restrict__ oQ = (const TA *)p.segQ[i] + (long long)seg * w;
-    const int *__restrict__ oN = p.segN[i] + (long long)seg * w;
-    TA *__restrict__ rS = S + (long long)slot * w;
-    TA *__restrict__ rQ = Q + (long long)slot * w;
-    int *__restrict__ rN = p.satN[i] + (long long)slot * w;
-    // the count table only where a count rule reads it (uniform per job)
-    const bool want_n = p.cnt_kind == ALN_CNT_GT;
+    const typename SP::type *__restrict__ o =
+        (const typename SP::type *)p.seg[i] + (long long)seg * w;
+    typename SP::type *__restrict__ r = (typename SP::type *)p.sat[i] + (long long)slot * w;
     TA cs = 0, cq = 0;
-    int cn = 0;
-    for (int c0 = 0; c0 < w; c0 += 32) {
-        const int c = c0 + lane;
-        const bool ok = c < w;
-        TA vs = 0, vq = 0;
-        int vn = 0;
-        if (ok) {
-            if (SQ) {
-                vs = rS[c] + oS[c];
-                vq = rQ[c] + oQ[c];
+    for (int c0 = 0; c0 < w; c0 += 32 * K) {
+        const int c = c0 + K * lane;
+        TA s[K], q[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            s[k] = q[k] = 0;
+            if (c + k < w) {
+                const typename SP::type a = r[c + k], b = __ldg(o + c + k);
+                s[k] = a.x + b.x;
+                q[k] = a.y + b.y;
             }
-            if (want_n)
-                vn = rN[c] + oN[c];
         }
-        if (SQ) {
-            vs = warp_incl_scan(vs, lane) + cs;
-            vq = warp_incl_scan(vq, lane) + cq;
+#pragma unroll
+        for (int k = 1; k < K; ++k) {
+            s[k] += s[k - 1];
+            q[k] += q[k - 1];
         }
-        if (want_n)
-            vn = warp_incl_scan(vn, lane) + cn;
-        if (ok) {
-            if (SQ) {
-                rS[c] = vs;
-                rQ[c] = vq;
-            }
-            if (want_n)
-                rN[c] = vn;
-        }
-        if (SQ) {
-            cs = __shfl_sync(0xffffffff, vs, 31);
-            cq = __shfl_sync(0xffffffff, vq, 31);
-        }
-        if (want_n)
-            cn = __shfl_sync(0xffffffff, vn, 31);
+        const TA ts = warp_incl_scan(s[K - 1], lane), tq = warp_incl_scan(q[K - 1], lane);
+        TA bs = __shfl_up_sync(0xffffffff, ts, 1), bq = __shfl_up_sync(0xffffffff, tq, 1);
+        bs = lane ? bs + cs : cs;
+        bq = lane ? bq + cq : cq;
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (c + k < w)
+                r[c + k] = SP::of(s[k] + bs, q[k] + bq);
+        cs += __shfl_sync(0xffffffff, ts, 31);
+        cq += __shfl_sync(0xffffffff, tq, 31);
     }
 }
 
@@ -485,20 +491,14 @@ __global__ void k2_sat2w(PairDev *pairs)
     const int len0 = p.need_hi[i][0] - p.need_lo[i][0] + 1;
     const int y = slot < len0 ? p.need_lo[i][0] + slot : p.need_lo[i][1] + slot - len0;
     const int lane = threadIdx.x & 31;
-    if (NONLY) {
-        if (p.sat_nonly)
-            sat2_row_counts(p, i, slot, y, lane);
-        else
-            sat2_row_any<long long, false>(p, i, slot, y, (long long *)p.satS[i],
-                                           (long long *)p.satQ[i], lane);
-    } else if (p.sat_nonly)
-        sat2_row_any<long long, false>(p, i, slot, y, (long long *)p.satS[i],
-                                       (long long *)p.satQ[i], lane);
-    else if (int_pixels(p.dt[i]))
-        sat2_row_any<long long, true>(p, i, slot, y, (long long *)p.satS[i],
-                                      (long long *)p.satQ[i], lane);
+    if (p.cnt_kind == ALN_CNT_GT)   // the count table only where a count rule reads it
+        sat2_row_counts(p, i, slot, y, lane);
+    if (NONLY || p.sat_nonly)
+        return;
+    if (int_pixels(p.dt[i]))
+        sat2_row_any<long long>(p, i, slot, y, lane);
     else
-        sat2_row_any<double, true>(p, i, slot, y, p.satS[i], p.satQ[i], lane);
+        sat2_row_any<double>(p, i, slot, y, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -1089,11 +1089,13 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
     const float invf = 1.0f / ((float)Nx * (float)Ny);
     const LagRow q = lag_row(p, y);
     const int key0 = (y < 0 ? y + Ny : y) * Nx;   // storage indices are < 2^26
-    if (r_int_ok(p, (long long)min(p.w[0], p.w[1]) * q.olh)) {
+    const int nmax = min(p.w[0], p.w[1]) * q.olh;   // largest overlap of the row
+    if (r_int_ok(p, nmax)) {
         // every lag of the row takes r_int: FP32 keys
-        const long long *S1 = (const long long *)p.satS[0], *Q1 = (const long long *)p.satQ[0];
-        const long long *S2 = (const long long *)p.satS[1], *Q2 = (const long long *)p.satQ[1];
+        const longlong2 *t1 = (const longlong2 *)p.sat[0], *t2 = (const longlong2 *)p.sat[1];
         const int m1 = (int)p.mu[0], m2 = (int)p.mu[1];
+        const bool narrow =
+            nmax < (p.dt[0] == ALN_U8 && p.dt[1] == ALN_U8 ? 1 << 23 : 1 << 15);
         float br = -1.0e30f;
         int bk = 0x7fffffff;
         for (int x = xa + lane; x <= xb; x += 32) {
@@ -1101,11 +1103,12 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
             int L2, R2;
             if (dx * dx > in || !lag_row_legal(p, q, x, L2, R2))
                 continue;
-            const float r = r_int((R2 - L2 + 1) * q.olh, __ldg(row + x) * invf,
-                                  row_box(S1, q.oT[0], q.oB[0], L2 - x, R2 - x),
-                                  row_box(Q1, q.oT[0], q.oB[0], L2 - x, R2 - x),
-                                  row_box(S2, q.oT[1], q.oB[1], L2, R2),
-                                  row_box(Q2, q.oT[1], q.oB[1], L2, R2), m1, m2);
+            const int n = (R2 - L2 + 1) * q.olh;
+            const float cs = __ldg(row + x) * invf;
+            const longlong2 a = row_box2(t1, q.oT[0], q.oB[0], L2 - x, R2 - x);
+            const longlong2 b = row_box2(t2, q.oT[1], q.oB[1], L2, R2);
+            const float r = narrow ? r_int32(n, cs, (unsigned)a.x, a.y, (unsigned)b.x, b.y, m1, m2)
+                                   : r_int(n, cs, a.x, a.y, b.x, b.y, m1, m2);
             const int k = key0 + (x < 0 ? x + Nx : x);
             if (r > br || (r == br && k < bk)) {
                 br = r;
@@ -1248,7 +1251,7 @@ __global__ void __launch_bounds__(256, SONLY ? 3 : 2) k2_lagimg(PairDev *pairs, 
             if (bk == 0x7fffffffffffffffLL || c > bc) {
                 double rv;
                 const int ix = x + p.cx;
-                if (lag_eval(p, x, y, 0.0, false, rv) && oval_ok(p, ix, iy)) {
+                if (lag_eval(p, lag_row(p, y), x, 0.0, false, rv) && oval_ok(p, ix, iy)) {
                     bc = c;
                     bk = (long long)iy * p.wR + ix;
                 }
@@ -1261,6 +1264,7 @@ __global__ void __launch_bounds__(256, SONLY ? 3 : 2) k2_lagimg(PairDev *pairs, 
     } else if (!SONLY && live) {
         const int y = p.ylo + j, iy = y + p.cy;
         const bool keyS = p.mode == JOB_IMAGES_S;
+        const LagRow lr = lag_row(p, y);
         for (int x = p.xlo + t; x <= p.xhi; x += T) {
             const int xs = x < 0 ? x + Nx : x;
             double S = 0.0, rv = 0.0;
@@ -1269,7 +1273,7 @@ __global__ void __launch_bounds__(256, SONLY ? 3 : 2) k2_lagimg(PairDev *pairs, 
                 ss += S;
                 ss2 += S * S;
             }
-            const bool legal = lag_eval(p, x, y, want_r ? (double)CR[xs] * inv : 0.0, want_r, rv);
+            const bool legal = lag_eval(p, lr, x, want_r ? (double)CR[xs] * inv : 0.0, want_r, rv);
             const double key = keyS ? S : rv;
             const long long o = (long long)j * Wx + (x - p.xlo);
             p.rr[o] = key;
