@@ -166,29 +166,25 @@ __device__ __forceinline__ float r_int(int n, float cs, long long s1, long long 
     const u64 un = (u64)n;
     const u64 d1 = un * (u64)q1 - (u64)s1 * (u64)s1, d2 = un * (u64)q2 - (u64)s2 * (u64)s2;
     const float f1 = u64_to_float(d1), f2 = u64_to_float(d2), fn = __int2float_rn(n);
-    if (f1 * f2 < fn * fn * 1.0e-9f)
-        return 0.0f;
     const float num = fmaf(fn, cs,
                            -(i64_to_float(s1 - (long long)n * m1) *
                              i64_to_float(s2 - (long long)n * m2)));
-    return num * (rsqrtf(f1) * rsqrtf(f2));
+    return f1 * f2 < fn * fn * 1.0e-9f ? 0.0f : num * (rsqrtf(f1) * rsqrtf(f2));
 }
 
-// r_int where the box sums S are below 2^31 (n times the largest pixel value
-// is): they and S - n mu are 32-bit integers, the same numbers with fewer
-// instructions.
-__device__ __forceinline__ float r_int32(int n, float cs, unsigned s1, unsigned long long q1,
-                                         unsigned s2, unsigned long long q2, int m1, int m2)
+// r_int where the box sums S are below 2^31 in size (n times the largest pixel
+// value is): they and S - n mu are 32-bit integers, the same numbers with
+// fewer instructions.  Also for sums of u = v - 128 with mu - 128.
+__device__ __forceinline__ float r_int32(int n, float cs, int s1, unsigned long long q1, int s2,
+                                         unsigned long long q2, int m1, int m2)
 {
     typedef unsigned long long u64;
-    const u64 d1 = (u64)(unsigned)n * q1 - (u64)s1 * s1;
-    const u64 d2 = (u64)(unsigned)n * q2 - (u64)s2 * s2;
+    const u64 d1 = (u64)(unsigned)n * q1 - (u64)((long long)s1 * s1);
+    const u64 d2 = (u64)(unsigned)n * q2 - (u64)((long long)s2 * s2);
     const float f1 = u64_to_float(d1), f2 = u64_to_float(d2), fn = __int2float_rn(n);
-    if (f1 * f2 < fn * fn * 1.0e-9f)
-        return 0.0f;
     const float num = fmaf(fn, cs,
-                           -(__int2float_rn((int)s1 - n * m1) * __int2float_rn((int)s2 - n * m2)));
-    return num * (rsqrtf(f1) * rsqrtf(f2));
+                           -(__int2float_rn(s1 - n * m1) * __int2float_rn(s2 - n * m2)));
+    return f1 * f2 < fn * fn * 1.0e-9f ? 0.0f : num * (rsqrtf(f1) * rsqrtf(f2));
 }
 
 // the overlap sizes for which r_int is exact on this pair's pixel types
@@ -200,13 +196,17 @@ __device__ __forceinline__ bool r_int_ok(const PairDev &p, long long n)
     return u8 || n < (1ll << 20);
 }
 
-// The summed-area rows that the overlap boxes of one lag row read, per image:
-// row T of the box and, when the box starts above row 0, row B - 1 (element
-// offsets into the tables).  The same for every lag of the row, so a scan
-// over a row computes them once.
+// What the lags of one lag row share, so that a scan over the row computes
+// it once and reads the job's descriptor no more: the summed-area rows that
+// their overlap boxes read, per image (row T of the box and, when the box
+// starts above row 0, row B - 1; element offsets into the tables), and the
+// legal box widths.
 struct LagRow {
     int olh;           // box height
+    int w1, w2;
+    int omin, omax;    // LegalRgn holds for widths omin..omax (all but a table)
     int oT[2], oB[2];  // oB < 0: the box starts at row 0
+    bool tbl, cnt;     // a legality table / a count rule to look up per lag
 };
 
 __device__ __forceinline__ LagRow lag_row(const PairDev &p, int y)
@@ -215,11 +215,35 @@ __device__ __forceinline__ LagRow lag_row(const PairDev &p, int y)
     const int B2 = max(0, y), T2 = max(min(p.h[1] - 1, y + p.h[0] - 1), B2);
     const int B[2] = {B2 - y, B2}, T[2] = {T2 - y, T2};
     q.olh = T2 - B2 + 1;
+    q.w1 = p.w[0];
+    q.w2 = p.w[1];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        q.oT[i] = sat_slot(p, i, T[i]) * p.w[i];
-        q.oB[i] = B[i] > 0 ? sat_slot(p, i, B[i] - 1) * p.w[i] : -1;
+        q.oT[i] = sat_slot(p, i, T[i]) * p.sp[i];
+        q.oB[i] = B[i] > 0 ? sat_slot(p, i, B[i] - 1) * p.sp[i] : -1;
     }
+    // rgn_ok for a box of q.olh rows as a range of widths: width * olh > area
+    // is width > floor(area / olh).  A transposed job evaluates LegalRgn on
+    // the caller's (untransposed) box.
+    const int kind = p.rgn_kind, a = p.rgn_a, b = p.rgn_b, INF = 0x7fffffff;
+    const long long area = p.rgn_area;
+    const int wide = area < 0 ? 0 : area >= INF ? INF
+                              : (int)((unsigned)area / (unsigned)q.olh) + 1;
+    const bool tr = p.transposed != 0;
+    q.omin = 0;
+    q.omax = INF;
+    if (kind == ALN_RGN_MIN) {
+        q.omin = (tr ? q.olh >= a : q.olh >= b) ? max(wide, tr ? b : a) : INF;
+    } else if (kind == ALN_RGN_SECTION) {
+        q.omin = max(wide, tr ? (q.olh >= a ? 0 : b >= INF - 1 ? INF : b + 1)
+                              : (q.olh > b ? 0 : a));
+    } else if (kind == ALN_RGN_EXACT) {
+        q.omin = q.omax = tr ? b : a;
+        if (q.olh != (tr ? a : b))
+            q.omin = INF;
+    }
+    q.tbl = kind == ALN_RGN_TABLE;
+    q.cnt = p.cnt_kind == ALN_CNT_GT;
     return q;
 }
 
@@ -261,12 +285,58 @@ __device__ __forceinline__ T2 row_box2(const T2 *__restrict__ t, int oT, int oB,
     return r;
 }
 
-// the pair as doubles (image i's table holds int64 or FP64 pairs)
+// Packed entries (uint8 images): with u = v - 128, one integer
+// sum(u^2) 2^29 + sum(u), modulo 2^64.  Entries add and subtract as they are,
+// and a box whose overlap has n < SAT_PACK_N pixels comes apart again: |sum u|
+// <= 128 n < 2^28, sum u^2 <= 128^2 n < 2^35.  Half the table's bytes and half
+// its additions.  The correlation needs no more: n sum v^2 - (sum v)^2 and
+// sum v - n mu are the same integers for u and mu - 128.
+#define SAT_PACK_N (1 << 21)
+__host__ __device__ __forceinline__ unsigned long long sat_pack(int su, unsigned su2)
+{
+    return ((unsigned long long)su2 << 29) + (unsigned long long)(long long)su;
+}
+__device__ __forceinline__ int sat_pack_s(unsigned long long e)
+{
+    return (int)((unsigned)e << 3) >> 3;
+}
+__device__ __forceinline__ unsigned long long sat_pack_q(unsigned long long e, int su)
+{
+    return (e - (unsigned long long)(long long)su) >> 29;
+}
+
+__device__ __forceinline__ unsigned long long row_box_p(const unsigned long long *__restrict__ t,
+                                                        int oT, int oB, int L, int R)
+{
+    unsigned long long r = __ldg(t + oT + R);
+    if (L > 0)
+        r -= __ldg(t + oT + L - 1);
+    if (oB >= 0) {
+        r -= __ldg(t + oB + R);
+        if (L > 0)
+            r += __ldg(t + oB + L - 1);
+    }
+    return r;
+}
+
+// the int64 sums of v and v^2 of a box of n pixels
+__device__ __forceinline__ longlong2 row_box_i(const PairDev &p, const LagRow &q, int i, int n,
+                                               int L, int R)
+{
+    if (!p.sat_packed)
+        return row_box2((const longlong2 *)p.sat[i], q.oT[i], q.oB[i], L, R);
+    const unsigned long long e =
+        row_box_p((const unsigned long long *)p.sat[i], q.oT[i], q.oB[i], L, R);
+    const int su = sat_pack_s(e);
+    return make_longlong2((long long)su + 128ll * n,
+                          (long long)sat_pack_q(e, su) + 256ll * su + 16384ll * n);
+}
+
+// the pair as doubles (image i's table holds integers or FP64 pairs)
 __device__ __forceinline__ double2 row_box_d(const PairDev &p, const LagRow &q, int i, int L, int R)
 {
     if ((p.sat_int >> i) & 1) {
-        const longlong2 v =
-            row_box2((const longlong2 *)p.sat[i], q.oT[i], q.oB[i], L, R);
+        const longlong2 v = row_box_i(p, q, i, (R - L + 1) * q.olh, L, R);
         return make_double2((double)v.x, (double)v.y);
     }
     return row_box2((const double2 *)p.sat[i], q.oT[i], q.oB[i], L, R);
@@ -278,15 +348,14 @@ __device__ __forceinline__ bool lag_row_legal(const PairDev &p, const LagRow &q,
                                               int &R2)
 {
     L2 = max(0, x);
-    R2 = max(min(p.w[1] - 1, x + p.w[0] - 1), L2);
-    const int L1 = L2 - x, R1 = R2 - x;
-    const int olw = R1 - L1 + 1, olh = q.olh;
-    // a transposed job evaluates LegalRgn on the caller's (untransposed) box
-    if (p.rgn_kind != ALN_RGN_NONE &&
-        !(p.transposed ? rgn_ok(p, olh, olw) : rgn_ok(p, olw, olh)))
+    R2 = max(min(q.w2 - 1, x + q.w1 - 1), L2);
+    const int olw = R2 - L2 + 1;
+    if (olw < q.omin || olw > q.omax)
         return false;
-    if (p.cnt_kind == ALN_CNT_GT) {
-        const int c1 = row_box_n(p.satN[0], q.oT[0], q.oB[0], L1, R1);
+    if (q.tbl && !(p.transposed ? rgn_ok(p, q.olh, olw) : rgn_ok(p, olw, q.olh)))
+        return false;
+    if (q.cnt) {
+        const int c1 = row_box_n(p.satN[0], q.oT[0], q.oB[0], L2 - x, R2 - x);
         const int c2 = row_box_n(p.satN[1], q.oT[1], q.oB[1], L2, R2);
         if (!(c1 > p.cnt_n && c2 > p.cnt_n))
             return false;
@@ -306,8 +375,8 @@ __device__ __forceinline__ bool lag_row_r(const PairDev &p, const LagRow &q, int
     const int L1 = L2 - x, R1 = R2 - x;
     const int olw = R1 - L1 + 1, olh = q.olh;
     if (r_int_ok(p, (long long)olw * olh)) {
-        const longlong2 a = row_box2((const longlong2 *)p.sat[0], q.oT[0], q.oB[0], L1, R1);
-        const longlong2 b = row_box2((const longlong2 *)p.sat[1], q.oT[1], q.oB[1], L2, R2);
+        const longlong2 a = row_box_i(p, q, 0, olw * olh, L1, R1);
+        const longlong2 b = row_box_i(p, q, 1, olw * olh, L2, R2);
         r = (double)r_int(olw * olh, cs, a.x, a.y, b.x, b.y, (int)p.mu[0], (int)p.mu[1]);
         return true;
     }
@@ -1661,6 +1730,8 @@ static void need_rows(const PairDev &d, int img, int lo[2], int hi[2])
 
 #include "aln_tune.cuh"
 
+static size_t sat_entry_bytes(const PairDev &d) { return d.sat_packed ? 8 : sizeof(double2); }
+
 // allow_split: the caller runs the register pipeline (batch path), whose row
 // kernels take the split lengths of ALN_CASES_LMIX; the allocation-free
 // entry point's kernels take powers of two only.
@@ -1905,6 +1976,10 @@ static int plan_pair(aln_ctx *ctx, const aln_pair &P, PairPlan &pl, bool allow_t
             d.need_lo[i][0] = d.need_lo[i][1] = 1;
             d.need_hi[i][0] = d.need_hi[i][1] = 0;
         }
+    // packed tables where every overlap fits them (the batch paths' k3_sat)
+    d.sat_packed = (spec || allow_split) && d.mode != JOB_P2I && !d.sat_nonly &&
+                   d.dt[0] == ALN_U8 && d.dt[1] == ALN_U8 &&
+                   (long long)std::min(d.w[0], d.w[1]) * std::min(d.h[0], d.h[1]) < SAT_PACK_N;
     const int L1 = d.Nx / 2 + 1;
     const int Wy = d.yhi - d.ylo + 1, Wx = d.xhi - d.xlo + 1;
     size_t b = 0;
@@ -1921,10 +1996,12 @@ static int plan_pair(aln_ctx *ctx, const aln_pair &P, PairPlan &pl, bool allow_t
         for (int k = 0; k < 2; ++k)
             if (d.need_hi[i][k] >= d.need_lo[i][k])
                 ns += d.need_hi[i][k] - d.need_lo[i][k] + 1;
-        b += al256((size_t)ns * d.w[i] * sizeof(double2)) + al256((size_t)ns * d.w[i] * sizeof(int));
+        d.sp[i] = d.sat_packed ? (d.w[i] + 1) & ~1 : d.w[i];
+        const size_t es = sat_entry_bytes(d);
+        b += al256((size_t)ns * d.sp[i] * es) + al256((size_t)ns * d.sp[i] * sizeof(int));
         b += al256((size_t)d.w[i] * sizeof(double));
-        b += al256((size_t)SAT_WARPS * d.w[i] * sizeof(double2)) +
-             al256((size_t)SAT_WARPS * d.w[i] * sizeof(int));
+        b += al256((size_t)SAT_WARPS * d.sp[i] * es) +
+             al256((size_t)SAT_WARPS * d.sp[i] * sizeof(int));
     }
     b += al256((size_t)L1 * d.Ny * sizeof(float2));
     b += al256((size_t)L1 * Wy * sizeof(float2));
@@ -1994,16 +2071,17 @@ static size_t carve(PairPlan &pl, char *base, const aln_pair &P)
         for (int k = 0; k < 2; ++k)
             if (d.need_hi[i][k] >= d.need_lo[i][k])
                 ns += d.need_hi[i][k] - d.need_lo[i][k] + 1;
+        const size_t es = sat_entry_bytes(d);
         d.sat[i] = (double2 *)p;
-        p += al256((size_t)ns * d.w[i] * sizeof(double2));
+        p += al256((size_t)ns * d.sp[i] * es);
         d.satN[i] = (int *)p;
-        p += al256((size_t)ns * d.w[i] * sizeof(int));
+        p += al256((size_t)ns * d.sp[i] * sizeof(int));
         d.colsum[i] = (double *)p;
         p += al256((size_t)d.w[i] * sizeof(double));
         d.seg[i] = (double2 *)p;
-        p += al256((size_t)SAT_WARPS * d.w[i] * sizeof(double2));
+        p += al256((size_t)SAT_WARPS * d.sp[i] * es);
         d.segN[i] = (int *)p;
-        p += al256((size_t)SAT_WARPS * d.w[i] * sizeof(int));
+        p += al256((size_t)SAT_WARPS * d.sp[i] * sizeof(int));
     }
     d.X2 = (float2 *)p;
     p += al256((size_t)L1 * d.Ny * sizeof(float2));
@@ -2239,6 +2317,7 @@ struct ChunkLaunch {
     int t8;                            // every transposed job is uint8 (128-byte tiles)
     int Nx, Ny, mode, both, sonly, frame_nx1, frame_ny1;
     int seg;                           // CorrPatches with segmented columns
+    int packed;                        // packed summed-area tables
     int fill_off, nfill, fill_maxh;    // spectrum-cache fills: sel[fill_off ...]
 };
 
@@ -2313,6 +2392,7 @@ static void prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, ch
     cl.frame_nx1 = chunk[0]->frame_nx1;
     cl.frame_ny1 = chunk[0]->frame_ny1;
     cl.seg = hd[0].nseg > 0;
+    cl.packed = hd[0].sat_packed;
 }
 
 // The chunk's kernels on the compute stream (its job table, fill list and
@@ -2338,8 +2418,13 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
                dim3(32, 8), 0, ctx->dpairs);
     const int mode = cl.mode;
     if (mode != JOB_P2I) {
-        LAUNCH(ctx, "k3_sat", k3_sat, dim3((cl.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS), 0,
-               ctx->dpairs);
+        if (cl.packed) {
+            smem_attr(ctx->device, (const void *)k3_satp, satp_smem());
+            LAUNCH(ctx, "k3_sat", k3_satp, dim3((cl.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
+                   satp_smem(), ctx->dpairs);
+        } else
+            LAUNCH(ctx, "k3_sat", k3_sat, dim3((cl.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS),
+                   0, ctx->dpairs);
         LAUNCH(ctx, "k_mean", k_mean, dim3(2, n), 256, 0, ctx->dpairs);
         if (cl.sonly)
             LAUNCH(ctx, "k2_sat2w", k2_sat2w<true>, dim3((cl.maxslots + 7) / 8, 2, n), 256, 0,
@@ -2699,15 +2784,16 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
     std::vector<std::vector<std::vector<PairPlan *>>> wchunks(windows.size());
     size_t max_stage = 0, max_work = 0, max_n = 1;
     for (size_t w = 0; w < windows.size(); ++w) {
-        std::map<std::tuple<int, int, int, int, int, int, int, int, int>,
+        std::map<std::tuple<int, int, int, int, int, int, int, int, int, int>,
                  std::vector<PairPlan *>>
             groups;
         size_t sb = 0;
         for (PairPlan *pl : windows[w]) {
-            // transposed jobs apart: their chunks alone launch the transpose
+            // transposed jobs apart: their chunks alone launch the transpose;
+            // packed tables apart: they have their own column walk
             groups[std::make_tuple(pl->d.Nx, pl->d.Ny, pl->frame_nx1, pl->frame_ny1, pl->d.mode,
                                    pl->d.want_r, pl->d.want_s, pl->d.nseg > 0,
-                                   pl->transposed ? 1 : 0)]
+                                   pl->transposed ? 1 : 0, pl->d.sat_packed)]
                 .push_back(pl);
             sb += pl->in_bytes[0] + pl->in_bytes[1] + 16;
         }

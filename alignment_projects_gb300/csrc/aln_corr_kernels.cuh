@@ -66,7 +66,10 @@ struct PairDev {
                         // the row pass skips b and the column pass reads X2
     float2 *Q;          // column-inverse output [kx][j], j = y - ylo, stride Wy
     double2 *sat[2];             // summed-area tables of v (.x) and v^2 (.y), [y][x]
-                                 // stride w: one 16-byte load reads both
+                                 // stride sp: one 16-byte load reads both
+    int sp[2];                   // table row pitch in entries (w; even when packed)
+    int sat_packed;              // 1: both images uint8 and their overlaps small enough
+                                 // for one 64-bit integer per entry (sat_pack)
     int *satN[2];                // summed-area table of (v != 0)
     int sat_int;                 // bit i: image i's table holds int64 pairs
     int sat_nonly;               // 1: only the count table N is needed (S key alone)

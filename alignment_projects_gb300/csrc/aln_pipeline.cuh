@@ -192,7 +192,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
             const bool first = y >= lo0 && y <= hi0;
             const int rend = min(y1 - 1, first ? hi0 : hi1);
             const long long base = first ? (long long)(y - lo0) : (long long)(len0 + y - lo1);
-            for (long long o = base * w + c; y <= rend; ++y, o += w) {
+            for (long long o = base * p.sp[i] + c; y <= rend; ++y, o += p.sp[i]) {
                 const AC v = (AC)__ldg(&col[y * st]);
                 if (SQ) {
                     s += v;
@@ -219,11 +219,199 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
         on += shN[g * 32 + tx];
     }
     if (SQ) {
-        ((typename SatPair<TA>::type *)p.seg[i])[ty * w + c] = SatPair<TA>::of(os, oq);
+        ((typename SatPair<TA>::type *)p.seg[i])[ty * p.sp[i] + c] = SatPair<TA>::of(os, oq);
         if (ty == SAT_WARPS - 1)
             p.colsum[i][c] = (double)(os + (TA)s);
     }
-    p.segN[i][ty * w + c] = on;
+    p.segN[i][ty * p.sp[i] + c] = on;
+}
+
+// The walk for packed tables (uint8): two columns per thread, 64 per CTA.
+// Each warp copies its rows to shared memory SATP_ROWS at a time with
+// asynchronous 16-byte copies, the next block's in flight while this one is
+// summed: the walk through registers kept 16 rows of 64 bytes per warp in
+// flight and waited on them (stall "long scoreboard" 13.6 per issue, 23 % of
+// issue slots).  Four rows at a time are turned into one word per column and
+// summed by dot products: about 2 instructions per pixel where the general
+// walk takes 5, and a stored row is one 16-byte store per thread of whole
+// sectors.
+#define SATP_ROWS 32
+#define SATP_PITCH 80   // 64 bytes of a row in 16-byte blocks, any start
+
+__host__ __device__ constexpr int satp_smem() { return SAT_WARPS * 2 * SATP_ROWS * SATP_PITCH; }
+
+__device__ __forceinline__ void cp_async16(unsigned dst_shared, const void *src_global)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_shared), "l"(src_global)
+                 : "memory");
+}
+
+template <bool COUNT>
+__device__ __forceinline__ void sat_cols_packed(const PairDev &p, int i, unsigned char *stage,
+                                                unsigned long long *shP, int *shN)
+{
+    typedef unsigned long long u64;
+    const int w = p.w[i], h = p.h[i], sp = p.sp[i];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int c0 = blockIdx.x * 64, c = c0 + 2 * tx;
+    const bool cok = c < w, two = c + 1 < w;
+    const int y0 = sat_seg_start(p, i, ty), y1 = sat_seg_start(p, i, ty + 1);
+    const long long st = p.stride[i];
+    const unsigned char *band = (const unsigned char *)p.img[i] + c0;
+    const int nb = min(64, w - c0);   // bytes of the band's rows
+    const int lo0 = p.need_lo[i][0], hi0 = p.need_hi[i][0];
+    const int lo1 = p.need_lo[i][1], hi1 = p.need_hi[i][1];
+    const int len0 = hi0 - lo0 + 1;
+    u64 *__restrict__ S = (u64 *)p.sat[i];
+    int *__restrict__ N = p.satN[i];
+    unsigned s0 = 0, s1 = 0, q0 = 0, q1 = 0;
+    int n0 = 0, n1 = 0;
+    unsigned char *mine = stage + ty * (2 * SATP_ROWS * SATP_PITCH);
+    const unsigned mine_s = (unsigned)__cvta_generic_to_shared(mine);
+    // rows [y, y + SATP_ROWS) of the segment -> buffer b, each from the 16-byte
+    // boundary at or below its first byte (a block that holds a byte of the row
+    // never leaves the row's allocation)
+    auto fetch = [&](int y, int b) {
+        const int rows = min(SATP_ROWS, y1 - y);
+        for (int e = tx; e < 5 * rows; e += 32) {
+            const int r = e / 5, k = e - 5 * r;
+            const unsigned char *a = band + (y + r) * st;
+            const int off = (int)((uintptr_t)a & 15);
+            if (16 * k < off + nb)
+                cp_async16(mine_s + (b * SATP_ROWS + r) * SATP_PITCH + 16 * k, a - off + 16 * k);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (y0 < y1)
+        fetch(y0, 0);
+    int buf = 0;
+    for (int yb = y0; yb < y1; yb += SATP_ROWS, buf ^= 1) {
+        if (yb + SATP_ROWS < y1) {
+            fetch(yb + SATP_ROWS, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        const unsigned char *src = mine + buf * SATP_ROWS * SATP_PITCH;
+        // the bytes of columns c, c + 1 in row y of the block
+        auto load2 = [&](int y) -> unsigned {
+            const unsigned at = ((unsigned)(uintptr_t)band + (unsigned)(y * st) & 15u) + 2 * tx;
+            const unsigned odd = at & 1u;
+            const unsigned short *b =
+                (const unsigned short *)(src + (y - yb) * SATP_PITCH + (at - odd));
+            const unsigned lo = b[0], hi = odd && two ? (unsigned)b[1] : 0u;
+            return (lo | hi << 16) >> (8 * odd);
+        };
+        const int ye = min(y1, yb + SATP_ROWS);
+        int y = cok ? yb : ye;
+        while (y < ye) {
+            int stop = ye;   // next needed row at or after y
+            if (hi0 >= lo0 && hi0 >= y)
+                stop = min(stop, max(lo0, y));
+            if (hi1 >= lo1 && hi1 >= y)
+                stop = min(stop, max(lo1, y));
+#pragma unroll 2
+            for (; y + 4 <= stop; y += 4) {
+                const unsigned r0 = load2(y), r1 = load2(y + 1), r2 = load2(y + 2),
+                               r3 = load2(y + 3);
+                const unsigned a = __byte_perm(r0, r1, 0x5140), b = __byte_perm(r2, r3, 0x5140);
+                const unsigned t0 = __byte_perm(a, b, 0x5410), t1 = __byte_perm(a, b, 0x7632);
+                s0 = __dp4a(t0, 0x01010101u, s0);
+                s1 = __dp4a(t1, 0x01010101u, s1);
+                q0 = __dp4a(t0, t0, q0);
+                q1 = __dp4a(t1, t1, q1);
+                if (COUNT) {
+                    n0 += __popc(__vcmpne4(t0, 0u)) >> 3;
+                    n1 += __popc(__vcmpne4(t1, 0u)) >> 3;
+                }
+            }
+            for (; y < stop; ++y) {
+                const unsigned v = load2(y), a = v & 0xffu, b = v >> 8 & 0xffu;
+                s0 += a;
+                s1 += b;
+                q0 += a * a;
+                q1 += b * b;
+                if (COUNT) {
+                    n0 += a != 0;
+                    n1 += b != 0;
+                }
+            }
+            if (y >= ye)
+                break;
+            // needed run: rows y .. end of its interval (within the block)
+            const bool first = y >= lo0 && y <= hi0;
+            const int rend = min(ye - 1, first ? hi0 : hi1);
+            const long long base = first ? (long long)(y - lo0) : (long long)(len0 + y - lo1);
+#pragma unroll 4
+            for (long long o = base * sp + c; y <= rend; ++y, o += sp) {
+                const unsigned v = load2(y), a = v & 0xffu, b = v >> 8 & 0xffu;
+                s0 += a;
+                s1 += b;
+                q0 += a * a;
+                q1 += b * b;
+                // sums of u = v - 128 over the m rows so far
+                const int m = y - y0 + 1;
+                ulonglong2 e;
+                e.x = sat_pack((int)s0 - 128 * m, q0 - 256u * s0 + 16384u * m);
+                e.y = sat_pack((int)s1 - 128 * m, q1 - 256u * s1 + 16384u * m);
+                *(ulonglong2 *)(S + o) = e;   // sp is even: aligned, inside the row
+                if (COUNT) {
+                    n0 += a != 0;
+                    n1 += b != 0;
+                    *(int2 *)(N + o) = make_int2(n0, n1);
+                }
+            }
+        }
+        __syncwarp();   // this buffer is copied into again two blocks on
+    }
+    const int m = y1 - y0;
+    shP[ty * 64 + 2 * tx] = sat_pack((int)s0 - 128 * m, q0 - 256u * s0 + 16384u * m);
+    shP[ty * 64 + 2 * tx + 1] = sat_pack((int)s1 - 128 * m, q1 - 256u * s1 + 16384u * m);
+    if (COUNT) {
+        shN[ty * 64 + 2 * tx] = n0;
+        shN[ty * 64 + 2 * tx + 1] = n1;
+    }
+    __syncthreads();
+    if (!cok)
+        return;
+    ulonglong2 os = make_ulonglong2(0, 0);
+    int2 on = make_int2(0, 0);
+    for (int g = 0; g < ty; ++g) {
+        os.x += shP[g * 64 + 2 * tx];
+        os.y += shP[g * 64 + 2 * tx + 1];
+        if (COUNT) {
+            on.x += shN[g * 64 + 2 * tx];
+            on.y += shN[g * 64 + 2 * tx + 1];
+        }
+    }
+    *(ulonglong2 *)((u64 *)p.seg[i] + (long long)ty * sp + c) = os;
+    if (COUNT)
+        *(int2 *)(p.segN[i] + (long long)ty * sp + c) = on;
+    if (ty == SAT_WARPS - 1) {   // column totals of v
+        p.colsum[i][c] =
+            (double)(sat_pack_s(os.x + shP[ty * 64 + 2 * tx]) + 128 * h);
+        if (two)
+            p.colsum[i][c + 1] =
+                (double)(sat_pack_s(os.y + shP[ty * 64 + 2 * tx + 1]) + 128 * h);
+    }
+}
+
+// Chunks whose jobs all have packed tables: grid (ceil(max w / 64), 2 * npairs),
+// satp_smem() bytes of dynamic shared memory.
+__global__ void __launch_bounds__(32 * SAT_WARPS, 2) k3_satp(PairDev *pairs)
+{
+    extern __shared__ __align__(16) unsigned char satp_stage[];
+    __shared__ unsigned long long shP[64 * SAT_WARPS];
+    __shared__ int shN[64 * SAT_WARPS];
+    const PairDev &p = pairs[blockIdx.y >> 1];
+    const int i = blockIdx.y & 1;
+    if (p.status != 0 || blockIdx.x * 64 >= p.w[i])
+        return;
+    if (p.cnt_kind == ALN_CNT_GT)
+        sat_cols_packed<true>(p, i, satp_stage, shP, shN);
+    else
+        sat_cols_packed<false>(p, i, satp_stage, shP, shN);
 }
 
 __global__ void k3_sat(PairDev *pairs)
@@ -410,8 +598,8 @@ __device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, 
     const int w = p.w[i];
     const int seg = sat_seg_of(p, i, y);
     const typename SP::type *__restrict__ o =
-        (const typename SP::type *)p.seg[i] + (long long)seg * w;
-    typename SP::type *__restrict__ r = (typename SP::type *)p.sat[i] + (long long)slot * w;
+        (const typename SP::type *)p.seg[i] + (long long)seg * p.sp[i];
+    typename SP::type *__restrict__ r = (typename SP::type *)p.sat[i] + (long long)slot * p.sp[i];
     TA cs = 0, cq = 0;
     for (int c0 = 0; c0 < w; c0 += 32 * K) {
         const int c = c0 + K * lane;
@@ -443,6 +631,42 @@ __device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, 
     }
 }
 
+// Packed tables: two entries (16 bytes) per lane, one scan per 64 columns.
+__device__ __forceinline__ void sat2_row_packed(const PairDev &p, int i, int slot, int y, int lane)
+{
+    typedef unsigned long long u64;
+    const int w = p.w[i], sp = p.sp[i];
+    const ulonglong2 *__restrict__ o =
+        (const ulonglong2 *)((const u64 *)p.seg[i] + (long long)sat_seg_of(p, i, y) * sp);
+    ulonglong2 *__restrict__ r = (ulonglong2 *)((u64 *)p.sat[i] + (long long)slot * sp);
+    u64 carry = 0;
+    constexpr int K = 4;   // steps whose loads are in flight together
+    for (int c0 = 0; c0 < sp; c0 += 64 * K) {
+        ulonglong2 e[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int c = c0 + 64 * k + 2 * lane;
+            e[k] = make_ulonglong2(0, 0);
+            if (c < sp) {
+                const ulonglong2 a = r[c >> 1], b = __ldg(o + (c >> 1));
+                e[k].x = a.x + b.x;
+                e[k].y = c + 1 < w ? a.y + b.y : 0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (c0 + 64 * k >= sp)
+                break;   // uniform over the warp
+            const int c = c0 + 64 * k + 2 * lane;
+            const u64 t = warp_incl_scan(e[k].x + e[k].y, lane) + carry;
+            const u64 x = t - e[k].y;   // modulo 2^64: exact
+            carry = __shfl_sync(0xffffffff, t, 31);
+            if (c < sp)
+                r[c >> 1] = make_ulonglong2(x, t);
+        }
+    }
+}
+
 // Counts-only form (CorrImagesS without a mincor): K rounds of 32 columns
 // per pass, their loads issued together (one memory latency per pass), then
 // scanned in registers in column order.  (Measured on the thumbnail sweep:
@@ -454,8 +678,8 @@ __device__ __forceinline__ void sat2_row_counts(const PairDev &p, int i, int slo
     constexpr int K = 8;
     const int w = p.w[i];
     const int seg = sat_seg_of(p, i, y);
-    const int *__restrict__ oN = p.segN[i] + (long long)seg * w;
-    int *__restrict__ rN = p.satN[i] + (long long)slot * w;
+    const int *__restrict__ oN = p.segN[i] + (long long)seg * p.sp[i];
+    int *__restrict__ rN = p.satN[i] + (long long)slot * p.sp[i];
     int cn = 0;
     for (int cb = 0; cb < w; cb += 32 * K) {
         int vn[K];
@@ -495,7 +719,9 @@ __global__ void k2_sat2w(PairDev *pairs)
         sat2_row_counts(p, i, slot, y, lane);
     if (NONLY || p.sat_nonly)
         return;
-    if (int_pixels(p.dt[i]))
+    if (p.sat_packed)
+        sat2_row_packed(p, i, slot, y, lane);
+    else if (int_pixels(p.dt[i]))
         sat2_row_any<long long>(p, i, slot, y, lane);
     else
         sat2_row_any<double>(p, i, slot, y, lane);
@@ -1066,6 +1292,57 @@ k2_lagrow(PairDev *pairs, const float2 *__restrict__ tw)
 // uneven pairs 7.3 -> 4.7 ms, 48 pairs of 512^2 over all lags 1120 -> 752 us.
 #define LAGSCAN_ROWS 8
 
+// The lags xa + lane, xa + lane + 32, ... <= xb of one row of an integer pair:
+// the best FP32 r and its storage index.  KIND: 0 packed tables, 1 int64
+// pairs with sums below 2^31, 2 int64 pairs; CHECK: a legality table or a
+// count rule is looked up too.  The body has no branch and reads past the
+// row's end at xb again, so that the unrolled loop's loads are in flight
+// together: with a branch per lag the scan waited for them one lag at a time.
+template <int KIND, bool CHECK>
+__device__ __forceinline__ void scan_row_int(const PairDev &p, const LagRow &q, int xa, int xb,
+                                             int y, long long in, int key0, float &br, int &bk)
+{
+    typedef unsigned long long u64;
+    const int lane = threadIdx.x & 31, ox = p.ox, Nx = p.Nx;
+    const int m1 = (int)p.mu[0] - (KIND == 0 ? 128 : 0), m2 = (int)p.mu[1] - (KIND == 0 ? 128 : 0);
+    // 1 / (Nx Ny): exact for power-of-two grids; on the split lengths one
+    // more FP32 rounding, below the transform's own error
+    const float invf = 1.0f / ((float)Nx * (float)p.Ny);
+    const float *__restrict__ row =
+        (const float *)p.rr + (long long)(y - p.ylo) * (p.xhi - p.xlo + 1) - p.xlo;
+    const void *t1 = p.sat[0], *t2 = p.sat[1];
+#pragma unroll 2
+    for (int x0 = xa; x0 <= xb; x0 += 32) {
+        const int x = min(x0 + lane, xb);
+        const int L2 = max(0, x), R2 = max(min(q.w2 - 1, x + q.w1 - 1), L2);
+        const int olw = R2 - L2 + 1, n = olw * q.olh;
+        const float cs = __ldg(row + x) * invf;
+        float r;
+        if (KIND == 0) {
+            const u64 a = row_box_p((const u64 *)t1, q.oT[0], q.oB[0], L2 - x, R2 - x);
+            const u64 b = row_box_p((const u64 *)t2, q.oT[1], q.oB[1], L2, R2);
+            const int s1 = sat_pack_s(a), s2 = sat_pack_s(b);
+            r = r_int32(n, cs, s1, sat_pack_q(a, s1), s2, sat_pack_q(b, s2), m1, m2);
+        } else {
+            const longlong2 a = row_box2((const longlong2 *)t1, q.oT[0], q.oB[0], L2 - x, R2 - x);
+            const longlong2 b = row_box2((const longlong2 *)t2, q.oT[1], q.oB[1], L2, R2);
+            r = KIND == 1 ? r_int32(n, cs, (int)a.x, a.y, (int)b.x, b.y, m1, m2)
+                          : r_int(n, cs, a.x, a.y, b.x, b.y, m1, m2);
+        }
+        const int dx = x - ox;
+        bool ok = olw >= q.omin && olw <= q.omax && (long long)dx * dx <= in;
+        if (CHECK && ok) {
+            int l, h;
+            ok = lag_row_legal(p, q, x, l, h);
+        }
+        const int k = key0 + (x < 0 ? x + Nx : x);
+        if (ok && (r > br || (r == br && k < bk))) {
+            br = r;
+            bk = k;
+        }
+    }
+}
+
 // grid (ceil(max Wy / LAGSCAN_ROWS), npairs), block 32 * LAGSCAN_ROWS
 __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
 {
@@ -1082,38 +1359,27 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
     // (an FP64 square root per row cost more than the test)
     const int xr = in < 0 ? -1 : (int)sqrtf(__uint2float_rn((unsigned)min(in, 1ll << 30))) + 2;
     const int xa = max(p.xlo, ox - xr), xb = xr < 0 ? xa - 1 : min(p.xhi, ox + xr);
-    const float *__restrict__ row =
-        (const float *)p.rr + (long long)j * (p.xhi - p.xlo + 1) - p.xlo;
-    // 1 / (Nx Ny): exact for power-of-two grids; on the split lengths one
-    // more FP32 rounding, below the transform's own error
-    const float invf = 1.0f / ((float)Nx * (float)Ny);
     const LagRow q = lag_row(p, y);
     const int key0 = (y < 0 ? y + Ny : y) * Nx;   // storage indices are < 2^26
-    const int nmax = min(p.w[0], p.w[1]) * q.olh;   // largest overlap of the row
+    const int nmax = min(q.w1, q.w2) * q.olh;     // largest overlap of the row
     if (r_int_ok(p, nmax)) {
         // every lag of the row takes r_int: FP32 keys
-        const longlong2 *t1 = (const longlong2 *)p.sat[0], *t2 = (const longlong2 *)p.sat[1];
-        const int m1 = (int)p.mu[0], m2 = (int)p.mu[1];
-        const bool narrow =
-            nmax < (p.dt[0] == ALN_U8 && p.dt[1] == ALN_U8 ? 1 << 23 : 1 << 15);
+        const bool check = q.tbl || q.cnt;
+        const bool narrow = nmax < (1 << 15) ||
+                            (p.dt[0] == ALN_U8 && p.dt[1] == ALN_U8 && nmax < (1 << 23));
         float br = -1.0e30f;
         int bk = 0x7fffffff;
-        for (int x = xa + lane; x <= xb; x += 32) {
-            const long long dx = x - ox;
-            int L2, R2;
-            if (dx * dx > in || !lag_row_legal(p, q, x, L2, R2))
-                continue;
-            const int n = (R2 - L2 + 1) * q.olh;
-            const float cs = __ldg(row + x) * invf;
-            const longlong2 a = row_box2(t1, q.oT[0], q.oB[0], L2 - x, R2 - x);
-            const longlong2 b = row_box2(t2, q.oT[1], q.oB[1], L2, R2);
-            const float r = narrow ? r_int32(n, cs, (unsigned)a.x, a.y, (unsigned)b.x, b.y, m1, m2)
-                                   : r_int(n, cs, a.x, a.y, b.x, b.y, m1, m2);
-            const int k = key0 + (x < 0 ? x + Nx : x);
-            if (r > br || (r == br && k < bk)) {
-                br = r;
-                bk = k;
-            }
+        if (p.sat_packed) {
+            if (check)
+                scan_row_int<0, true>(p, q, xa, xb, y, in, key0, br, bk);
+            else
+                scan_row_int<0, false>(p, q, xa, xb, y, in, key0, br, bk);
+        } else if (check) {
+            scan_row_int<2, true>(p, q, xa, xb, y, in, key0, br, bk);
+        } else if (narrow) {
+            scan_row_int<1, false>(p, q, xa, xb, y, in, key0, br, bk);
+        } else {
+            scan_row_int<2, false>(p, q, xa, xb, y, in, key0, br, bk);
         }
         for (int o = 16; o > 0; o >>= 1) {
             const float r2 = __shfl_down_sync(0xffffffff, br, o);
@@ -1129,6 +1395,9 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
         }
         return;
     }
+    const float invf = 1.0f / ((float)Nx * (float)Ny);
+    const float *__restrict__ row =
+        (const float *)p.rr + (long long)j * (p.xhi - p.xlo + 1) - p.xlo;
     double br = -1.0e30;
     long long bk = 0x7fffffffffffffffLL;
     for (int x = xa + lane; x <= xb; x += 32) {

@@ -1,0 +1,111 @@
+"""The lag scan's tables and legality (k3_satp, k2_sat2w, k2_lagscan).
+
+uint8 pairs whose overlaps fit take packed tables, the same pixels as uint16
+take 64-bit pairs; both hold exact integers, so the two calls give the same
+numbers bit for bit.  A LegalRgn rule tabulated by the caller is looked up per
+lag, the typed rule becomes a range of box widths per lag row: the same again.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import alignment_projects_gb300 as aln
+    c = aln.Context(0)
+    c.set_tuning(False)   # one column plan for both pixel types
+    yield c
+    c.close()
+
+
+def _pair(rng, w, h, extreme=False, zeros=0.0):
+    big = rng.integers(0, 256, (h + 8, w + 8))
+    if extreme:
+        big = np.where(big < 128, 0, 255)
+    big[rng.random(big.shape) < zeros] = 0
+    a = big[4:4 + h, 4:4 + w]
+    ty, tx = (int(v) for v in rng.integers(-3, 4, 2))
+    b = big[4 + ty:4 + ty + h, 4 + tx:4 + tx + w]
+    return a.astype(np.uint8), b.astype(np.uint8)
+
+
+def _view(t, col, pitch):
+    """The same raster on the device inside a wider one, at column col."""
+    import torch
+    host = torch.from_numpy(t)
+    big = torch.zeros((t.shape[0], pitch), dtype=host.dtype, device="cuda")
+    big[:, col:col + t.shape[1]] = host.cuda()
+    return big[:, col:col + t.shape[1]]
+
+
+@pytest.mark.parametrize("w,h,radius,cnt", [
+    (8, 9, 4096, 0), (17, 40, 4096, 0), (63, 65, 20, 0), (64, 64, 4096, 1), (65, 130, 4096, 1),
+    (127, 500, 30, 0), (235, 700, 64, 0), (129, 33, 4096, 1), (700, 130, 64, 1),
+    (300, 301, 4096, 0)])
+def test_packed_tables_equal_wide_ones(ctx, w, h, radius, cnt):
+    import alignment_projects_gb300 as aln
+    rng = np.random.default_rng(w * 1000 + h)
+    jobs = []
+    for k in range(4):
+        a, b = _pair(rng, w, h, extreme=k == 1, zeros=0.3 if cnt else 0.0)
+        lg = aln.legal(aln.RGN_MIN, min(5, w), min(5, h), 0,
+                       aln.CNT_GT if cnt else aln.CNT_NONE, w * h // 10)
+        col, pitch = (0, w) if k < 2 else (k - 1, w + 5 + k)   # odd starts and strides
+        jobs.append([dict(a=_view(x, col, pitch), b=_view(y, col, pitch), radius=radius, legal=lg)
+                     for x, y in ((a, b), (a.astype(np.uint16), b.astype(np.uint16)))])
+    got8 = ctx.corr_patches_batch([j[0] for j in jobs])
+    got16 = ctx.corr_patches_batch([j[1] for j in jobs])
+    assert got8 == got16
+    assert any(g["status"] == aln.ALN_OK for g in got8)
+
+
+@pytest.mark.parametrize("w,h", [(1448, 1448), (1449, 1448)])
+def test_packing_limit(ctx, w, h):
+    """Overlaps just below 2^21 pixels (packed) and just above (not)."""
+    rng = np.random.default_rng(w)
+    a, b = _pair(rng, w, h, extreme=True)
+    one = dict(radius=6)
+    got = [ctx.corr_patches_batch([dict(a=x, b=y, **one)])[0]
+           for x, y in ((a, b), (a.astype(np.uint16), b.astype(np.uint16)))]
+    # 16-bit overlaps from 2^20 pixels take the FP64 formula for r
+    assert abs(got[0]["r"] - got[1]["r"]) < 1e-6
+    assert (got[0]["peak_x"], got[0]["peak_y"]) == (got[1]["peak_x"], got[1]["peak_y"])
+    white = np.full((h, w), 255, np.uint8)
+    white[::7, ::5] = 0
+    g = ctx.corr_patches_batch([dict(a=white, b=white, **one)])[0]
+    # every lag of the pattern's period (5, 7) matches exactly
+    assert (g["peak_x"] % 5, g["peak_y"] % 7) == (0, 0) and abs(g["r"] - 1) < 1e-5
+
+
+def _rule(kind, sx, sy, a, b, area):
+    import alignment_projects_gb300 as aln
+    if kind == aln.RGN_MIN:
+        return (sx >= a) & (sy >= b) & (sx * sy > area)
+    if kind == aln.RGN_SECTION:
+        return (sx * sy > area) & ((sx >= a) | (sy > b))
+    return (sx == a) & (sy == b)
+
+
+@pytest.mark.parametrize("w,h", [(60, 90), (110, 70)])   # as is, and solved transposed
+@pytest.mark.parametrize("kind,a,b,area", [
+    (1, 20, 30, 0), (1, 0, 0, 1500), (1, 55, 61, 3000), (1, 7, 9, -5), (1, 10, 10, 1 << 40),
+    (2, 30, 45, 1200), (2, 0, 80, 2000), (2, 200, 200, 0), (2, 52, 0, 900), (3, 47, 66, 0),
+    (3, 500, 1, 0)])
+def test_typed_rule_equals_its_table(ctx, w, h, kind, a, b, area):
+    import alignment_projects_gb300 as aln
+    rng = np.random.default_rng(w + a + b)
+    sx, sy = np.meshgrid(np.arange(1, w + 1), np.arange(1, h + 1))
+    table = _rule(kind, sx, sy, a, b, area).astype(np.uint8)
+    A, B = _pair(rng, w, h)
+    for dt in (np.uint8, np.uint16, np.float32):
+        x, y = A.astype(dt), B.astype(dt)
+        got = ctx.corr_patches_batch([
+            dict(a=x, b=y, radius=40, legal=aln.legal(kind, a, b, area)),
+            dict(a=x, b=y, radius=40, legal=aln.legal(table=table))])
+        assert got[0] == got[1], dt
+        imgs = ctx.corr_images_batch([
+            dict(kind=aln.CORR_R, a=x, b=y, legal=aln.legal(kind, a, b, area)),
+            dict(kind=aln.CORR_R, a=x, b=y, legal=aln.legal(table=table))])
+        assert imgs[0] == imgs[1], dt
