@@ -1025,10 +1025,10 @@ __host__ __device__ constexpr int corrseg_radix()
     return NS == 512 ? 8 : fft_radix(NS);
 }
 
-// Where a thread keeps its parked a-spectrum points and the column's
-// accumulated product: registers at radix <= 8 (each thread owns the same R
-// points throughout; a third fewer shared-memory wavefronts than parking
-// them in shared memory, 2 CTAs per SM at 128 registers instead of 3 at 80:
+// Where a thread keeps its a-spectrum points and the column's accumulated
+// product: registers at radix <= 8 (each thread owns the same R points
+// throughout; a third fewer shared-memory wavefronts than parking them in
+// shared memory, 2 CTAs per SM at 128 registers instead of 3 at 80:
 // k2_corrseg<512> 10.18 -> 9.84 ms per montage step), shared memory at
 // radix 16 (32 more points per thread spilled 260-280 bytes).
 template <int NS>
@@ -1059,7 +1059,7 @@ k2_corrseg(PairDev *pairs, const float2 *__restrict__ tw)
     const int kxc = live ? kx : L1 - 1;   // idle teams compute a copy, store nothing
     float2 *sm = smem + team * FF::SMEM;
     constexpr bool REGS = corrseg_regs<NS>();
-    float2 parkr[REGS ? R : 1], accr[REGS ? R : 1];
+    float2 accr[REGS ? R : 1];
     float2 *park = REGS ? nullptr : smem + G * FF::SMEM + team * (2 * NS);
     float2 *acc = REGS ? nullptr : park + NS;
     const float2 *Ta = p.T[0] + (long long)kxc * p.Ts[0];
@@ -1070,33 +1070,40 @@ k2_corrseg(PairDev *pairs, const float2 *__restrict__ tw)
     const int lb = B + Wy - 1;
     for (int s = 0; s < nseg; ++s) {
         const int y0 = s * B;
-        float2 v[R];
+        // b's loads are in flight while a is transformed: at radix 8 they take
+        // the registers that a's spectrum holds while b is transformed (waiting
+        // for each load in turn left the warps on the long scoreboard, 2.7 stalled
+        // per issue: 4096 strips 9.50 -> 8.97 ms)
+        float2 va[R], vb[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int j = t + r * T, y = y0 + j;
-            v[r] = (j < B && y < ha) ? Ta[y] : make_float2(0.f, 0.f);
+            va[r] = (j < B && y < ha) ? Ta[y] : make_float2(0.f, 0.f);
         }
-        FF::run_team(v, sm, t, tw, team);
+        auto load_b = [&]() {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if constexpr (REGS)
-                parkr[r] = v[r];
-            else
-                park[r * T + t] = v[r];
-        }
+            for (int r = 0; r < R; ++r) {
+                const int j = t + r * T, y = y0 + ylo + j;
+                vb[r] = (j < lb && y >= 0 && y < hb) ? Tb[y] : make_float2(0.f, 0.f);
+            }
+        };
+        if constexpr (REGS)
+            load_b();
+        FF::run_team(va, sm, t, tw, team);
+        if constexpr (!REGS) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int j = t + r * T, y = y0 + ylo + j;
-            v[r] = (j < lb && y >= 0 && y < hb) ? Tb[y] : make_float2(0.f, 0.f);
+            for (int r = 0; r < R; ++r)
+                park[r * T + t] = va[r];
+            load_b();
         }
-        FF::run_team(v, sm, t, tw, team);
+        FF::run_team(vb, sm, t, tw, team);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if constexpr (REGS) {
-                const float2 q = cmulc(v[r], parkr[r]);   // X2 * conj(X1)
+                const float2 q = cmulc(vb[r], va[r]);   // X2 * conj(X1)
                 accr[r] = s == 0 ? q : cadd(accr[r], q);
             } else {
-                const float2 q = cmulc(v[r], park[r * T + t]);
+                const float2 q = cmulc(vb[r], park[r * T + t]);
                 acc[r * T + t] = s == 0 ? q : cadd(acc[r * T + t], q);
             }
         }
