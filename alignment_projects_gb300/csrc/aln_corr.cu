@@ -2113,6 +2113,15 @@ static size_t carve(PairPlan &pl, char *base, const aln_pair &P)
     return (size_t)(p - base);
 }
 
+static int sm_count(aln_ctx *ctx)
+{
+    if (!ctx->sms) {
+        cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        ctx->sms = std::max(ctx->sms, 1);
+    }
+    return ctx->sms;
+}
+
 static int rows_per_cta(int L) { return std::max(1, std::min(16, 4096 / L)); }
 static int cols_per_cta(int Ny) { return std::max(1, std::min(16, 4096 / Ny)); }
 
@@ -2201,12 +2210,8 @@ template <int NS>
 static void launch_corrseg(aln_ctx *ctx, int n, int L)
 {
     constexpr int T = NS / corrseg_radix<NS>(), GMAX = 256 / T;
-    if (!ctx->sms) {
-        cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
-        ctx->sms = std::max(ctx->sms, 1);
-    }
     int G = GMAX;
-    while (G > 1 && (long long)((L + 1 + G - 1) / G) * n < 2LL * ctx->sms)
+    while (G > 1 && (long long)((L + 1 + G - 1) / G) * n < 2LL * sm_count(ctx))
         G /= 2;
     // float2 per team: k2_corrseg's exchange buffer (FF::SMEM), then the parked
     // spectrum and accumulator when they are not held in registers
@@ -2244,11 +2249,23 @@ template <int LL>
 static void launch_lagimg2(aln_ctx *ctx, int n, int maxWy, bool both, bool sonly)
 {
     constexpr int T = RegFFT<LL, +1>::T;
-    const int thr = std::max(256, T), G = thr / T;
+    constexpr int thr = T > 256 ? T : 256, G = thr / T;
+    static_assert(thr == 256, "k2_lagss's block");
+    const int groups = (maxWy + G - 1) / G;
+    if (sonly) {
+        // several row groups per CTA (each copies the next one's rows while it
+        // works) once the chip has four rounds of three CTAs per SM
+        const long long full = 12LL * sm_count(ctx);
+        const int per = (int)std::max(1LL, std::min(8LL, (long long)groups * n / full));
+        const size_t sm = (size_t)G * lag_pitch<LL>() * 2 * sizeof(float2);
+        smem_attr(ctx->device, (const void *)k2_lagss<LL>, sm);
+        LAUNCH(ctx, "k2_lagimg", k2_lagss<LL>, dim3((groups + per - 1) / per, n), thr, sm,
+               ctx->dpairs, ctx->tw);
+        return;
+    }
     const size_t sm = (size_t)G * lag_pitch<LL>() * (both ? 2 : 1) * sizeof(float2);
-    void (*kern)(PairDev *, const float2 *) = sonly ? k2_lagimg<LL, true> : k2_lagimg<LL, false>;
-    smem_attr(ctx->device, (const void *)kern, sm);
-    LAUNCH(ctx, "k2_lagimg", kern, dim3((maxWy + G - 1) / G, n), thr, sm, ctx->dpairs, ctx->tw);
+    smem_attr(ctx->device, (const void *)k2_lagimg<LL>, sm);
+    LAUNCH(ctx, "k2_lagimg", k2_lagimg<LL>, dim3(groups, n), thr, sm, ctx->dpairs, ctx->tw);
 }
 
 #define ALN_CASES_L(X) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
