@@ -793,6 +793,24 @@ k2_rowfft(PairDev *pairs, const float2 *__restrict__ tw, int only_img, const int
             }
             v[q] = z;
         }
+    } else if (dt == ALN_F32) {
+        // the shift is an FP32 number (k_mean), and the FP64 difference of two
+        // FP32 numbers rounds to FP32 as the FP32 difference does: no FP64
+        // instruction (they held this kernel's sweep rows at 50 % of that pipe)
+        const float mu = (float)p.mu[i];
+        const float *row = (const float *)img + y * st;
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            const int xa = 2 * F::in_idx(t, q), xb = xa + 1;
+            float2 z = make_float2(0.f, 0.f);
+            if (y < h) {
+                if (xa < w)
+                    z.x = __fsub_rn(__ldg(row + xa), mu);
+                if (xb < w)
+                    z.y = __fsub_rn(__ldg(row + xb), mu);
+            }
+            v[q] = z;
+        }
     } else {
         const double mu = p.mu[i];
 #pragma unroll
