@@ -2183,8 +2183,9 @@ static void launch_corrcol_var(aln_ctx *ctx, int n, int L, int cached)
     constexpr int T = NY / corrcol_radix<NY, VAR>();
     constexpr int thr = corrcol_threads<NY, VAR>(), G = thr / T;
     // per team: k2_corrcol's exchange buffer (FF::SMEM) and b's spectrum (NY)
-    const size_t sm =
-        (size_t)G * (RegFFT<NY, -1, corrcol_radix<NY, VAR>()>::SMEM + NY) * sizeof(float2);
+    const size_t sm = (size_t)G *
+                      (RegFFT<NY, -1, corrcol_radix<NY, VAR>()>::SMEM + (VAR == 3 ? 0 : NY)) *
+                      sizeof(float2);
     void (*kern)(PairDev *, const float2 *, int) = k2_corrcol<NY, VAR>;
     smem_attr(ctx->device, (const void *)kern, sm);
     LAUNCH(ctx, "k2_corrcol", kern, dim3((L + 1 + G - 1) / G, n), thr, sm, ctx->dpairs, ctx->tw,
@@ -2198,6 +2199,8 @@ static void launch_corrcol2(aln_ctx *ctx, int n, int L, int cached, int var)
         launch_corrcol_var<NY, 1>(ctx, n, L, cached);
     else if (var == 2)
         launch_corrcol_var<NY, 2>(ctx, n, L, cached);
+    else if (var == 3)
+        launch_corrcol_var<NY, 3>(ctx, n, L, cached);
     else
         launch_corrcol_var<NY, 0>(ctx, n, L, cached);
 }
@@ -2275,7 +2278,7 @@ static void launch_lagimg2(aln_ctx *ctx, int n, int maxWy, bool both, bool sonly
 // lag rows.  L = Nx/2 in [16, 4096], Ny in [16, 8192].
 static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int maxWy,
                                int mode = JOB_PATCHES, bool both = false, bool sonly = false,
-                               bool seg = false)
+                               bool seg = false, bool cached = false)
 {
     switch (L) {
 #define X(v) case v: launch_rowfft2<v>(ctx, n, maxh); break;
@@ -2284,6 +2287,7 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
 #undef X
     default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "row length %d", L);
     }
+    const int var = mode == JOB_PATCHES ? 1 : !sonly ? 0 : cached ? 3 : 2;
     if (seg) {
         switch (Ny) {
 #define X(v) case v: launch_corrseg<v>(ctx, n, L); break;
@@ -2292,7 +2296,7 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "segment length %d", Ny);
         }
     } else switch (Ny) {
-#define X(v) case v: launch_corrcol2<v>(ctx, n, L, 0, mode == JOB_PATCHES ? 1 : sonly ? 2 : 0); break;
+#define X(v) case v: launch_corrcol2<v>(ctx, n, L, 0, var); break;
         ALN_CASES_NY(X)
 #undef X
     default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "column length %d", Ny);
@@ -2335,6 +2339,7 @@ struct ChunkLaunch {
     int Nx, Ny, mode, both, sonly, frame_nx1, frame_ny1;
     int seg;                           // CorrPatches with segmented columns
     int packed;                        // packed summed-area tables
+    int cached;                        // every job's b is a cached spectrum
     int fill_off, nfill, fill_maxh;    // spectrum-cache fills: sel[fill_off ...]
 };
 
@@ -2410,6 +2415,9 @@ static void prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, ch
     cl.frame_ny1 = chunk[0]->frame_ny1;
     cl.seg = hd[0].nseg > 0;
     cl.packed = hd[0].sat_packed;
+    cl.cached = 1;
+    for (int k = 0; k < n; ++k)
+        cl.cached &= hd[k].b_cached;
 }
 
 // The chunk's kernels on the compute stream (its job table, fill list and
@@ -2468,7 +2476,7 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
     const bool reg_path = L >= 8 && L <= 4096 && Ny >= 8 && Ny <= 8192;
     if (reg_path) {
         if (int rc = launch_fft_pipeline(ctx, L, Ny, n, cl.maxh, cl.maxWy, mode, cl.both != 0,
-                                         cl.sonly != 0, cl.seg != 0))
+                                         cl.sonly != 0, cl.seg != 0, cl.cached != 0))
             return rc;
     } else if (mode != JOB_PATCHES) {
         return set_err(ctx, ALN_ERR_UNSUPPORTED, "CorrImages FFT size %d x %d", Nx, Ny);

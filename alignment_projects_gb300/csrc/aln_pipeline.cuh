@@ -24,6 +24,17 @@
 
 __device__ __forceinline__ bool int_pixels(int dt) { return dt == ALN_U8 || dt == ALN_U16; }
 
+// asynchronous copies, global -> shared without registers
+__device__ __forceinline__ void cp_async8(void *dst_shared, const void *src_global)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_shared);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src_global) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all()
+{
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
 // s + e += x with the rounding error of the sum kept in e (Knuth's TwoSum;
 // explicit round-to-nearest operations, so nothing is contracted or reordered)
 __device__ __forceinline__ void two_sum_acc(float &s, float &e, float x)
@@ -873,8 +884,10 @@ k2_rowfft(PairDev *pairs, const float2 *__restrict__ tw, int only_img, const int
 // ---------------------------------------------------------------------------
 
 // VAR: 1 = CorrPatches chunks (plain inverse only, no low-pass, no
-// whitening), 2 = CorrImagesS without a mincor (whitened inverse only),
-// 0 = any job; the specialised forms are compiled without the other jobs'
+// whitening), 2 = CorrImagesS without a mincor (whitened inverse only), 3 = the
+// same where every job's b is a cached spectrum, read from global memory at the
+// product instead of parked in shared memory (which bounds this kernel: a fifth
+// of its wavefronts, and half of its allocation), 0 = any job; the specialised forms are compiled without the other jobs'
 // branches.
 // Per-thread radix of the column FFTs, per kernel form.  (Measured on the
 // montage batch: 8 points per thread at 4096 -- twice the threads per
@@ -896,10 +909,10 @@ __host__ __device__ constexpr int corrcol_threads()
 template <int NY, int VAR>
 __global__ void __launch_bounds__(corrcol_threads<NY, VAR>(),
                                   (NY >= 8192 || corrcol_threads<NY, VAR>() > 256) ? 1
-                                                                                 : (VAR == 2 ? 3 : 2))
+                                                                                 : (VAR >= 2 ? 3 : 2))
 k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
 {
-    constexpr bool PLAIN = VAR == 1, SONLY = VAR == 2;
+    constexpr bool PLAIN = VAR == 1, SONLY = VAR >= 2, DIRECT = VAR == 3;
     using FF = RegFFT<NY, -1, corrcol_radix<NY, VAR>()>;
     using FI = RegFFT<NY, +1, corrcol_radix<NY, VAR>()>;
     static_assert(FI::SMEM <= FF::SMEM, "the inverse runs in the forward transform's buffer");
@@ -919,7 +932,7 @@ k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
     float2 *sb = smem + G * FF::SMEM + team * NY;   // b's spectrum, this team's own slots
     const int kxc = live ? kx : L1 - 1;   // idle teams compute a copy, store nothing
     float2 va[R];
-    {
+    if constexpr (!DIRECT) {
         float2 vb[R];
         if (use_cached_b || p.b_cached) {
 #pragma unroll
@@ -950,8 +963,10 @@ k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
     }
     FF::run_team(va, sm, t, tw, team);
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-        va[r] = cmulc(sb[r * T + t], va[r]);   // X2 * conj(X1)
+    for (int r = 0; r < R; ++r) {
+        const float2 x2 = DIRECT ? __ldg(&p.X2[(long long)kxc * NY + t + r * T]) : sb[r * T + t];
+        va[r] = cmulc(x2, va[r]);   // X2 * conj(X1)
+    }
     const bool is_p2i = VAR == 0 && p.mode == JOB_P2I;
     if (is_p2i && p.p2i_filter) {
         // CorrPatchToImage's low-pass (0_GEN/Correlation.cpp:1255-1283): the
@@ -1217,16 +1232,6 @@ __device__ __forceinline__ const PairDev &stage_job(const PairDev *pairs, int j,
 // this replaces kept four per thread in flight, and the lag kernels waited on
 // them (long-scoreboard stalls, k2_lagimg 33 % warps active).  The caller's
 // __syncthreads after the call publishes the rows to the CTA.
-__device__ __forceinline__ void cp_async8(void *dst_shared, const void *src_global)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_shared);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src_global) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all()
-{
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 template <int L, int T, int G = (T >= 256 ? T : 256) / T>
 __device__ __forceinline__ void load_lag_rows(float2 *base, int stride,
                                               const float2 *__restrict__ Q, int Wy, int j0)
