@@ -73,6 +73,8 @@ struct PairDev {
     int *satN[2];                // summed-area table of (v != 0)
     int sat_int;                 // bit i: image i's table holds int64 pairs
     int sat_nonly;               // 1: only the count table N is needed (S key alone)
+    int sat_shared;              // 1: image 1's count table is the previous job's (the
+                                 // same b); its column walk and row pass are skipped
     int s_float;                 // S key alone: rr holds the FP32 correlation c,
                                  // RowBest r/ssum/ssum2 are in c units (S = c / NxNy)
     double2 *seg[2];             // per column-walk segment: exclusive column offsets

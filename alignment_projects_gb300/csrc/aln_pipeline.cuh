@@ -431,7 +431,7 @@ __global__ void k3_sat(PairDev *pairs)
     __shared__ int shN[32 * SAT_WARPS];
     const PairDev &p = pairs[blockIdx.y >> 1];
     const int i = blockIdx.y & 1;
-    if (p.status != 0 || blockIdx.x * 32 >= p.w[i])
+    if (p.status != 0 || blockIdx.x * 32 >= p.w[i] || (i == 1 && p.sat_shared))
         return;
     if (p.sat_nonly) {   // counts only (CorrImagesS without a mincor)
         if (p.cnt_kind != ALN_CNT_GT)
@@ -721,7 +721,7 @@ __global__ void k2_sat2w(PairDev *pairs)
     const PairDev &p = pairs[blockIdx.z];
     const int i = blockIdx.y;
     const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (p.status != 0 || slot >= nslots(p, i))
+    if (p.status != 0 || slot >= nslots(p, i) || (i == 1 && p.sat_shared))
         return;
     const int len0 = p.need_hi[i][0] - p.need_lo[i][0] + 1;
     const int y = slot < len0 ? p.need_lo[i][0] + slot : p.need_lo[i][1] + slot - len0;
