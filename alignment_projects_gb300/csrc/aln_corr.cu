@@ -930,9 +930,8 @@ __device__ double stored_value(const PairDev &p, int xs, int ys, bool raw)
     return r;
 }
 
-// grid (npairs), block 256; raw: see stored_value
-__global__ void k_final(PairDev *pairs, ResultDev *res, int nreal_x_is_one, int nreal_y_is_one,
-                        int raw)
+// grid (npairs), block 256; p.fin bit 2: see stored_value's raw
+__global__ void k_final(PairDev *pairs, ResultDev *res)
 {
     __shared__ double red_r[32];
     __shared__ long long red_k[32];
@@ -986,13 +985,13 @@ __global__ void k_final(PairDev *pairs, ResultDev *res, int nreal_x_is_one, int 
     // FFT-sized raster (nx, ny and the storage indices xs, ys are the
     // reference's, which may be larger than the transform grid).
     const int xs = bigx < 0 ? bigx + p.rnx : bigx, ys = bigy < 0 ? bigy + p.rny : bigy;
-    const int nx = nreal_x_is_one ? 1 : p.rnx, ny = nreal_y_is_one ? 1 : p.rny;
+    const int nx = (p.fin & 1) ? 1 : p.rnx, ny = (p.fin & 2) ? 1 : p.rny;
     const int ix = bigx, iy = bigy;
     const bool inx = ix - 1 >= 0 && ix + 1 < nx, iny = iy - 1 >= 0 && iy + 1 < ny;
     const int way = (threadIdx.x & 1) ? 1 : -1;
     if (threadIdx.x < 2 ? inx : iny)
-        near[threadIdx.x] = threadIdx.x < 2 ? stored_value(p, ix + way, ys, raw != 0)
-                                            : stored_value(p, xs, iy + way, raw != 0);
+        near[threadIdx.x] = threadIdx.x < 2 ? stored_value(p, ix + way, ys, (p.fin & 4) != 0)
+                                            : stored_value(p, xs, iy + way, (p.fin & 4) != 0);
     __syncwarp(0xf);
     if (threadIdx.x != 0)
         return;
@@ -1586,7 +1585,6 @@ struct ImgSpec {
 struct PairPlan {
     PairDev d;
     int orig_nx, orig_ny;        // the reference's FFT size (caller's frame)
-    int frame_nx1, frame_ny1;    // the solving frame's FFT size is 1 on that axis
     int transposed;
     size_t ws_bytes;
     size_t in_bytes[2];          // staging of host inputs (caller's layout)
@@ -1776,8 +1774,7 @@ static int plan_pair(aln_ctx *ctx, const aln_pair &P, PairPlan &pl, bool allow_t
         std::swap(d.ox, d.oy);
     }
     const int fnx = ceil_pow2(d.w[0] + d.w[1] - 1), fny = ceil_pow2(d.h[0] + d.h[1] - 1);
-    pl.frame_nx1 = fnx == 1;
-    pl.frame_ny1 = fny == 1;
+    d.fin = (fnx == 1 ? 1 : 0) | (fny == 1 ? 2 : 0);
     d.Nx = std::max(2, fnx);
     d.Ny = std::max(2, fny);
     if (d.Nx > ALN_MAX_N || d.Ny > ALN_MAX_N)
@@ -1819,7 +1816,7 @@ static int plan_pair(aln_ctx *ctx, const aln_pair &P, PairPlan &pl, bool allow_t
         d.logNy = ilog2(d.Ny);
         pl.orig_nx = d.Nx;
         pl.orig_ny = d.Ny;
-        pl.frame_nx1 = pl.frame_ny1 = 0;
+        d.fin = 0;
         d.p2i_filter = spec->p2i_filter;
         d.p2i_w1 = spec->p2i_w1;
         d.p2i_h1 = spec->p2i_h1;
@@ -2309,8 +2306,6 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
 #undef X
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "row length %d", L);
         }
-        LAUNCH(ctx, "k2_lagscan", k2_lagscan, dim3((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n),
-               32 * LAGSCAN_ROWS, 0, ctx->dpairs);
     } else if (mode == JOB_P2I) {
         switch (L) {
 #define X(v) case v: launch_lagp2i<v>(ctx, n, maxWy); break;
@@ -2329,38 +2324,59 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
     return ALN_OK;
 }
 
-// One chunk of jobs sharing (Nx, Ny, kind): the sizes its launches need and
-// where its jobs sit in the batch's job table.
+// The sizes that the launches over a run of jobs need, and where the jobs sit
+// in the batch's job table.
+struct JobSpan {
+    int off = 0, n = 0;                // jobs [off, off + n) of the batch table
+    int maxw = 1, maxh = 1, maxslots = 1, maxWy = 1;
+    int sw = 0, sh = 0;                // largest caller-frame image of transposed jobs
+    int t8 = 1;                        // every transposed job is uint8 (128-byte tiles)
+    int packed = 0, plain = 0;         // jobs with packed / other summed-area tables
+    void add(const JobSpan &o)
+    {
+        n += o.n;
+        maxw = std::max(maxw, o.maxw);
+        maxh = std::max(maxh, o.maxh);
+        maxslots = std::max(maxslots, o.maxslots);
+        maxWy = std::max(maxWy, o.maxWy);
+        sw = std::max(sw, o.sw);
+        sh = std::max(sh, o.sh);
+        t8 &= o.t8;
+        packed += o.packed;
+        plain += o.plain;
+    }
+};
+
+// One chunk of jobs sharing (Nx, Ny, kind): its transforms' launches.
 struct ChunkLaunch {
-    int off, n;                        // jobs [off, off + n) of the batch table
-    int maxw, maxh, maxslots, maxWy;
-    int sw, sh;                        // largest caller-frame image of transposed jobs
-    int t8;                            // every transposed job is uint8 (128-byte tiles)
-    int Nx, Ny, mode, both, sonly, frame_nx1, frame_ny1;
+    JobSpan s;
+    int Nx, Ny, mode, both, sonly;
     int seg;                           // CorrPatches with segmented columns
-    int packed;                        // packed summed-area tables
     int cached;                        // every job's b is a cached spectrum
     int fill_off, nfill, fill_maxh;    // spectrum-cache fills: sel[fill_off ...]
 };
 
+static bool register_path(int Nx, int Ny)
+{
+    return Nx / 2 >= 8 && Nx / 2 <= 4096 && Ny >= 8 && Ny <= 8192;
+}
+
 // Host side of a chunk: carve each job's workspace (the chunk's work buffer
 // is reused by every chunk, in stream order), resolve spectrum-cache keys,
 // write the job table entries hd[0..n).
-static void prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, char *work_base,
-                       PairDev *hd, std::vector<int> &fills, ChunkLaunch &cl)
+static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, char *work_base,
+                         PairDev *hd, std::vector<int> &fills, ChunkLaunch &cl)
 {
     const int n = (int)chunk.size();
-    cl.off = off;
-    cl.n = n;
-    cl.maxw = cl.maxh = cl.maxslots = cl.maxWy = 1;
-    cl.sw = cl.sh = 0;
-    cl.t8 = 1;
+    JobSpan &sp = cl.s;
+    sp.off = off;
+    sp.n = n;
     cl.Nx = chunk[0]->d.Nx;
     cl.Ny = chunk[0]->d.Ny;
     cl.fill_off = (int)fills.size();
     cl.fill_maxh = 1;
     char *work = work_base;
-    const bool reg_path = cl.Nx / 2 >= 8 && cl.Nx / 2 <= 4096 && cl.Ny >= 8 && cl.Ny <= 8192;
+    const bool reg_path = register_path(cl.Nx, cl.Ny);
     ++ctx->spec_tick;
     for (int k = 0; k < n; ++k) {
         PairPlan &pl = *chunk[k];
@@ -2390,20 +2406,20 @@ static void prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, ch
             }
         }
         for (int i = 0; i < 2; ++i) {
-            cl.maxw = std::max(cl.maxw, pl.d.w[i]);
-            cl.maxh = std::max(cl.maxh, pl.d.h[i]);
+            sp.maxw = std::max(sp.maxw, pl.d.w[i]);
+            sp.maxh = std::max(sp.maxh, pl.d.h[i]);
             int ns = 0;
             for (int q = 0; q < 2; ++q)
                 if (pl.d.need_hi[i][q] >= pl.d.need_lo[i][q])
                     ns += pl.d.need_hi[i][q] - pl.d.need_lo[i][q] + 1;
-            cl.maxslots = std::max(cl.maxslots, ns);
+            sp.maxslots = std::max(sp.maxslots, ns);
             if (pl.d.transposed) {
-                cl.sw = std::max(cl.sw, pl.d.h[i]);
-                cl.sh = std::max(cl.sh, pl.d.w[i]);
-                cl.t8 &= pl.d.dt[i] == ALN_U8;
+                sp.sw = std::max(sp.sw, pl.d.h[i]);
+                sp.sh = std::max(sp.sh, pl.d.w[i]);
+                sp.t8 &= pl.d.dt[i] == ALN_U8;
             }
         }
-        cl.maxWy = std::max(cl.maxWy, pl.d.yhi - pl.d.ylo + 1);
+        sp.maxWy = std::max(sp.maxWy, pl.d.yhi - pl.d.ylo + 1);
         pl.d.sat_int = (pl.d.dt[0] == ALN_U8 || pl.d.dt[0] == ALN_U16 ? 1 : 0) |
                        (pl.d.dt[1] == ALN_U8 || pl.d.dt[1] == ALN_U16 ? 2 : 0);
         // a sweep correlates one thumbnail b at many angles, one job after the
@@ -2420,59 +2436,81 @@ static void prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, ch
                 pl.d.satN[1] = a.satN[1];
             }
         }
+        if (pl.d.mode == JOB_PATCHES && reg_path)
+            pl.d.fin |= 4;
+        ++(pl.d.sat_packed ? sp.packed : sp.plain);
         hd[k] = pl.d;
     }
     cl.nfill = (int)fills.size() - cl.fill_off;
     cl.mode = hd[0].mode;
     cl.both = hd[0].want_r && hd[0].want_s;
     cl.sonly = hd[0].s_float != 0;
-    cl.frame_nx1 = chunk[0]->frame_nx1;
-    cl.frame_ny1 = chunk[0]->frame_ny1;
     cl.seg = hd[0].nseg > 0;
-    cl.packed = hd[0].sat_packed;
     cl.cached = 1;
     for (int k = 0; k < n; ++k)
         cl.cached &= hd[k].b_cached;
+    return (size_t)(work - work_base);
 }
 
-// The chunk's kernels on the compute stream (its job table, fill list and
-// staged inputs are already on the device, in stream order).
+// Transposes, summed-area tables and mean shifts of a span of jobs (its job
+// table, fill lists and staged inputs are already on the device, in stream
+// order).  These kernels do not depend on the transform lengths, so one launch
+// covers the chunks of several grids.
+static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *> *> &chunks,
+                         const JobSpan &sp, int mode, bool sonly)
+{
+    const int n = sp.n;
+    ctx->dpairs = ctx->dpairs_base + sp.off;
+    for (const auto *chunk : chunks)
+        for (const PairPlan *pl : *chunk)   // tabulated legality (pageable source: staged at the call)
+            if (pl->d.rgn_kind == ALN_RGN_TABLE)
+                CK(cudaMemcpyAsync((void *)pl->d.table, pl->src->legal.table,
+                                   (size_t)pl->d.table_w * pl->d.table_h, cudaMemcpyHostToDevice,
+                                   ctx->stream));
+    if (sp.sw > 0)
+        LAUNCH(ctx, "k_transpose", k_transpose,
+               dim3(sp.t8 ? (sp.sw + 128 * TR_TILES - 1) / (128 * TR_TILES)
+                          : (sp.sw + 32 * TR_TILES - 1) / (32 * TR_TILES),
+                    (sp.sh + 31) / 32, 2 * n),
+               dim3(32, 8), 0, ctx->dpairs);
+    if (mode == JOB_P2I)
+        return ALN_OK;
+    if (sp.packed) {
+        smem_attr(ctx->device, (const void *)k3_satp, satp_smem());
+        LAUNCH(ctx, "k3_sat", k3_satp, dim3((sp.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
+               satp_smem(), ctx->dpairs);
+    }
+    if (sp.plain)
+        LAUNCH(ctx, "k3_sat", k3_sat, dim3((sp.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS), 0,
+               ctx->dpairs);
+    LAUNCH(ctx, "k_mean", k_mean, dim3(2, n), 256, 0, ctx->dpairs);
+    if (sonly)
+        LAUNCH(ctx, "k2_sat2w", k2_sat2w<true>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
+               ctx->dpairs);
+    else
+        LAUNCH(ctx, "k2_sat2w", k2_sat2w<false>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
+               ctx->dpairs);
+    return ALN_OK;
+}
+
+// The lag scans and peaks of a span of CorrPatches jobs.
+static void launch_peaks(aln_ctx *ctx, const JobSpan &sp)
+{
+    ctx->dpairs = ctx->dpairs_base + sp.off;
+    LAUNCH(ctx, "k2_lagscan", k2_lagscan,
+           dim3((sp.maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, sp.n), 32 * LAGSCAN_ROWS, 0,
+           ctx->dpairs);
+    LAUNCH(ctx, "k_final", k_final, sp.n, 256, 0, ctx->dpairs, ctx->dres_base + sp.off);
+}
+
+// The chunk's transforms, and the peaks of CorrImages and CorrPatchToImage.
 static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const ChunkLaunch &cl)
 {
-    const int n = cl.n, Nx = cl.Nx, Ny = cl.Ny, L = Nx / 2;
+    const int n = cl.s.n, Nx = cl.Nx, Ny = cl.Ny, L = Nx / 2, mode = cl.mode;
     ctx->chunks++;
-    ctx->dpairs = ctx->dpairs_base + cl.off;
-    ctx->dres = ctx->dres_base + cl.off;
+    ctx->dpairs = ctx->dpairs_base + cl.s.off;
+    ctx->dres = ctx->dres_base + cl.s.off;
     ctx->dsel_cur = ctx->dsel + cl.fill_off;
-    cudaStream_t st = ctx->stream;
-    for (int k = 0; k < n; ++k)   // tabulated legality (pageable source: staged at the call)
-        if (chunk[k]->d.rgn_kind == ALN_RGN_TABLE)
-            CK(cudaMemcpyAsync((void *)chunk[k]->d.table, chunk[k]->src->legal.table,
-                               (size_t)chunk[k]->d.table_w * chunk[k]->d.table_h,
-                               cudaMemcpyHostToDevice, st));
-    if (cl.sw > 0)
-        LAUNCH(ctx, "k_transpose", k_transpose,
-               dim3(cl.t8 ? (cl.sw + 128 * TR_TILES - 1) / (128 * TR_TILES)
-                          : (cl.sw + 32 * TR_TILES - 1) / (32 * TR_TILES),
-                    (cl.sh + 31) / 32, 2 * n),
-               dim3(32, 8), 0, ctx->dpairs);
-    const int mode = cl.mode;
-    if (mode != JOB_P2I) {
-        if (cl.packed) {
-            smem_attr(ctx->device, (const void *)k3_satp, satp_smem());
-            LAUNCH(ctx, "k3_sat", k3_satp, dim3((cl.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
-                   satp_smem(), ctx->dpairs);
-        } else
-            LAUNCH(ctx, "k3_sat", k3_sat, dim3((cl.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS),
-                   0, ctx->dpairs);
-        LAUNCH(ctx, "k_mean", k_mean, dim3(2, n), 256, 0, ctx->dpairs);
-        if (cl.sonly)
-            LAUNCH(ctx, "k2_sat2w", k2_sat2w<true>, dim3((cl.maxslots + 7) / 8, 2, n), 256, 0,
-                   ctx->dpairs);
-        else
-            LAUNCH(ctx, "k2_sat2w", k2_sat2w<false>, dim3((cl.maxslots + 7) / 8, 2, n), 256,
-                   0, ctx->dpairs);
-    }
     if (cl.nfill > 0) {
         switch (L) {
 #define X(v) case v: launch_fill_rows<v>(ctx, cl.nfill, cl.fill_maxh); break;
@@ -2488,9 +2526,8 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "column length %d", Ny);
         }
     }
-    const bool reg_path = L >= 8 && L <= 4096 && Ny >= 8 && Ny <= 8192;
-    if (reg_path) {
-        if (int rc = launch_fft_pipeline(ctx, L, Ny, n, cl.maxh, cl.maxWy, mode, cl.both != 0,
+    if (register_path(Nx, Ny)) {
+        if (int rc = launch_fft_pipeline(ctx, L, Ny, n, cl.s.maxh, cl.s.maxWy, mode, cl.both != 0,
                                          cl.sonly != 0, cl.seg != 0, cl.cached != 0))
             return rc;
     } else if (mode != JOB_PATCHES) {
@@ -2499,7 +2536,7 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
         {
             const int RB = rows_per_cta(L);
             const size_t sm = 2 * (size_t)RB * (L + 1) * sizeof(float2);
-            LAUNCH(ctx, "k_rowfft", k_rowfft, dim3((cl.maxh + RB - 1) / RB, 2, n), 256, sm,
+            LAUNCH(ctx, "k_rowfft", k_rowfft, dim3((cl.s.maxh + RB - 1) / RB, 2, n), 256, sm,
                    ctx->dpairs, ctx->tw, RB, -1);
         }
         {
@@ -2512,14 +2549,11 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
         {
             const int RBL = std::max(1, std::min(8, 4096 / std::max(1, L)));
             const size_t sm = 2 * (size_t)RBL * (L + 1) * sizeof(float2);
-            LAUNCH(ctx, "k_lagrow", k_lagrow, dim3((cl.maxWy + RBL - 1) / RBL, n), 256, sm,
+            LAUNCH(ctx, "k_lagrow", k_lagrow, dim3((cl.s.maxWy + RBL - 1) / RBL, n), 256, sm,
                    ctx->dpairs, ctx->tw, RBL);
         }
     }
-    if (mode == JOB_PATCHES)
-        LAUNCH(ctx, "k_final", k_final, n, 256, 0, ctx->dpairs, ctx->dres, cl.frame_nx1,
-               cl.frame_ny1, (int)reg_path);
-    else if (mode == JOB_P2I)
+    if (mode == JOB_P2I)
         LAUNCH(ctx, "k_final_p2i", k_final_p2i, n, 256, 0, ctx->dpairs, ctx->dres);
     else if (mode == JOB_IMAGES_F) {
         int mw = 1, mh = 1;
@@ -2530,7 +2564,7 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
         LAUNCH(ctx, "k_makef", k_makef, dim3((mw + 31) / 32, (mh + 7) / 8, n), dim3(32, 8), 0,
                ctx->dpairs);
         LAUNCH(ctx, "k_fpeak", k_fpeak, n, FPK_THREADS, 0, ctx->dpairs, ctx->dres);
-    } else
+    } else if (mode != JOB_PATCHES)
         LAUNCH(ctx, "k_final_img", k_final_img, n, 256, 0, ctx->dpairs, ctx->dres);
     CK(cudaGetLastError());
     return ALN_OK;
@@ -2821,48 +2855,63 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
             sb += st;
         }
     }
-    std::vector<std::vector<std::vector<PairPlan *>>> wchunks(windows.size());
-    size_t max_stage = 0, max_work = 0, max_n = 1;
+    // Chunks of CorrPatches jobs that fit a quarter of the workspace budget
+    // together form a span: the kernels that do not depend on the transform
+    // lengths run once per span (launch_tables, launch_peaks).  A mixed batch
+    // has a chunk per grid, and each of its small launches filled the chip for a
+    // part of its time only (3000 uneven pairs: 74 chunks in 9 spans, 629 -> 323
+    // launches, 18.4 -> 16.0 ms).
+    // A quarter, so that the host prepares the next span while this one runs.
+    std::vector<std::vector<std::vector<std::vector<PairPlan *>>>> wspans(windows.size());
+    const size_t span_cap = ctx->ws_budget / 4;
+    size_t max_stage = 0, max_work = 0;
     for (size_t w = 0; w < windows.size(); ++w) {
-        std::map<std::tuple<int, int, int, int, int, int, int, int, int, int>,
-                 std::vector<PairPlan *>>
+        std::map<std::tuple<int, int, int, int, int, int, int, int>, std::vector<PairPlan *>>
             groups;
         size_t sb = 0;
         for (PairPlan *pl : windows[w]) {
-            // transposed jobs apart: their chunks alone launch the transpose;
-            // packed tables apart: they have their own column walk
-            groups[std::make_tuple(pl->d.Nx, pl->d.Ny, pl->frame_nx1, pl->frame_ny1, pl->d.mode,
-                                   pl->d.want_r, pl->d.want_s, pl->d.nseg > 0,
-                                   pl->transposed ? 1 : 0, pl->d.sat_packed)]
+            // transposed jobs and packed tables apart, so that a span of few
+            // grids launches the transpose and each column walk for its own jobs
+            groups[std::make_tuple(pl->transposed ? 1 : 0, pl->d.sat_packed, pl->d.Nx, pl->d.Ny,
+                                   pl->d.mode, pl->d.want_r, pl->d.want_s, pl->d.nseg > 0)]
                 .push_back(pl);
             sb += pl->in_bytes[0] + pl->in_bytes[1] + 16;
         }
         max_stage = std::max(max_stage, sb);
+        size_t span_bytes = 0, span_jobs = 0;
+        auto put = [&](std::vector<PairPlan *> &chunk, size_t wb) {
+            auto &spans = wspans[w];
+            const bool more = !spans.empty() && chunk[0]->d.mode == JOB_PATCHES &&
+                              spans.back()[0][0]->d.mode == JOB_PATCHES &&
+                              span_bytes + wb <= span_cap && span_jobs + chunk.size() <= 16384;
+            if (!more) {
+                spans.emplace_back();
+                span_bytes = span_jobs = 0;
+            }
+            spans.back().push_back(std::move(chunk));
+            span_bytes += wb;
+            span_jobs += spans.back().back().size();
+            max_work = std::max(max_work, span_bytes);
+            chunk.clear();
+        };
         for (auto &g : groups) {
             std::vector<PairPlan *> chunk;
             size_t wb = 0;
             for (PairPlan *pl : g.second) {
                 const size_t wk = pl->ws_bytes - pl->in_bytes[0] - pl->in_bytes[1];
                 if (!chunk.empty() && (wb + wk > ctx->ws_budget || chunk.size() >= 4096)) {
-                    max_work = std::max(max_work, wb);
-                    max_n = std::max(max_n, chunk.size());
-                    wchunks[w].push_back(chunk);
-                    chunk.clear();
+                    put(chunk, wb);
                     wb = 0;
                 }
                 chunk.push_back(pl);
                 wb += wk;
             }
-            if (!chunk.empty()) {
-                max_work = std::max(max_work, wb);
-                max_n = std::max(max_n, chunk.size());
-                wchunks[w].push_back(chunk);
-            }
+            if (!chunk.empty())
+                put(chunk, wb);
         }
     }
     max_stage = al256(max_stage);
     max_work = al256(max_work);
-    (void)max_n;
     // one staging buffer per window parity; a single window needs one
     const size_t nstage = windows.size() > 1 ? 2 : 1;
     if (int rc = ensure_ws(ctx, nstage * max_stage + max_work))
@@ -2911,26 +2960,42 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
         const size_t cw = w - 1;   // the window computed now
         const int wp = (int)(cw & 1);
         CK(cudaStreamWaitEvent(st, ctx->ev_copy[wp], 0));
-        for (auto &chunk : wchunks[cw]) {
+        for (auto &span : wspans[cw]) {
             const auto t0 = std::chrono::steady_clock::now();
-            ChunkLaunch cl;
-            prep_chunk(ctx, chunk, off, ctx->ws + nstage * max_stage, ctx->htab + off, fills,
-                       cl);
+            const size_t c0 = cls.size();
+            JobSpan js;
+            js.off = off;
+            char *work = ctx->ws + nstage * max_stage;
+            std::vector<std::vector<PairPlan *> *> chunks;
+            for (auto &chunk : span) {
+                ChunkLaunch cl;
+                work += prep_chunk(ctx, chunk, off, work, ctx->htab + off, fills, cl);
+                off += cl.s.n;
+                js.add(cl.s);
+                cls.push_back(cl);
+                chunks.push_back(&chunk);
+                order.push_back(&chunk);
+            }
             prep_us += std::chrono::duration_cast<std::chrono::microseconds>(
                            std::chrono::steady_clock::now() - t0)
                            .count();
-            CK(cudaMemcpyAsync(ctx->dpairs_base + off, ctx->htab + off,
-                               (size_t)cl.n * sizeof(PairDev), cudaMemcpyHostToDevice, st));
-            if (cl.nfill) {   // through page-locked memory: no stream sync on the host
-                memcpy(ctx->hsel + cl.fill_off, fills.data() + cl.fill_off,
-                       (size_t)cl.nfill * sizeof(int));
-                CK(cudaMemcpyAsync(ctx->dsel + cl.fill_off, ctx->hsel + cl.fill_off,
-                                   (size_t)cl.nfill * sizeof(int), cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(ctx->dpairs_base + js.off, ctx->htab + js.off,
+                               (size_t)js.n * sizeof(PairDev), cudaMemcpyHostToDevice, st));
+            const int f0 = cls[c0].fill_off, nf = (int)fills.size() - f0;
+            if (nf) {   // through page-locked memory: no stream sync on the host
+                memcpy(ctx->hsel + f0, fills.data() + f0, (size_t)nf * sizeof(int));
+                CK(cudaMemcpyAsync(ctx->dsel + f0, ctx->hsel + f0, (size_t)nf * sizeof(int),
+                                   cudaMemcpyHostToDevice, st));
             }
-            cls.push_back(cl);
-            order.push_back(&chunk);
-            off += cl.n;
-            if (int rc = launch_chunk(ctx, chunk, cl)) {
+            int rc = launch_tables(ctx, chunks, js, cls[c0].mode, cls[c0].sonly != 0);
+            for (size_t c = 0; rc == ALN_OK && c < chunks.size(); ++c)
+                rc = launch_chunk(ctx, *chunks[c], cls[c0 + c]);
+            if (rc == ALN_OK && cls[c0].mode == JOB_PATCHES) {
+                launch_peaks(ctx, js);
+                if (cudaGetLastError() != cudaSuccess)
+                    rc = set_err(ctx, ALN_ERR_CUDA, "peak kernels");
+            }
+            if (rc != ALN_OK) {
                 cudaStreamSynchronize(ctx->cstream);
                 cudaStreamSynchronize(st);
                 return rc;
@@ -2948,8 +3013,8 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
     CK(cudaStreamSynchronize(st));
     prof_collect(ctx);
     for (size_t c = 0; c < order.size(); ++c)
-        for (int k = 0; k < cls[c].n; ++k) {
-            const ResultDev &r = ctx->hres[cls[c].off + k];
+        for (int k = 0; k < cls[c].s.n; ++k) {
+            const ResultDev &r = ctx->hres[cls[c].s.off + k];
             PairDev &d = (*order[c])[k]->d;
             d.r = r.r;
             d.dx = r.dx;
@@ -3638,7 +3703,7 @@ extern "C" int aln_corr_patches_noalloc(const aln_image *a, const aln_image *b, 
         const size_t sm = 2 * (size_t)RBL * (L + 1) * sizeof(float2);
         k_lagrow<<<dim3((Wy + RBL - 1) / RBL, 1), 256, sm, st>>>(dpair, tw, RBL);
     }
-    k_final<<<1, 256, 0, st>>>(dpair, dres, pl.orig_nx == 1, pl.orig_ny == 1, 0);
+    k_final<<<1, 256, 0, st>>>(dpair, dres);
     CK(cudaGetLastError());
     ResultDev hr;
     CK(cudaMemcpyAsync(&hr, dres, sizeof hr, cudaMemcpyDeviceToHost, st));

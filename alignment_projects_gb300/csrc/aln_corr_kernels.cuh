@@ -80,6 +80,8 @@ struct PairDev {
     double2 *seg[2];             // per column-walk segment: exclusive column offsets
     int *segN[2];
     double *colsum[2];           // per-column totals (mean shift)
+    int fin;                     // k_final: bit 0 / 1 the frame's FFT size is 1 in x / y,
+                                 // bit 2 rr holds the lag image (k2_lagrow, k2_lagscan)
     double *rr;                  // r over the lag window [j][x - xlo] (the key image)
     RowBest *rb;                 // per lag row
     double mu[2];                // mean shift applied before the FFT

@@ -408,8 +408,8 @@ __device__ __forceinline__ void sat_cols_packed(const PairDev &p, int i, unsigne
     }
 }
 
-// Chunks whose jobs all have packed tables: grid (ceil(max w / 64), 2 * npairs),
-// satp_smem() bytes of dynamic shared memory.
+// The jobs with packed tables: grid (ceil(max w / 64), 2 * npairs), satp_smem()
+// bytes of dynamic shared memory.
 __global__ void __launch_bounds__(32 * SAT_WARPS, 2) k3_satp(PairDev *pairs)
 {
     extern __shared__ __align__(16) unsigned char satp_stage[];
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(32 * SAT_WARPS, 2) k3_satp(PairDev *pairs)
     __shared__ int shN[64 * SAT_WARPS];
     const PairDev &p = pairs[blockIdx.y >> 1];
     const int i = blockIdx.y & 1;
-    if (p.status != 0 || blockIdx.x * 64 >= p.w[i])
+    if (p.status != 0 || !p.sat_packed || blockIdx.x * 64 >= p.w[i])
         return;
     if (p.cnt_kind == ALN_CNT_GT)
         sat_cols_packed<true>(p, i, satp_stage, shP, shN);
@@ -431,7 +431,7 @@ __global__ void k3_sat(PairDev *pairs)
     __shared__ int shN[32 * SAT_WARPS];
     const PairDev &p = pairs[blockIdx.y >> 1];
     const int i = blockIdx.y & 1;
-    if (p.status != 0 || blockIdx.x * 32 >= p.w[i] || (i == 1 && p.sat_shared))
+    if (p.status != 0 || p.sat_packed || blockIdx.x * 32 >= p.w[i] || (i == 1 && p.sat_shared))
         return;
     if (p.sat_nonly) {   // counts only (CorrImagesS without a mincor)
         if (p.cnt_kind != ALN_CNT_GT)
@@ -1377,7 +1377,7 @@ __device__ __forceinline__ void scan_row_int(const PairDev &p, const LagRow &q, 
 __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
 {
     const PairDev &p = pairs[blockIdx.y];
-    if (p.status != 0)
+    if (p.status != 0 || !(p.fin & 4))
         return;
     const int j = blockIdx.x * LAGSCAN_ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (j >= p.yhi - p.ylo + 1)
