@@ -1728,6 +1728,11 @@ static void need_rows(const PairDev &d, int img, int lo[2], int hi[2])
 
 #include "aln_tune.cuh"
 
+static bool float_tables(const PairDev &d)
+{
+    auto is_int = [](int dt) { return dt == ALN_U8 || dt == ALN_U16; };
+    return d.mode == JOB_IMAGES_R && !(is_int(d.dt[0]) && is_int(d.dt[1]));
+}
 static size_t sat_entry_bytes(const PairDev &d) { return d.sat_packed ? 8 : sizeof(double2); }
 
 // allow_split: the caller runs the register pipeline (batch path), whose row
@@ -1996,6 +2001,8 @@ static int plan_pair(aln_ctx *ctx, const aln_pair &P, PairPlan &pl, bool allow_t
         d.sp[i] = d.sat_packed ? (d.w[i] + 1) & ~1 : d.w[i];
         const size_t es = sat_entry_bytes(d);
         b += al256((size_t)ns * d.sp[i] * es) + al256((size_t)ns * d.sp[i] * sizeof(int));
+        if (float_tables(d))
+            b += al256((size_t)ns * d.sp[i] * sizeof(float2));
         b += al256((size_t)d.w[i] * sizeof(double));
         b += al256((size_t)SAT_WARPS * d.sp[i] * es) +
              al256((size_t)SAT_WARPS * d.sp[i] * sizeof(int));
@@ -2073,6 +2080,10 @@ static size_t carve(PairPlan &pl, char *base, const aln_pair &P)
         p += al256((size_t)ns * d.sp[i] * es);
         d.satN[i] = (int *)p;
         p += al256((size_t)ns * d.sp[i] * sizeof(int));
+        if (float_tables(d)) {
+            d.satf[i] = (float2 *)p;
+            p += al256((size_t)ns * d.sp[i] * sizeof(float2));
+        }
         d.colsum[i] = (double *)p;
         p += al256((size_t)d.w[i] * sizeof(double));
         d.seg[i] = (double2 *)p;
@@ -2298,7 +2309,7 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
 #undef X
     default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "column length %d", Ny);
     }
-    if (mode == JOB_PATCHES) {
+    if (mode == JOB_PATCHES || mode == JOB_IMAGES_R) {
         switch (L) {
 #define X(v) case v: launch_lagrow2<v>(ctx, n, maxWy); break;
             ALN_CASES_L(X)
@@ -2306,6 +2317,10 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
 #undef X
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "row length %d", L);
         }
+        if (mode == JOB_IMAGES_R)
+            LAUNCH(ctx, "k2_lagscan", k2_imgscan,
+                   dim3((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n), 32 * LAGSCAN_ROWS, 0,
+                   ctx->dpairs);
     } else if (mode == JOB_P2I) {
         switch (L) {
 #define X(v) case v: launch_lagp2i<v>(ctx, n, maxWy); break;
@@ -2436,8 +2451,9 @@ static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, 
                 pl.d.satN[1] = a.satN[1];
             }
         }
-        if (pl.d.mode == JOB_PATCHES && reg_path)
+        if ((pl.d.mode == JOB_PATCHES || pl.d.mode == JOB_IMAGES_R) && reg_path)
             pl.d.fin |= 4;
+        pl.d.reach = ord_float(pl.d.mincor > 0.0 ? (float)pl.d.mincor - 1.0e-4f : -2.0f);
         ++(pl.d.sat_packed ? sp.packed : sp.plain);
         hd[k] = pl.d;
     }

@@ -67,6 +67,7 @@ struct PairDev {
     float2 *Q;          // column-inverse output [kx][j], j = y - ylo, stride Wy
     double2 *sat[2];             // summed-area tables of v (.x) and v^2 (.y), [y][x]
                                  // stride sp: one 16-byte load reads both
+    float2 *satf[2];             // CorrImagesR, float pixels: the tables in FP32
     int sp[2];                   // table row pitch in entries (w; even when packed)
     int sat_packed;              // 1: both images uint8 and their overlaps small enough
                                  // for one 64-bit integer per entry (sat_pack)
@@ -80,6 +81,8 @@ struct PairDev {
     double2 *seg[2];             // per column-walk segment: exclusive column offsets
     int *segN[2];
     double *colsum[2];           // per-column totals (mean shift)
+    int reach;                   // CorrImagesR: the best legal R some row has found so
+                                 // far (ord_float), below which a lag is not looked at
     int fin;                     // k_final: bit 0 / 1 the frame's FFT size is 1 in x / y,
                                  // bit 2 rr holds the lag image (k2_lagrow, k2_lagscan)
     double *rr;                  // r over the lag window [j][x - xlo] (the key image)

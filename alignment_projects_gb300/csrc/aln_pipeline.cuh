@@ -577,6 +577,30 @@ __global__ void k_transpose(PairDev *pairs)
     }
 }
 
+// An FP64 number as FP32, toward zero, in integer instructions (conversions
+// share the narrow FP64 pipe).  Out of FP32's normal range: 0, or infinity (NaN
+// too).
+__device__ __forceinline__ float d2f_trunc(double v)
+{
+    const int hi = __double2hiint(v), m = (hi & 0x7fffffff) - 0x38000000;
+    const unsigned lo = (unsigned)__double2loint(v);
+    const unsigned b = m < 0x00100000 ? 0u : m > 0x0fdfffff ? 0x7f800000u
+                                            : __funnelshift_l(lo, (unsigned)m, 3);
+    return __uint_as_float(b | ((unsigned)hi & 0x80000000u));
+}
+// An FP64 number rounded to FP32 as the conversion does, in integer
+// instructions where the result is a normal number.
+__device__ __forceinline__ float d2f_rn(double v)
+{
+    const int hi = __double2hiint(v), m = (hi & 0x7fffffff) - 0x38000000;
+    const unsigned lo = (unsigned)__double2loint(v);
+    if (m < 0x00100000 || m > 0x0fdfffff)
+        return (float)v;
+    const unsigned b = __funnelshift_l(lo, (unsigned)m, 3), rem = lo << 3;   // the 29 bits cut
+    const unsigned up = rem > 0x80000000u || (rem == 0x80000000u && (b & 1u));
+    return __uint_as_float((b + up) | ((unsigned)hi & 0x80000000u));
+}
+
 // The row pass of the summed-area tables: per needed row, add the warp
 // segment offsets of k3_sat and take the x-prefix.  One warp per row (no
 // block-wide synchronisation, so a CTA carries eight rows and small images
@@ -611,6 +635,7 @@ __device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, 
     const typename SP::type *__restrict__ o =
         (const typename SP::type *)p.seg[i] + (long long)seg * p.sp[i];
     typename SP::type *__restrict__ r = (typename SP::type *)p.sat[i] + (long long)slot * p.sp[i];
+    float2 *__restrict__ rf = p.satf[i] ? p.satf[i] + (long long)slot * p.sp[i] : nullptr;
     TA cs = 0, cq = 0;
     for (int c0 = 0; c0 < w; c0 += 32 * K) {
         const int c = c0 + K * lane;
@@ -635,8 +660,12 @@ __device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, 
         bq = lane ? bq + cq : cq;
 #pragma unroll
         for (int k = 0; k < K; ++k)
-            if (c + k < w)
-                r[c + k] = SP::of(s[k] + bs, q[k] + bq);
+            if (c + k < w) {
+                const typename SP::type e = SP::of(s[k] + bs, q[k] + bq);
+                r[c + k] = e;
+                if (rf)
+                    rf[c + k] = make_float2(d2f_trunc((double)e.x), d2f_trunc((double)e.y));
+            }
         cs += __shfl_sync(0xffffffff, ts, 31);
         cq += __shfl_sync(0xffffffff, tq, 31);
     }
@@ -824,16 +853,16 @@ k2_rowfft(PairDev *pairs, const float2 *__restrict__ tw, int only_img, const int
         }
     } else {
         const double mu = p.mu[i];
+        const double *row = (const double *)img + y * st;
 #pragma unroll
         for (int q = 0; q < V; ++q) {
-            const int n = F::in_idx(t, q);
+            const int xa = 2 * F::in_idx(t, q), xb = xa + 1;
             float2 z = make_float2(0.f, 0.f);
             if (y < h) {
-                const int xa = 2 * n, xb = 2 * n + 1;
                 if (xa < w)
-                    z.x = (float)(load_px(img, dt, y * st + xa) - mu);
+                    z.x = d2f_rn(__dsub_rn(__ldg(row + xa), mu));
                 if (xb < w)
-                    z.y = (float)(load_px(img, dt, y * st + xb) - mu);
+                    z.y = d2f_rn(__dsub_rn(__ldg(row + xb), mu));
             }
             v[q] = z;
         }
@@ -1826,30 +1855,235 @@ __global__ void __launch_bounds__(256, 3) k2_lagss(PairDev *pairs, const float2 
     }
 }
 
+// an FP32 number as an integer that orders the same way, and back
+__host__ __device__ __forceinline__ int ord_float(float f)
+{
+#ifdef __CUDA_ARCH__
+    const int b = __float_as_int(f);
+#else
+    int b;
+    memcpy(&b, &f, 4);
+#endif
+    return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float from_ord_float(int o)
+{
+    return __int_as_float(o ^ ((o >> 31) & 0x7fffffff));
+}
+
+// R of a lag of the lag image (CorrImagesR: the value the R image holds there,
+// legal or not), FP64 as RCalc::CalcR.
+__device__ __forceinline__ double img_r(const PairDev &p, int ix, int iy)
+{
+    const float c = ((const float *)p.rr)[(long long)iy * p.wR + ix];
+    double r;
+    lag_eval(p, lag_row(p, iy - p.cy), ix - p.cx,
+             (double)c * (1.0 / ((double)p.Nx * (double)p.Ny)), true, r);
+    return r;
+}
+
+// An upper bound of R at a lag, FP32: box sums of the FP32 tables, with the
+// error that their truncation (2^-23 of each corner) and the FP32 arithmetic
+// can have made.  Infinite or NaN where the bound says nothing.
+__device__ __forceinline__ float4 row_box_f(const float2 *__restrict__ t, int oT, int oB, int L,
+                                            int R)
+{
+    // sums S, Q and the errors they may carry
+    float2 r = __ldg(t + oT + R);
+    float as = fabsf(r.x);
+    const float top = r.y;   // sum v^2 grows along both axes: the largest corner
+    if (L > 0) {
+        const float2 a = __ldg(t + oT + L - 1);
+        r.x -= a.x;
+        r.y -= a.y;
+        as += fabsf(a.x);
+    }
+    if (oB >= 0) {
+        const float2 b = __ldg(t + oB + R);
+        r.x -= b.x;
+        r.y -= b.y;
+        as += fabsf(b.x);
+        if (L > 0) {
+            const float2 c = __ldg(t + oB + L - 1);
+            r.x += c.x;
+            r.y += c.y;
+            as += fabsf(c.x);
+        }
+    }
+    // per corner 2^-23, per difference 2^-24 of an operand: 2^-21 of the sum of
+    // magnitudes covers both with room
+    return make_float4(r.x, r.y, 4.8e-7f * as, 1.9e-6f * top);
+}
+
+__device__ __forceinline__ float r_bound(float n, float cs, const float4 &A, const float4 &B,
+                                         float mu1, float mu2)
+{
+    const float EPS = 4.8e-7f;   // a few FP32 roundings of a term
+    const float a = A.x - n * mu1, b = B.x - n * mu2;
+    const float ea = A.z + EPS * (fabsf(A.x) + fabsf(n * mu1));
+    const float eb = B.z + EPS * (fabsf(B.x) + fabsf(n * mu2));
+    const float d1 = n * A.y - A.x * A.x, d2 = n * B.y - B.x * B.x;
+    const float e1 = n * A.w + (2.0f * fabsf(A.x) + A.z) * A.z + EPS * (n * A.y + A.x * A.x);
+    const float e2 = n * B.w + (2.0f * fabsf(B.x) + B.z) * B.z + EPS * (n * B.y + B.x * B.x);
+    const float num = n * cs - a * b + (fabsf(a) + ea) * eb + fabsf(b) * ea +
+                      EPS * (fabsf(n * cs) + fabsf(a * b));
+    const float lo1 = d1 - e1, lo2 = d2 - e2;
+    if (!(lo1 > 1e-30f && lo2 > 1e-30f && lo1 < 1e30f && lo2 < 1e30f))
+        return __int_as_float(0x7f800000);
+    // (num < 0: the larger denominator would bound it; 0 does)
+    return fmaxf(num, 0.0f) * (rsqrtf(lo1) * rsqrtf(lo2)) * (1.0f + 1.0e-6f) + 1.0e-6f;
+}
+
+// CorrImagesR's scan of the lag image k2_lagrow wrote: one warp per lag row.
+// R itself is FP64 (RCalc::CalcR, clamped to (-1, 1)), and this GPU computes
+// FP64 two lanes per clock and SM: with R, its box sums, conversions and
+// comparisons in FP64 at every lag the scan took 1063 of 1543 us for 24 pairs
+// of 300 x 421.  So each lag's R is first bounded from above without FP64 --
+// integer images by r_int, others from FP32 copies of their tables -- and the
+// FP64 R, the counts and the exact comparison are made where the bound reaches
+// the best R that any row of the job has found so far (p.reach; what is skipped
+// lies below that one, so the result does not depend on the rows' order): 234
+// us.  grid (ceil(max Wy / LAGSCAN_ROWS), njobs), block 32 * LAGSCAN_ROWS.
+template <bool INT>
+__device__ __forceinline__ void scan_row_img(const PairDev &p, const LagRow &q, int j, int lo,
+                                             int hi, bool check, int *job_reach, double &br,
+                                             int &bk)
+{
+    const int lane = threadIdx.x & 31, y = p.ylo + j, iy = y + p.cy;
+    const float *__restrict__ row =
+        (const float *)p.rr + (long long)j * (p.xhi - p.xlo + 1) - p.xlo;
+    // 1 / (Nx Ny): CorrImages grids are powers of two
+    const double inv = __hiloint2double((1023 - p.logNx - p.logNy) << 20, 0);
+    const double mincor = p.mincor;
+    const float invf = (float)inv;
+    const int key0 = iy * p.wR + p.cx;   // key of lag x: key0 + x
+    const float mu1 = (float)p.mu[0], mu2 = (float)p.mu[1];
+    const int m1 = INT ? (int)p.mu[0] : 0, m2 = INT ? (int)p.mu[1] : 0;
+    float reach = from_ord_float(*(volatile int *)job_reach);   // R below it cannot win
+#pragma unroll 2
+    for (int x0 = lo; x0 <= hi; x0 += 32) {
+        const int x = min(x0 + lane, hi);
+        const int L2 = max(0, x), R2 = max(min(q.w2 - 1, x + q.w1 - 1), L2);
+        const int n = (R2 - L2 + 1) * q.olh;
+        const float c = __ldg(row + x);
+        float top;
+        if (INT) {
+            const longlong2 A = row_box_i(p, q, 0, n, L2 - x, R2 - x);
+            const longlong2 B = row_box_i(p, q, 1, n, L2, R2);
+            top = r_int(n, c * invf, A.x, A.y, B.x, B.y, m1, m2);
+            // r_int's FP32 rounding, its flat-overlap guard near the FP64 one, and
+            // R = 0 where the FP64 r falls outside (-1, 1)
+            top = top == 0.0f ? __int_as_float(0x7f800000) : fmaxf(top, 0.0f) + 1.0e-4f;
+        } else {
+            top = r_bound((float)n, c * invf,
+                          row_box_f(p.satf[0], q.oT[0], q.oB[0], L2 - x, R2 - x),
+                          row_box_f(p.satf[1], q.oT[1], q.oB[1], L2, R2), mu1, mu2);
+        }
+        const bool cand = x0 + lane <= hi && !(top < reach);   // (NaN: look closer)
+        if (__any_sync(0xffffffff, cand)) {
+            if (cand) {
+                double rv;
+                bool ok = lag_eval(p, q, x, (double)c * inv, true, rv);
+                if (check)
+                    ok = ok && oval_ok(p, x + p.cx, iy);
+                if (ok && (mincor <= 0.0 || rv > mincor) &&
+                    (rv > br || (rv == br && key0 + x < bk))) {
+                    br = rv;
+                    bk = key0 + x;
+                }
+            }
+            const int m = __reduce_max_sync(
+                0xffffffff, ord_float(bk == 0x7fffffff ? -2.0f : __double2float_rd(br)));
+            reach = fmaxf(reach, from_ord_float(m));
+            if (lane == 0 && m > *(volatile int *)job_reach)
+                reach = fmaxf(reach, from_ord_float(atomicMax(job_reach, m)));
+            reach = __shfl_sync(0xffffffff, reach, 0);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_imgscan(PairDev *pairs)
+{
+    const PairDev &p = pairs[blockIdx.y];
+    if (p.status != 0)
+        return;
+    const int j = blockIdx.x * LAGSCAN_ROWS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (j >= p.yhi - p.ylo + 1)
+        return;
+    const int y = p.ylo + j;
+    const LagRow q = lag_row(p, y);
+    const bool check = q.tbl || q.omax != 0x7fffffff;
+    int lo, hi;
+    legal_span(p, q, y + p.cy, lo, hi);
+    double br = -1.0e30;
+    int bk = 0x7fffffff;
+    // (r_int's integers hold for every overlap of an 8-bit row, of a 16-bit one
+    // below 2^20 pixels; the rest bound nothing and take the FP64 R at each lag)
+    if (!p.satf[0] && r_int_ok(p, (long long)min(q.w1, q.w2) * q.olh)) {
+        scan_row_img<true>(p, q, j, lo, hi, check, &pairs[blockIdx.y].reach, br, bk);
+    } else if (p.satf[0]) {
+        scan_row_img<false>(p, q, j, lo, hi, check, &pairs[blockIdx.y].reach, br, bk);
+    } else {
+        const double inv = __hiloint2double((1023 - p.logNx - p.logNy) << 20, 0);
+        const float *row = (const float *)p.rr + (long long)j * (p.xhi - p.xlo + 1) - p.xlo;
+        for (int x = lo + lane; x <= hi; x += 32) {
+            double rv;
+            if (lag_eval(p, q, x, (double)row[x] * inv, true, rv) &&
+                (!check || oval_ok(p, x + p.cx, y + p.cy)) &&
+                (p.mincor <= 0.0 || rv > p.mincor) && (bk == 0x7fffffff || rv > br)) {
+                br = rv;
+                bk = (y + p.cy) * p.wR + p.cx + x;
+            }
+        }
+    }
+    long long k = bk == 0x7fffffff ? 0x7fffffffffffffffLL : bk;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double r2 = __shfl_down_sync(0xffffffff, br, o);
+        const long long k2 = __shfl_down_sync(0xffffffff, k, o);
+        best_merge(br, k, r2, k2);
+    }
+    if (lane == 0) {
+        RowBest rb;
+        rb.r = br;
+        rb.key = k;
+        rb.ssum = rb.ssum2 = 0.0;
+        p.rb[j] = rb;
+    }
+}
+
+// The key image (the window is the whole R image) at R-image pixel (rx, ry),
+// k = 0, or its neighbour k = 1..4 (0 outside the image).
+__device__ double img_near(const PairDev &p, int rx, int ry, int k)
+{
+    const int x = rx + (k == 1 ? -1 : k == 2 ? 1 : 0), y = ry + (k == 3 ? -1 : k == 4 ? 1 : 0);
+    if (x < 0 || y < 0 || x >= p.wR || y >= p.hR)
+        return 0.0;
+    if (p.fin & 4)   // CorrImagesR: R from the lag image
+        return img_r(p, x, y);
+    const long long o = (long long)y * p.wR + x;
+    return p.s_float ? (double)((const float *)p.rr)[o] : p.rr[o];
+}
+
 // ParabPeak on the key image at R-image pixel (rx, ry) (neighbours must be
 // > 0, 0_GEN/Correlation.cpp:2975-3010), ReturnR's offsets (:3016-3043); the
 // S score 10 (S - mean) / (sd sqrt(nR)) with the sample sd for CorrImagesS
 // (:3285-3289).  Writes the job's result.
-__device__ void img_result(PairDev &p, int rx, int ry, double ss, double ss2, ResultDev &o)
+__device__ void img_result(PairDev &p, int rx, int ry, double ss, double ss2, const double *v,
+                           ResultDev &o)
 {
+    // v: the key image at the peak, left, right, below, above (img_near); the
+    // FP32 c when s_float: ParabPeak's ratios and the S score are the same in
+    // c units
     const int wR = p.wR, hR = p.hR;
-    // the key image (the window is the whole R image); FP32 c when s_float:
-    // ParabPeak's ratios and the S score are the same in c units
-    const double *Id = p.rr;
-    const float *If = (const float *)p.rr;
-    const bool fl = p.s_float != 0;
-    auto I = [&](long long k) -> double { return fl ? (double)If[k] : Id[k]; };
     double xpk = rx, ypk = ry;
-    const double z1 = I(rx + (long long)wR * ry);
+    const double z1 = v[0];
     double z0, z2;
-    if (rx - 1 >= 0 && rx + 1 < wR && (z0 = I(rx - 1 + (long long)wR * ry)) > 0.0 &&
-        (z2 = I(rx + 1 + (long long)wR * ry)) > 0.0) {
+    if (rx - 1 >= 0 && rx + 1 < wR && (z0 = v[1]) > 0.0 && (z2 = v[2]) > 0.0) {
         z0 = (z0 - z2) / (2 * (z0 + z2 - z1 - z1));
         if (fabs(z0) <= 8)
             xpk += z0;
     }
-    if (ry - 1 >= 0 && ry + 1 < hR && (z0 = I(rx + (long long)wR * (ry - 1))) > 0.0 &&
-        (z2 = I(rx + (long long)wR * (ry + 1))) > 0.0) {
+    if (ry - 1 >= 0 && ry + 1 < hR && (z0 = v[3]) > 0.0 && (z2 = v[4]) > 0.0) {
         z0 = (z0 - z2) / (2 * (z0 + z2 - z1 - z1));
         if (fabs(z0) <= 8)
             ypk += z0;
@@ -1911,8 +2145,14 @@ __global__ void k_final_img(PairDev *pairs, ResultDev *res)
         red_s2[wid] = ss2;
     }
     __syncthreads();
-    if (threadIdx.x != 0)
+    if (threadIdx.x >= 5)
         return;
+    // five threads: each finds the peak and fetches one value of the key image
+    __shared__ double near[5];
+    br = red_r[0];
+    bk = red_k[0];
+    ss = red_s[0];
+    ss2 = red_s2[0];
     for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
         best_merge(br, bk, red_r[q], red_k[q]);
         ss += red_s[q];
@@ -1920,14 +2160,19 @@ __global__ void k_final_img(PairDev *pairs, ResultDev *res)
     }
     ResultDev &o = res[blockIdx.x];
     if (bk == 0x7fffffffffffffffLL) {   // no candidate lag
-        p.status = ALN_NO_PEAK;
-        o.r = o.dx = o.dy = 0.0;
-        o.status = ALN_NO_PEAK;
-        o.px = o.py = 0;
+        if (threadIdx.x == 0) {
+            p.status = ALN_NO_PEAK;
+            o.r = o.dx = o.dy = 0.0;
+            o.status = ALN_NO_PEAK;
+            o.px = o.py = 0;
+        }
         return;
     }
     const int ry = (int)(bk / p.wR), rx = (int)(bk - (long long)ry * p.wR);
-    img_result(p, rx, ry, ss, ss2, o);
+    near[threadIdx.x] = img_near(p, rx, ry, threadIdx.x);
+    __syncwarp(0x1f);
+    if (threadIdx.x == 0)
+        img_result(p, rx, ry, ss, ss2, near, o);
 }
 
 // ---------------------------------------------------------------------------
@@ -2099,8 +2344,12 @@ __global__ void __launch_bounds__(FPK_THREADS) k_fpeak(PairDev *pairs, ResultDev
             }
             hi = __syncthreads_or(hi);
             if (!hi) {
-                if (tid == 0)
-                    img_result(p, rx, ry, 0.0, 0.0, o);
+                if (tid == 0) {
+                    double v[5];
+                    for (int m = 0; m < 5; ++m)
+                        v[m] = img_near(p, rx, ry, m);
+                    img_result(p, rx, ry, 0.0, 0.0, v, o);
+                }
                 return;
             }
         }

@@ -109,3 +109,43 @@ def test_typed_rule_equals_its_table(ctx, w, h, kind, a, b, area):
             dict(kind=aln.CORR_R, a=x, b=y, legal=aln.legal(kind, a, b, area)),
             dict(kind=aln.CORR_R, a=x, b=y, legal=aln.legal(table=table))])
         assert imgs[0] == imgs[1], dt
+
+
+@pytest.mark.parametrize("data", ["normal", "f32", "offset", "tiny", "flat", "u8", "u16", "mixed"])
+@pytest.mark.parametrize("rule", ["none", "min", "counts", "oval", "mincor", "mincor-none"])
+def test_corr_images_r_bound(ctx, orc, data, rule):
+    """CorrImagesR's scan looks closer only where an FP32 bound of R reaches the
+    best R found: the oracle's peak for images that make the bound tight, loose
+    or useless, under each kind of rule."""
+    import oracle as O
+    from test_gpu_images import aln_legal, check
+    rng = np.random.default_rng(len(data) * 100 + len(rule))
+    big = rng.standard_normal((70, 66))
+    for _ in range(2):   # some structure: neighbours alike
+        big = (big + np.roll(big, 1, 0) + np.roll(big, 1, 1)) / 1.7
+    a, b = big[5:47, 6:45], big[9:61, 3:58]
+    b = b + 0.2 * rng.standard_normal(b.shape)
+    if data == "offset":
+        a, b = 3000.0 + a, 3000.0 + b
+    elif data == "tiny":
+        a, b = 1e-9 * a, 1e-9 * b
+    elif data == "flat":
+        a, b = np.where(a < 1.5, 0.0, a), np.where(b < 1.0, 0.0, b)
+    elif data in ("u8", "u16", "mixed"):
+        top = 255 if data != "u16" else 4095
+        a, b = (np.clip(np.rint((v + 4) * top / 8), 0, top) for v in (a, b))
+        a = a.astype(np.uint16 if data == "u16" else np.uint8)
+        b = b.astype({"u8": np.uint8, "u16": np.uint16, "mixed": np.float32}[data])
+    if data in ("f32", "flat"):
+        a, b = a.astype(np.float32), b.astype(np.float32)
+    n = 400 if rule == "counts" else 0
+    lg = O.legal(*((O.RGN_MIN, 12, 12, 300) if rule != "none" else (0, 0, 0, 0)),
+                 1 if rule == "counts" else 0, n)
+    mincor = 0.05 if rule == "mincor" else 1.5 if rule == "mincor-none" else 0.0
+    disc = (3, -4, 17, 9) if rule == "oval" else (0, 0, -1, -1)
+    g = ctx.corr_images(1, a, b, aln_legal(lg), mincor, 0.75, *disc)
+    pts = [np.stack([v.ravel() for v in np.mgrid[0:m.shape[0], 0:m.shape[1]][::-1]], 1)
+           .astype(np.float64) for m in (a, b)]
+    o = orc.corr_images(1, pts[0], a.ravel().astype(np.float64), pts[1],
+                        b.ravel().astype(np.float64), lg, mincor, 0.75, *disc)
+    check(g, o, 1, (data, rule))
