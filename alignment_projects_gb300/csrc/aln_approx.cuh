@@ -4,8 +4,8 @@
 // after aln_sweep.cuh.
 //
 // The stages run batched over the pairs: the overlap crop is a strided view
-// of each tile (no copy), MakeThumbs is one aln_decimate_batch over all crops,
-// the sweep one aln_thm_call_batch, PostTweaks and FinishAtFullRes one
+// of each tile (no copy), MakeThumbs is one aln_decimate_batch over all crops
+// whose thumbnails stay on the device, the sweep one aln_thm_call_batch, PostTweaks and FinishAtFullRes one
 // batch each.  The host does the integer box arithmetic and, at the end,
 // IsectToImageCoords and the LIMXY test (a few flops per pair).
 #pragma once
@@ -30,21 +30,29 @@ void boxes_from_shifts(IBoxI &B1, IBoxI &B2, int w1, int h1, int w2, int h2, int
     B1.T = B2.T - y;
 }
 
-// A decimated (or full-resolution) thumbnail on the host: grid values,
-// presence mask, and the aln_thumbs view of a pair of them.
+// A decimated (or full-resolution) thumbnail on the device: grid values and
+// presence mask (absent bins hold 0), each grid row's present span.
 struct Thumb {
-    std::vector<double> v;
-    std::vector<unsigned char> m;
+    const double *v = nullptr;
+    const unsigned char *m = nullptr;
     int w = 0, h = 0;
     double sd = 0.0;
     long long present = 0;
+    std::vector<int2> rows;
 };
 
-// aln_thumbs of a pair: A as its grid with the mask over the present bins'
-// bounding box, B as a raster over its bounding box (absent bins 0), both
-// with their corner offsets (the reference's point lists are relative to
-// the crop's corner, absent bins simply missing)
-bool thumbs_of(const Thumb &a, const Thumb &b, std::vector<double> &bras, aln_thumbs &T)
+// Device memory of one call's thumbnails
+struct ThumbMem {
+    char *p = nullptr;
+    ~ThumbMem() { cudaFree(p); }
+};
+
+// aln_thumbs of a pair, device pointers: A as its grid with the mask over the
+// present bins' bounding box, B as a raster over its bounding box (absent bins
+// 0), both with their corner offsets (the reference's point lists are
+// relative to the crop's corner, absent bins simply missing).  rows: A's spans
+// inside its box.
+bool thumbs_of(const Thumb &a, const Thumb &b, std::vector<int2> &rows, aln_thumbs &T)
 {
     auto bbox = [](const Thumb &t, int &x0, int &y0, int &x1, int &y1) {
         x0 = t.w;
@@ -52,42 +60,39 @@ bool thumbs_of(const Thumb &a, const Thumb &b, std::vector<double> &bras, aln_th
         x1 = -1;
         y1 = -1;
         for (int y = 0; y < t.h; ++y)
-            for (int x = 0; x < t.w; ++x)
-                if (t.m[(size_t)y * t.w + x]) {
-                    x0 = std::min(x0, x);
-                    x1 = std::max(x1, x);
-                    y0 = std::min(y0, y);
-                    y1 = std::max(y1, y);
-                }
+            if (t.rows[y].x >= 0) {
+                x0 = std::min(x0, t.rows[y].x);
+                x1 = std::max(x1, t.rows[y].y);
+                y0 = std::min(y0, y);
+                y1 = std::max(y1, y);
+            }
         return x1 >= 0;
     };
     int ax0, ay0, ax1, ay1, bx0, by0, bx1, by1;
     if (!bbox(a, ax0, ay0, ax1, ay1) || !bbox(b, bx0, by0, bx1, by1))
         return false;
     memset(&T, 0, sizeof T);
-    T.a = a.v.data() + (size_t)ay0 * a.w + ax0;
-    T.a_mask = a.m.data() + (size_t)ay0 * a.w + ax0;
+    T.a = a.v + (size_t)ay0 * a.w + ax0;
+    T.a_mask = a.m + (size_t)ay0 * a.w + ax0;
     T.a_w = ax1 - ax0 + 1;
     T.a_h = ay1 - ay0 + 1;
     T.a_stride = a.w;
     T.a_x0 = ax0;
     T.a_y0 = ay0;
-    const int bw = bx1 - bx0 + 1, bh = by1 - by0 + 1;
-    bras.assign((size_t)bw * bh, 0.0);
-    for (int y = 0; y < bh; ++y)
-        for (int x = 0; x < bw; ++x) {
-            const size_t s = (size_t)(y + by0) * b.w + (x + bx0);
-            if (b.m[s])
-                bras[(size_t)y * bw + x] = b.v[s];
+    rows.assign(a.rows.begin() + ay0, a.rows.begin() + ay1 + 1);
+    for (int2 &r : rows)
+        if (r.x >= 0) {
+            r.x -= ax0;
+            r.y -= ax0;
         }
-    T.b.data = bras.data();
+    T.b.data = b.v + (size_t)by0 * b.w + bx0;
     T.b.dtype = ALN_F64;
-    T.b.w = bw;
-    T.b.h = bh;
-    T.b.stride = bw;
+    T.b.w = bx1 - bx0 + 1;
+    T.b.h = by1 - by0 + 1;
+    T.b.stride = b.w;
     T.b.x0 = bx0;
     T.b.y0 = by0;
-    T.b.on_device = 0;
+    T.b.on_device = 1;
     return true;
 }
 
@@ -152,45 +157,43 @@ extern "C" int aln_approx_match_batch(aln_ctx *ctx, int n, const aln_tile_pair *
     if (m == 0)
         return ALN_OK;
     // ---- MakeThumbs (CThmUtil.cpp:470-523) at THMDEC and at 1 --------------
-    auto make_thumbs = [&](int dec, std::vector<Thumb> &th) -> int {
-        th.assign(2 * (size_t)m, Thumb());
-        std::vector<double *> ov(2 * (size_t)m);
-        std::vector<unsigned char *> om(2 * (size_t)m);
-        std::vector<double> sd(2 * (size_t)m);
-        for (int q = 0; q < 2 * m; ++q) {
-            th[q].w = (crop[q].w + dec - 1) / dec;
-            th[q].h = (crop[q].h + dec - 1) / dec;
-            th[q].v.resize((size_t)th[q].w * th[q].h);
-            th[q].m.resize((size_t)th[q].w * th[q].h);
-            ov[q] = th[q].v.data();
-            om[q] = th[q].m.data();
-        }
-        if (int rc = aln_decimate_batch(ctx, 2 * m, crop.data(), nullptr, dec, 1, ov.data(),
-                                        om.data(), sd.data()))
+    // They stay on the device: the sweep reads them there.  (Through the host --
+    // result copies, masks counted and boxed there, rasters copied back -- the
+    // chain on three 1024^2 pairs took 14 of its 20 ms.)
+    auto make_thumbs = [&](int dec, std::vector<Thumb> &th, ThumbMem &mem) -> int {
+        std::vector<DecJob> jobs;
+        std::vector<std::vector<int2>> rows;
+        if (int rc = decimate_device(ctx, 2 * m, crop.data(), nullptr, dec, 1, jobs, &rows,
+                                     &mem.p))
             return rc;
+        th.assign(2 * (size_t)m, Thumb());
         for (int q = 0; q < 2 * m; ++q) {
-            th[q].sd = sd[q];
-            long long c = 0;
-            for (unsigned char b : th[q].m)
-                c += b != 0;
-            th[q].present = c;
+            th[q].v = jobs[q].vals;
+            th[q].m = jobs[q].pres;
+            th[q].w = jobs[q].ow;
+            th[q].h = jobs[q].oh;
+            th[q].sd = jobs[q].sd;
+            th[q].present = jobs[q].np;
+            th[q].rows.swap(rows[q]);
         }
         return ALN_OK;
     };
     const int dec = P->thmdec;
     const long long req_thumb = P->olap2d / ((long long)dec * dec);
+    ThumbMem thm_mem, full_mem;
     std::vector<Thumb> thm;
-    if (int rc = make_thumbs(dec, thm))
+    if (int rc = make_thumbs(dec, thm, thm_mem))
         return rc;
     std::vector<int> act;                 // pairs with usable thumbnails
     std::vector<aln_thumbs> T;
-    std::vector<std::vector<double>> bras(m);
+    std::vector<std::vector<int2>> rows(m);
+    std::vector<DevThumbs> D;
     for (int q = 0; q < m; ++q) {
         aln_approx_result &o = out[live[q]];
         const Thumb &a = thm[2 * q], &b = thm[2 * q + 1];
         aln_thumbs t;
         if (a.present < req_thumb || !(a.sd > 0.0) || !(b.sd > 0.0) ||
-            !thumbs_of(a, b, bras[q], t)) {
+            !thumbs_of(a, b, rows[q], t)) {
             o.status = 2;
             continue;
         }
@@ -198,6 +201,7 @@ extern "C" int aln_approx_match_batch(aln_ctx *ctx, int n, const aln_tile_pair *
         t.olap1d = P->olap1d / dec;
         t.b_key = 0;
         T.push_back(t);
+        D.push_back(DevThumbs{rows[q].data()});
         act.push_back(q);
     }
     const int na = (int)act.size();
@@ -226,9 +230,9 @@ extern "C" int aln_approx_match_batch(aln_ctx *ctx, int n, const aln_tile_pair *
         args[4 * q + 2] = 0.5;
         args[4 * q + 3] = 0.0;
     }
-    if (int rc = aln_thm_call_batch(ctx, na, T.data(), &prm,
-                                    P->mode_prior ? ALN_THMOP_PRIOR : ALN_THMOP_DENOVO,
-                                    args.data(), best.data(), tw.data(), ret.data()))
+    if (int rc = thm_call(ctx, na, T.data(), D.data(), &prm,
+                          P->mode_prior ? ALN_THMOP_PRIOR : ALN_THMOP_DENOVO, args.data(),
+                          best.data(), tw.data(), ret.data()))
         return rc;
     std::vector<int> fin;   // pairs whose sweep succeeded
     for (int q = 0; q < na; ++q) {
@@ -248,16 +252,18 @@ extern "C" int aln_approx_match_batch(aln_ctx *ctx, int n, const aln_tile_pair *
         return ALN_OK;
     // ---- Finish (CThmUtil.cpp:889-971) ------------------------------------
     std::vector<aln_thumbs> Tf(nf);
+    std::vector<DevThumbs> Df(nf);
     std::vector<aln_thm_result> bf(nf);
     std::vector<double> twf(6 * (size_t)nf), zargs(4 * (size_t)nf, 0.0);
     for (int i = 0; i < nf; ++i) {
         Tf[i] = T[fin[i]];
+        Df[i] = D[fin[i]];
         bf[i] = best[fin[i]];
         memcpy(&twf[6 * i], &tw[6 * fin[i]], 6 * sizeof(double));
     }
     if (P->tweaks)
-        if (int rc = aln_thm_call_batch(ctx, nf, Tf.data(), &prm, ALN_THMOP_POSTTWEAKS,
-                                        zargs.data(), bf.data(), twf.data(), nullptr))
+        if (int rc = thm_call(ctx, nf, Tf.data(), Df.data(), &prm, ALN_THMOP_POSTTWEAKS,
+                              zargs.data(), bf.data(), twf.data(), nullptr))
             return rc;
     for (int i = 0; i < nf; ++i) {   // undo the thumbnail scale
         bf[i].X *= dec;
@@ -265,28 +271,30 @@ extern "C" int aln_approx_match_batch(aln_ctx *ctx, int n, const aln_tile_pair *
     }
     std::vector<Thumb> full;
     if (dec > 1) {
-        if (int rc = make_thumbs(1, full))
+        if (int rc = make_thumbs(1, full, full_mem))
             return rc;
     } else
         full = thm;
-    std::vector<std::vector<double>> brf(nf);
+    std::vector<std::vector<int2>> rowsf(nf);
     std::vector<int> ok(nf, 1);
     for (int i = 0; i < nf; ++i) {
         const int q = act[fin[i]];
         const Thumb &a = full[2 * q], &b = full[2 * q + 1];
         if (a.present < P->olap2d || !(a.sd > 0.0) || !(b.sd > 0.0) ||
-            !thumbs_of(a, b, brf[i], Tf[i])) {
+            !thumbs_of(a, b, rowsf[i], Tf[i])) {
             ok[i] = 0;
             out[live[q]].status = 2;
             // a stand-in the call can run on; its result is not used
             Tf[i] = T[fin[i]];
+        } else {
+            Df[i].rows = rowsf[i].data();
         }
         Tf[i].req_area = P->olap2d;
         Tf[i].olap1d = P->olap1d;
         Tf[i].b_key = 0;
     }
-    if (int rc = aln_thm_call_batch(ctx, nf, Tf.data(), &prm, ALN_THMOP_FULLRES, zargs.data(),
-                                    bf.data(), twf.data(), nullptr))
+    if (int rc = thm_call(ctx, nf, Tf.data(), Df.data(), &prm, ALN_THMOP_FULLRES, zargs.data(),
+                          bf.data(), twf.data(), nullptr))
         return rc;
     for (int i = 0; i < nf; ++i) {
         if (!ok[i])

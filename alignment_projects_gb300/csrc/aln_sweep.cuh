@@ -189,8 +189,7 @@ struct ThmPair {
     const aln_thumbs *in;
     std::vector<std::pair<long long, long long>> hull;   // convex hull of A's points
     double Tptwk[6];
-    const double *dev_a;            // device copies
-    const float *dev_af;            // A's values in FP32 (what the splat reads)
+    const float *dev_af;            // A's values in FP32 (what the splat reads), on the device
     const unsigned char *dev_mask;
     aln_image dev_b;
     // pretweak sweep records (TCD.vT)
@@ -217,19 +216,31 @@ static double cross3(const std::pair<long long, long long> &o, const std::pair<l
            (double)(a.second - o.second) * (double)(b.first - o.first);
 }
 
+// A pair's thumbnails that are on the device already (ApproximateMatch's):
+// aln_thumbs' a, a_mask and b.data are device pointers then, and A's present
+// points come as each grid row's first and last one (x < 0: none).
+struct DevThumbs {
+    const int2 *rows;   // a_h entries
+};
+
 // Monotone-chain hull of the present A grid points (absolute coordinates).
-static void make_hull(ThmPair &tp)
+static void make_hull(ThmPair &tp, const int2 *rows)
 {
     const aln_thumbs &T = *tp.in;
     std::vector<std::pair<long long, long long>> pts;
     for (int y = 0; y < T.a_h; ++y) {
         int xl = -1, xr = -1;   // extreme present points of the row suffice
-        for (int x = 0; x < T.a_w; ++x)
-            if (!T.a_mask || T.a_mask[x + (size_t)T.a_stride * y]) {
-                if (xl < 0)
-                    xl = x;
-                xr = x;
-            }
+        if (rows) {
+            xl = rows[y].x;
+            xr = rows[y].y;
+        } else {
+            for (int x = 0; x < T.a_w; ++x)
+                if (!T.a_mask || T.a_mask[x + (size_t)T.a_stride * y]) {
+                    if (xl < 0)
+                        xl = x;
+                    xr = x;
+                }
+        }
         if (xl >= 0) {
             pts.push_back({xl + T.a_x0, y + T.a_y0});
             if (xr != xl)
@@ -705,7 +716,8 @@ static int scan_with_tweaks(SweepCtx &S, const std::vector<int> &ids,
 // Device copies of the thumbnails, hulls and the initial sweep state
 // (CThmScan::Initialize) for every pair; *dbuf receives the allocation.
 static int sweep_setup(aln_ctx *ctx, SweepCtx &S, int npairs, const aln_thumbs *thumbs,
-                       const aln_thm_params *params, char **dbuf_out)
+                       const aln_thm_params *params, char **dbuf_out,
+                       const DevThumbs *dev = nullptr)
 {
     *dbuf_out = nullptr;
     CK(cudaSetDevice(ctx->device));
@@ -720,8 +732,10 @@ static int sweep_setup(aln_ctx *ctx, SweepCtx &S, int npairs, const aln_thumbs *
         if (!T.a || T.a_w < 1 || T.a_h < 1 || T.a_stride < T.a_w || !T.b.data ||
             T.b.dtype != ALN_F64 || T.b.w < 1 || T.b.h < 1 || T.b.stride < T.b.w)
             return set_err(ctx, ALN_ERR_ARG, "thumbnail pair %d: bad grid/raster", k);
-        bytes += al256((size_t)T.a_stride * T.a_h * 8) + al256((size_t)T.a_stride * T.a_h * 4) +
-                 al256((size_t)T.a_stride * T.a_h) + al256((size_t)T.b.stride * T.b.h * 8);
+        bytes += al256((size_t)T.a_stride * T.a_h * 4);
+        if (!dev)
+            bytes += al256((size_t)T.a_stride * T.a_h * 8) + al256((size_t)T.a_stride * T.a_h) +
+                     al256((size_t)T.b.stride * T.b.h * 8);
     }
     char *dbuf = nullptr;
     if (bytes) {
@@ -740,38 +754,35 @@ static int sweep_setup(aln_ctx *ctx, SweepCtx &S, int npairs, const aln_thumbs *
         tp.ncalls = 0;
         tp.err = 0;
         aff_one(tp.Tptwk);
-        const size_t ab = (size_t)T.a_stride * T.a_h * 8;
-        tp.dev_a = (const double *)p;
-        if (cudaMemcpyAsync(p, T.a, ab, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
-            rc = set_err(ctx, ALN_ERR_CUDA, "thumbnail copy");
-        p += al256(ab);
+        // elements from the first point to the last one
+        const size_t na = (size_t)T.a_stride * (T.a_h - 1) + T.a_w;
+        const size_t nbr = (size_t)T.b.stride * (T.b.h - 1) + T.b.w;
+        const double *dev_a = T.a;
+        tp.dev_mask = T.a_mask;
+        tp.dev_b = T.b;
+        tp.dev_b.on_device = 1;
+        auto copy = [&](const void *src, size_t n, size_t room, const char *what) -> const void * {
+            if (cudaMemcpyAsync(p, src, n, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+                rc = set_err(ctx, ALN_ERR_CUDA, "%s copy", what);
+            ctx->h2d_bytes += (long long)n;
+            const void *q = p;
+            p += al256(room);
+            return q;
+        };
+        if (!dev) {
+            const size_t room = (size_t)T.a_stride * T.a_h;
+            dev_a = (const double *)copy(T.a, na * 8, room * 8, "thumbnail");
+            if (T.a_mask)
+                tp.dev_mask = (const unsigned char *)copy(T.a_mask, na, room, "mask");
+            tp.dev_b.data = copy(T.b.data, nbr * 8, (size_t)T.b.stride * T.b.h * 8, "thumbnail");
+        }
         // the splat multiplies in FP32: convert once here instead of per
         // gathered point (FP64 conversions run on the narrow FP64 pipe)
         tp.dev_af = (const float *)p;
-        {
-            const size_t na = (size_t)T.a_stride * T.a_h;
-            LAUNCH(ctx, "k_f64_to_f32", k_f64_to_f32,
-                   (unsigned)std::min<size_t>((na + 255) / 256, 1024), 256, 0, tp.dev_a,
-                   (float *)p, na);
-            p += al256(na * 4);
-        }
-        tp.dev_mask = nullptr;
-        if (T.a_mask) {
-            tp.dev_mask = (const unsigned char *)p;
-            if (cudaMemcpyAsync(p, T.a_mask, (size_t)T.a_stride * T.a_h, cudaMemcpyHostToDevice,
-                                ctx->stream) != cudaSuccess)
-                rc = set_err(ctx, ALN_ERR_CUDA, "mask copy");
-        }
-        p += al256((size_t)T.a_stride * T.a_h);
-        const size_t bb = (size_t)T.b.stride * T.b.h * 8;
-        tp.dev_b = T.b;
-        tp.dev_b.data = p;
-        tp.dev_b.on_device = 1;
-        if (cudaMemcpyAsync(p, T.b.data, bb, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
-            rc = set_err(ctx, ALN_ERR_CUDA, "thumbnail copy");
-        p += al256(bb);
-        ctx->h2d_bytes += (long long)(ab + bb + (T.a_mask ? (size_t)T.a_stride * T.a_h : 0));
-        make_hull(tp);
+        LAUNCH(ctx, "k_f64_to_f32", k_f64_to_f32,
+               (unsigned)std::min<size_t>((na + 255) / 256, 1024), 256, 0, dev_a, (float *)p, na);
+        p += al256((size_t)T.a_stride * T.a_h * 4);
+        make_hull(tp, dev ? dev[k].rows : nullptr);
         if (tp.hull.empty())
             rc = set_err(ctx, ALN_ERR_ARG, "thumbnail pair %d: no A points", k);
         tp.best.X = tp.best.Y = tp.best.A = tp.best.R = -999.0;   // CThmScan::Initialize
@@ -951,9 +962,10 @@ extern "C" int aln_thm_finish_batch(aln_ctx *ctx, int npairs, const aln_thumbs *
 // One CThmScan member-function call per pair from the caller's object
 // state (best record, err, pretweak transform); see aln_thm_call_batch in
 // the header for the ops and their arguments.
-extern "C" int aln_thm_call_batch(aln_ctx *ctx, int npairs, const aln_thumbs *thumbs,
-                                  const aln_thm_params *params, int op, const double *args,
-                                  aln_thm_result *best, double *tptwk, double *ret)
+// dev: the thumbnails are on the device (ApproximateMatch).
+static int thm_call(aln_ctx *ctx, int npairs, const aln_thumbs *thumbs, const DevThumbs *dev,
+                    const aln_thm_params *params, int op, const double *args,
+                    aln_thm_result *best, double *tptwk, double *ret)
 {
     if (!ctx || npairs < 0 || (npairs && (!thumbs || !params || !args || !best)))
         return ctx ? set_err(ctx, ALN_ERR_ARG, "bad arguments") : ALN_ERR_ARG;
@@ -969,7 +981,7 @@ extern "C" int aln_thm_call_batch(aln_ctx *ctx, int npairs, const aln_thumbs *th
         P.usecorrr = 1;   // SetUseCorrR(true)
     SweepCtx S;
     char *dbuf = nullptr;
-    int rc = sweep_setup(ctx, S, npairs, thumbs, &P, &dbuf);
+    int rc = sweep_setup(ctx, S, npairs, thumbs, &P, &dbuf, dev);
     std::vector<int> all(npairs);
     std::vector<double> a0(npairs), rv(npairs, 0.0);
     std::vector<ThmRec> b0(npairs);
@@ -1121,6 +1133,13 @@ extern "C" int aln_thm_call_batch(aln_ctx *ctx, int npairs, const aln_thumbs *th
     return ALN_OK;
 }
 
+extern "C" int aln_thm_call_batch(aln_ctx *ctx, int npairs, const aln_thumbs *thumbs,
+                                  const aln_thm_params *params, int op, const double *args,
+                                  aln_thm_result *best, double *tptwk, double *ret)
+{
+    return thm_call(ctx, npairs, thumbs, nullptr, params, op, args, best, tptwk, ret);
+}
+
 // ---------------------------------------------------------------------------
 // MakeThumbs' binning and normalisation (1_DMesh/CThmUtil.cpp:470-523):
 // DecimateVector (0_GEN/Maths.cpp:1315-1364) and Normalize (:192-212)
@@ -1136,7 +1155,27 @@ struct DecJob {
     double sums[2];             // sum of v, sum of v^2 over the present bins
     int np;                     // present bins
     double sd;
+    int2 *rows;                 // device: each bin row's first and last present bin (or null)
 };
+
+// grid (ceil(max oh / 8), n), block 256: one warp per bin row
+__global__ void k_dec_rows(DecJob *jobs)
+{
+    const DecJob &J = jobs[blockIdx.y];
+    const int y = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (y >= J.oh)
+        return;
+    int lo = 0x7fffffff, hi = -1;
+    for (int x = lane; x < J.ow; x += 32)
+        if (J.pres[(long long)y * J.ow + x]) {
+            lo = min(lo, x);
+            hi = x;
+        }
+    lo = __reduce_min_sync(0xffffffff, lo);
+    hi = __reduce_max_sync(0xffffffff, hi);
+    if (lane == 0)
+        J.rows[y] = make_int2(hi < 0 ? -1 : lo, hi);
+}
 
 // Sum and count of one bin of integer pixels.  The sum is exact in any
 // order, so it is the double the reference's accumulation ends with.  Bins of
@@ -1525,20 +1564,20 @@ __global__ void k_normalize(DecJob *jobs)
             J.vals[k] = __ddiv_rn(__dsub_rn(J.vals[k], avg), sd);
 }
 
-extern "C" int aln_decimate_batch(aln_ctx *ctx, int n, const aln_image *in,
-                                  const unsigned char *const *mask, int lbin, int normalize,
-                                  double *const *out_vals, unsigned char *const *out_mask,
-                                  double *out_sd)
+// The binned (and normalised) images of n rasters on the device: jobs[k].vals,
+// .pres and, when rows is not null, each bin row's present span (on the host,
+// rows[k][y]).  *out receives the allocation that holds them.  With rows, the
+// copies of the rasters are given back and the stream is synchronised; without,
+// the caller synchronises before it reads jobs or frees *out.
+static int decimate_device(aln_ctx *ctx, int n, const aln_image *in,
+                           const unsigned char *const *mask, int lbin, int normalize,
+                           std::vector<DecJob> &jobs, std::vector<std::vector<int2>> *rows,
+                           char **out)
 {
-    if (!ctx || n < 0 || (n && (!in || !out_vals || !out_mask)) || lbin < 1)
-        return ctx ? set_err(ctx, ALN_ERR_ARG, "bad arguments") : ALN_ERR_ARG;
-    if (!n)
-        return ALN_OK;
-    if (n > 65535)   // one grid z index per image
-        return set_err(ctx, ALN_ERR_ARG, "at most 65535 images per call (%d)", n);
+    *out = nullptr;
     CK(cudaSetDevice(ctx->device));
-    std::vector<DecJob> jobs(n);
-    size_t bytes = 0;
+    jobs.assign(n, DecJob());
+    size_t ibytes = 0, vbytes = 0;
     int mw = 1, mh = 1;
     for (int k = 0; k < n; ++k) {
         const aln_image &I = in[k];
@@ -1554,44 +1593,50 @@ extern "C" int aln_decimate_batch(aln_ctx *ctx, int n, const aln_image *in,
         mw = std::max(mw, J.ow);
         mh = std::max(mh, J.oh);
         const size_t ib = (size_t)I.stride * I.h;
-        bytes += al256(ib * dtype_size(I.dtype)) + (mask && mask[k] ? al256(ib) : 0) +
-                 al256((size_t)J.ow * J.oh * 9);
+        ibytes += al256(ib * dtype_size(I.dtype)) + (mask && mask[k] ? al256(ib) : 0);
+        vbytes += al256((size_t)J.ow * J.oh * 9) + (rows ? al256((size_t)J.oh * sizeof(int2)) : 0);
     }
-    char *buf = nullptr;
-    {
-        cudaError_t e = cudaMalloc(&buf, bytes + al256((size_t)n * sizeof(DecJob)));
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return set_err(ctx, ALN_ERR_NOMEM, "decimation buffers: %s", cudaGetErrorString(e));
-        }
+    const size_t jbytes = al256((size_t)n * sizeof(DecJob));
+    char *ibuf = nullptr, *vbuf = nullptr;
+    vbytes += jbytes;
+    cudaError_t e = cudaMalloc(&vbuf, vbytes + (rows ? 0 : ibytes));
+    if (e == cudaSuccess && rows)
+        e = cudaMalloc(&ibuf, ibytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(vbuf);
+        return set_err(ctx, ALN_ERR_NOMEM, "decimation buffers: %s", cudaGetErrorString(e));
     }
     cudaStream_t st = ctx->stream;
-    char *p = buf;
+    char *p = rows ? ibuf : vbuf + vbytes, *v = vbuf;
     int rc = ALN_OK;
     for (int k = 0; k < n && rc == ALN_OK; ++k) {
         const aln_image &I = in[k];
         DecJob &J = jobs[k];
         const size_t ib = (size_t)I.stride * I.h;
+        const size_t nel = (size_t)I.stride * (I.h - 1) + I.w;   // first pixel to last
         // host or device sources alike (unified addressing)
-        if (cudaMemcpyAsync(p, I.data, ib * dtype_size(I.dtype), cudaMemcpyDefault, st) !=
+        if (cudaMemcpyAsync(p, I.data, nel * dtype_size(I.dtype), cudaMemcpyDefault, st) !=
             cudaSuccess)
             rc = set_err(ctx, ALN_ERR_CUDA, "image %d copy", k);
         J.img = p;
         p += al256(ib * dtype_size(I.dtype));
         J.mask = nullptr;
         if (mask && mask[k]) {
-            if (cudaMemcpyAsync(p, mask[k], ib, cudaMemcpyDefault, st) != cudaSuccess)
+            if (cudaMemcpyAsync(p, mask[k], nel, cudaMemcpyDefault, st) != cudaSuccess)
                 rc = set_err(ctx, ALN_ERR_CUDA, "mask %d copy", k);
             J.mask = (const unsigned char *)p;
             p += al256(ib);
         }
-        J.vals = (double *)p;
-        J.pres = (unsigned char *)(p + (size_t)J.ow * J.oh * 8);
-        p += al256((size_t)J.ow * J.oh * 9);
-        J.sums[0] = J.sums[1] = J.sd = 0.0;
-        J.np = 0;
+        J.vals = (double *)v;
+        J.pres = (unsigned char *)(v + (size_t)J.ow * J.oh * 8);
+        v += al256((size_t)J.ow * J.oh * 9);
+        if (rows) {
+            J.rows = (int2 *)v;
+            v += al256((size_t)J.oh * sizeof(int2));
+        }
     }
-    DecJob *dj = (DecJob *)p;
+    DecJob *dj = (DecJob *)v;
     if (rc == ALN_OK &&
         cudaMemcpyAsync(dj, jobs.data(), (size_t)n * sizeof(DecJob), cudaMemcpyHostToDevice,
                         st) != cudaSuccess)
@@ -1605,17 +1650,55 @@ extern "C" int aln_decimate_batch(aln_ctx *ctx, int n, const aln_image *in,
             LAUNCH(ctx, "k_normalize", k_normalize,
                    dim3((unsigned)std::min<long long>((mb + 1023) / 1024, 256), n), 256, 0, dj);
         }
-        for (int k = 0; k < n && rc == ALN_OK; ++k) {
-            const size_t nb = (size_t)jobs[k].ow * jobs[k].oh;
-            if (cudaMemcpyAsync(out_vals[k], jobs[k].vals, nb * 8, cudaMemcpyDefault, st) !=
-                    cudaSuccess ||
-                cudaMemcpyAsync(out_mask[k], jobs[k].pres, nb, cudaMemcpyDefault, st) !=
-                    cudaSuccess)
-                rc = set_err(ctx, ALN_ERR_CUDA, "result %d copy", k);
+        if (rows) {
+            LAUNCH(ctx, "k_dec_rows", k_dec_rows, dim3((mh + 7) / 8, n), 256, 0, dj);
+            rows->assign(n, std::vector<int2>());
+            for (int k = 0; k < n && rc == ALN_OK; ++k) {
+                (*rows)[k].resize(jobs[k].oh);
+                if (cudaMemcpyAsync((*rows)[k].data(), jobs[k].rows,
+                                    (size_t)jobs[k].oh * sizeof(int2), cudaMemcpyDeviceToHost,
+                                    st) != cudaSuccess)
+                    rc = set_err(ctx, ALN_ERR_CUDA, "row spans %d copy", k);
+            }
         }
         if (rc == ALN_OK && cudaMemcpyAsync(jobs.data(), dj, (size_t)n * sizeof(DecJob),
                                             cudaMemcpyDeviceToHost, st) != cudaSuccess)
             rc = set_err(ctx, ALN_ERR_CUDA, "job table read-back");
+    }
+    if ((rows || rc != ALN_OK) && cudaStreamSynchronize(st) != cudaSuccess && rc == ALN_OK)
+        rc = set_err(ctx, ALN_ERR_CUDA, "decimation");
+    cudaFree(ibuf);
+    if (rc != ALN_OK) {
+        cudaFree(vbuf);
+        return rc;
+    }
+    *out = vbuf;
+    return ALN_OK;
+}
+
+extern "C" int aln_decimate_batch(aln_ctx *ctx, int n, const aln_image *in,
+                                  const unsigned char *const *mask, int lbin, int normalize,
+                                  double *const *out_vals, unsigned char *const *out_mask,
+                                  double *out_sd)
+{
+    if (!ctx || n < 0 || (n && (!in || !out_vals || !out_mask)) || lbin < 1)
+        return ctx ? set_err(ctx, ALN_ERR_ARG, "bad arguments") : ALN_ERR_ARG;
+    if (!n)
+        return ALN_OK;
+    if (n > 65535)   // one grid z index per image
+        return set_err(ctx, ALN_ERR_ARG, "at most 65535 images per call (%d)", n);
+    std::vector<DecJob> jobs;
+    char *buf = nullptr;
+    int rc = decimate_device(ctx, n, in, mask, lbin, normalize, jobs, nullptr, &buf);
+    if (rc != ALN_OK)
+        return rc;
+    for (int k = 0; k < n && rc == ALN_OK; ++k) {
+        const size_t nb = (size_t)jobs[k].ow * jobs[k].oh;
+        if (cudaMemcpyAsync(out_vals[k], jobs[k].vals, nb * 8, cudaMemcpyDefault, ctx->stream) !=
+                cudaSuccess ||
+            cudaMemcpyAsync(out_mask[k], jobs[k].pres, nb, cudaMemcpyDefault, ctx->stream) !=
+                cudaSuccess)
+            rc = set_err(ctx, ALN_ERR_CUDA, "result %d copy", k);
     }
     cudaStreamSynchronize(ctx->stream);
     cudaFree(buf);
