@@ -808,30 +808,60 @@ k2_rowfft(PairDev *pairs, const float2 *__restrict__ tw, int only_img, const int
         // the region's first 16-byte boundary (at most 8 bytes in): the row's
         // <= 4L + 30 staged bytes end inside the region (rowfft_pitch)
         unsigned char *sb = (unsigned char *)(((uintptr_t)sm + 15) & ~(uintptr_t)15);
-        int off = 0;
+        int at = 0;   // the staged row's first byte
         if (y < h) {
             const unsigned char *base = (const unsigned char *)img + (long long)y * st * es;
             const uintptr_t a0 = (uintptr_t)base & ~(uintptr_t)15;
-            off = (int)((uintptr_t)base - a0);
-            const int nvec = (off + w * es + 15) >> 4;
+            const int off = (int)((uintptr_t)base - a0), nb = w * es;
+            const int nvec = (off + nb + 15) >> 4;
             const uint4 *src = (const uint4 *)a0;
-            for (int k = t; k < nvec; k += T)
-                ((uint4 *)sb)[k] = src[k];
+            // a thread reads its pixel pairs as one 2- or 4-byte word: a row that
+            // starts between such words is staged shifted onto one
+            const int odd = off & (2 * es - 1);
+            at = off - odd;
+            if (odd == 0) {
+                for (int k = t; k < nvec; k += T)
+                    ((uint4 *)sb)[k] = src[k];
+            } else {
+                for (int k = t; k < nvec; k += T) {
+                    const uint4 v4 = src[k];
+                    const unsigned nx = k + 1 < nvec ? *(const unsigned *)(src + k + 1) : 0u;
+                    ((uint4 *)sb)[k] = make_uint4(__funnelshift_r(v4.x, v4.y, 8 * odd),
+                                                  __funnelshift_r(v4.y, v4.z, 8 * odd),
+                                                  __funnelshift_r(v4.z, v4.w, 8 * odd),
+                                                  __funnelshift_r(v4.w, nx, 8 * odd));
+                }
+            }
+        }
+        team_sync<T>(team);
+        if (y < h) {   // the padding holds mu, which becomes 0
+            if (es == 1)
+                for (int k = w + t; k < 2 * L; k += T)
+                    sb[at + k] = (unsigned char)mu;
+            else
+                for (int k = w + t; k < 2 * L; k += T)
+                    *(unsigned short *)(sb + at + 2 * k) = (unsigned short)mu;
         }
         team_sync<T>(team);   // each team reads back its own row only
-        const unsigned char *rb8 = sb + off;
+        // (rows past the image read what is there: their bins are not stored)
+        const unsigned char *row = sb + at;
+        // 2^23 + pixel is the float with the pixel as its last bits: less 2^23 + mu
+        // it is the shifted pixel, exactly, without a conversion
+        const float bias = 8388608.0f + (float)mu;
+        if (es == 1) {
 #pragma unroll
-        for (int q = 0; q < V; ++q) {
-            const int n = F::in_idx(t, q);
-            float2 z = make_float2(0.f, 0.f);
-            if (y < h) {
-                const int xa = 2 * n, xb = 2 * n + 1;
-                if (xa < w)
-                    z.x = (float)((es == 1 ? (int)rb8[xa] : (int)((const uint16_t *)rb8)[xa]) - mu);
-                if (xb < w)
-                    z.y = (float)((es == 1 ? (int)rb8[xb] : (int)((const uint16_t *)rb8)[xb]) - mu);
+            for (int q = 0; q < V; ++q) {
+                const unsigned d = *(const unsigned short *)(row + 2 * F::in_idx(t, q));
+                v[q].x = __uint_as_float(__byte_perm(d, 0x4b000000u, 0x7440)) - bias;
+                v[q].y = __uint_as_float(__byte_perm(d, 0x4b000000u, 0x7441)) - bias;
             }
-            v[q] = z;
+        } else {
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+                const unsigned d = *(const unsigned *)(row + 4 * F::in_idx(t, q));
+                v[q].x = __uint_as_float(__byte_perm(d, 0x4b000000u, 0x7410)) - bias;
+                v[q].y = __uint_as_float(__byte_perm(d, 0x4b000000u, 0x7432)) - bias;
+            }
         }
     } else if (dt == ALN_F32) {
         // the shift is an FP32 number (k_mean), and the FP64 difference of two
@@ -889,22 +919,19 @@ k2_rowfft(PairDev *pairs, const float2 *__restrict__ tw, int only_img, const int
     float2 *lo = p.T[i] + y0 + rr + kx0 * Ts;          // bin kx
     float2 *hi = p.T[i] + y0 + rr + (L - kx0) * Ts;    // bin L - kx
     const float2 *twk = tw + tw_base(2 * L) + 2 * L;   // exp(-2 pi i k / 2L) at twk[k]
+    // With A = Z[kx], B = Z[L - kx], e the even and d the odd part's spectrum at
+    // kx, both bins need one product t = -i d w(kx): bin kx is e + t, and bin
+    // L - kx, where w(L - kx) = -conj(w(kx)), is conj(e - t).
     for (int kx = kx0; kx <= L / 2; kx += THR / G, lo += (THR / G) * Ts, hi -= (THR / G) * Ts) {
         const float2 A = Z[kx];
         const float2 B = Z[kx == 0 ? 0 : L - kx];
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int k = hh ? L - kx : kx;
-            if (hh && k == kx)
-                break;   // kx = L/2: one bin
-            const float2 a = hh ? B : A;
-            const float2 b = cconj(hh ? A : B);
-            const float2 ev = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y));
-            const float2 dd = make_float2(0.5f * (a.x - b.x), 0.5f * (a.y - b.y));
-            const float2 o = make_float2(dd.y, -dd.x);
-            const float2 wv = __ldg(&twk[k]);
-            *(hh ? hi : lo) = cadd(ev, cmul(o, wv));
-        }
+        const float2 ev = make_float2(0.5f * (A.x + B.x), 0.5f * (A.y - B.y));
+        const float2 dd = make_float2(0.5f * (A.x - B.x), 0.5f * (A.y + B.y));
+        const float2 o = make_float2(dd.y, -dd.x);
+        const float2 tt = cmul(o, __ldg(&twk[kx]));
+        *lo = cadd(ev, tt);
+        if (kx != L / 2)
+            *hi = make_float2(ev.x - tt.x, tt.y - ev.y);
     }
 }
 
