@@ -1157,41 +1157,52 @@ k2_corrseg(PairDev *pairs, const float2 *__restrict__ tw)
     const int B = p.seg_len, nseg = p.nseg, ylo = p.ylo;
     const int Wy = p.yhi - p.ylo + 1;
     const int lb = B + Wy - 1;
-    for (int s = 0; s < nseg; ++s) {
-        const int y0 = s * B;
-        // b's loads are in flight while a is transformed: at radix 8 they take
-        // the registers that a's spectrum holds while b is transformed (waiting
-        // for each load in turn left the warps on the long scoreboard, 2.7 stalled
-        // per issue: 4096 strips 9.50 -> 8.97 ms)
-        float2 va[R], vb[R];
+    auto load_a = [&](int s, float2 *v) {
+        const int y0 = s * B, n = min(B, ha - y0);
+        const float2 *src = Ta + y0 + t;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int j = t + r * T, y = y0 + j;
-            va[r] = (j < B && y < ha) ? Ta[y] : make_float2(0.f, 0.f);
-        }
-        auto load_b = [&]() {
+        for (int r = 0; r < R; ++r)
+            v[r] = t + r * T < n ? src[r * T] : make_float2(0.f, 0.f);
+    };
+    auto load_b = [&](int s, float2 *v) {
+        const int y0 = s * B + ylo, lo = max(0, -y0);
+        const unsigned n = (unsigned)max(0, min(lb, hb - y0) - lo);
+        const float2 *src = Tb + y0 + t;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            v[r] = (unsigned)(t + r * T - lo) < n ? src[r * T] : make_float2(0.f, 0.f);
+    };
+    float2 va[R], vb[R];
+    if constexpr (REGS)
+        load_a(0, va);
+    for (int s = 0; s < nseg; ++s) {
+        if constexpr (REGS) {
+            // b's loads are in flight while a is transformed, the next segment's
+            // a while b is (waiting for each load in turn left the warps on the
+            // long scoreboard, 2.7 stalled per issue: 4096 strips 9.50 -> 8.12 ms)
+            load_b(s, vb);
+            FF::run_team(va, sm, t, tw, team);
+            float2 na[R];
+            load_a(s + 1 < nseg ? s + 1 : s, na);
+            FF::run_team(vb, sm, t, tw, team);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const int j = t + r * T, y = y0 + ylo + j;
-                vb[r] = (j < lb && y >= 0 && y < hb) ? Tb[y] : make_float2(0.f, 0.f);
+                const float2 q = cmulc(vb[r], va[r]);   // X2 * conj(X1)
+                accr[r] = s == 0 ? q : cadd(accr[r], q);
+                va[r] = na[r];
             }
-        };
-        if constexpr (REGS)
-            load_b();
-        FF::run_team(va, sm, t, tw, team);
-        if constexpr (!REGS) {
+        } else {
+            load_a(s, va);
+            fresh(tw);
+            FF::run_team(va, sm, t, tw, team);
 #pragma unroll
             for (int r = 0; r < R; ++r)
                 park[r * T + t] = va[r];
-            load_b();
-        }
-        FF::run_team(vb, sm, t, tw, team);
+            load_b(s, vb);
+            fresh(tw);
+            FF::run_team(vb, sm, t, tw, team);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if constexpr (REGS) {
-                const float2 q = cmulc(vb[r], va[r]);   // X2 * conj(X1)
-                accr[r] = s == 0 ? q : cadd(accr[r], q);
-            } else {
+            for (int r = 0; r < R; ++r) {
                 const float2 q = cmulc(vb[r], park[r * T + t]);
                 acc[r * T + t] = s == 0 ? q : cadd(acc[r * T + t], q);
             }
@@ -1205,6 +1216,8 @@ k2_corrseg(PairDev *pairs, const float2 *__restrict__ tw)
         else
             v[r] = acc[r * T + t];
     }
+    if constexpr (!REGS)
+        fresh(tw);
     FI::run_team(v, sm, t, tw, team);
     if (live) {
         float2 *Q = p.Q + (long long)kx * Wy;
