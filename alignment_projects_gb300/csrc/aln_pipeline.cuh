@@ -24,6 +24,17 @@
 
 __device__ __forceinline__ bool int_pixels(int dt) { return dt == ALN_U8 || dt == ALN_U16; }
 
+// The table pointer as if new: the next transform loads its twiddles again.
+// Without it the compiler kept up to 60 registers of them from one transform
+// to the next of the radix-16 column kernels and spilled as much (k2_corrcol
+// 2.38 -> 2.13 ms and k2_corrseg 1.30 -> 1.16 ms per 3000 uneven pairs,
+// k2_corrcol of the coarse scan of 48 thumbnail pairs 7.83 -> 7.22 ms; the
+// radix-8 segments ran 2 % slower with it).
+__device__ __forceinline__ void fresh(const float2 *__restrict__ &tw)
+{
+    asm volatile("" : "+l"(tw));
+}
+
 // asynchronous copies, global -> shared without registers
 __device__ __forceinline__ void cp_async8(void *dst_shared, const void *src_global)
 {
@@ -1017,6 +1028,7 @@ k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
             va[r] = y < ha ? Ta[y] : make_float2(0.f, 0.f);
         }
     }
+    fresh(tw);
     FF::run_team(va, sm, t, tw, team);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -1039,16 +1051,18 @@ k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
     }
     // CorrPatches / CorrImagesR need the plain inverse; CorrImagesS the inverse
     // of the whitened product P / sqrt(|P|) (0_GEN/Correlation.cpp:2311-2317)
-    const bool want_r = PLAIN || (!SONLY && (p.mode == JOB_PATCHES || is_p2i || p.want_r));
+    // (always so for the plain form: as a run-time condition it keeps the inverse's
+    // twiddle loads out of the forward transform, where they cost 150 bytes of
+    // spills)
+    const bool want_r = PLAIN ? p.mode == JOB_PATCHES : (!SONLY && (p.mode == JOB_PATCHES || is_p2i || p.want_r));
     const bool want_s = SONLY || (!PLAIN && p.want_s != 0);
     if (want_r && want_s) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
             sb[r * T + t] = va[r];
     }
-    const int Wy = p.yhi - p.ylo + 1;
-    const int nnegy = p.h[0] - 1;
     if (want_r) {
+        fresh(tw);
         FI::run_team(va, sm, t, tw, team);
         if (live && is_p2i) {   // every storage row, in storage order
             float2 *Q = p.Q + (long long)kx * NY;
@@ -1056,13 +1070,14 @@ k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
             for (int r = 0; r < R; ++r)
                 Q[t + r * T] = va[r];
         } else if (live) {
+            const int ylo = p.ylo, Wy = p.yhi - ylo + 1, nnegy = p.h[0] - 1;
             float2 *Q = p.Q + (long long)kx * Wy;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const int ys = t + r * T;
-                const int y = ys >= NY - nnegy ? ys - NY : ys;
-                if (y >= p.ylo && y <= p.yhi)
-                    Q[y - p.ylo] = va[r];
+                const int j = (ys >= NY - nnegy ? ys - NY : ys) - ylo;
+                if ((unsigned)j < (unsigned)Wy)
+                    Q[j] = va[r];
             }
         }
     }
@@ -1077,15 +1092,17 @@ k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
             }
             va[r] = v;
         }
+        fresh(tw);
         FI::run_team(va, sm, t, tw, team);
         if (live) {
+            const int ylo = p.ylo, Wy = p.yhi - ylo + 1, nnegy = p.h[0] - 1;
             float2 *Q = (want_r ? p.Q2 : p.Q) + (long long)kx * Wy;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const int ys = t + r * T;
-                const int y = ys >= NY - nnegy ? ys - NY : ys;
-                if (y >= p.ylo && y <= p.yhi)
-                    Q[y - p.ylo] = va[r];
+                const int j = (ys >= NY - nnegy ? ys - NY : ys) - ylo;
+                if ((unsigned)j < (unsigned)Wy)
+                    Q[j] = va[r];
             }
         }
     }
