@@ -2843,18 +2843,20 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
     // window, jobs are grouped by FFT size and job kind (submission order
     // kept) and split into chunks bounded by the workspace budget.
     // Device-resident inputs need no staging: then the whole batch is one
-    // window.  Host batches of at least 512 MB are cut into about four
-    // windows (at least 128 MB each), so only the first window's copy is not
+    // window.  Host batches of at least 128 MB are cut into about four
+    // windows (at least 64 MB each), so only the first window's copy is not
     // hidden behind computation: at the host link's ~210 GB/s a window's
-    // copy takes half the time of its kernels for the montage strips.  (Eight
-    // and sixteen windows measured slower end to end on the montage batch:
-    // 96.9k and 85.9k pairs/s against 98.8k with four.)
+    // copy takes half the time of its kernels for the montage strips.  (Strips
+    // of 2048 px, one window against this rule: 135 MB 1.71 / 1.71 ms, 193 MB
+    // 2.43 / 2.28, 260 MB 3.19 / 2.97, 366 MB 4.41 / 3.91, 493 MB 5.77 / 4.94.
+    // Eight and sixteen windows measured slower on the 4096-pair batch: 96.9k
+    // and 85.9k pairs/s against 98.8k with four.)
     size_t host_bytes = 0;
     for (const auto &pl : plans)
         if (pl.d.status == 0)
             host_bytes += pl.in_bytes[0] + pl.in_bytes[1];
-    const size_t win_cap = host_bytes >= ((size_t)512 << 20)
-                               ? std::max((size_t)128 << 20, (host_bytes + 3) / 4)
+    const size_t win_cap = host_bytes >= ((size_t)128 << 20)
+                               ? std::max((size_t)64 << 20, (host_bytes + 3) / 4)
                                : std::max((size_t)64 << 20, ctx->ws_budget * 4);
     std::vector<std::vector<PairPlan *>> windows(1);
     {
