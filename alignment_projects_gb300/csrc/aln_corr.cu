@@ -491,18 +491,10 @@ __global__ void k_colsum(PairDev *pairs)
     }
 }
 
-// grid (2, npairs), block 256: deterministic total -> mean shift
-__global__ void k_mean(PairDev *pairs)
+// Image i's mean shift from its column totals, by a block of 256 threads
+// (deterministic).  All threads of the block must call it.
+__device__ __forceinline__ void mean_shift(PairDev &p, int i)
 {
-    PairDev &p = pairs[blockIdx.y];
-    const int i = blockIdx.x;
-    if (p.status != 0)
-        return;
-    if (p.sat_nonly) {   // no value sums: CorrImagesS correlates unshifted images
-        if (threadIdx.x == 0)
-            p.mu[i] = 0.0;
-        return;
-    }
     __shared__ double part[256];
     double s = 0.0;
     for (int c = threadIdx.x; c < p.w[i]; c += blockDim.x)
@@ -521,6 +513,14 @@ __global__ void k_mean(PairDev *pairs)
             mu = (double)(float)mu;   // exactly representable in the FP32 row pass
         p.mu[i] = p.no_shift ? 0.0 : mu;
     }
+}
+
+// grid (2, npairs), block 256
+__global__ void k_mean(PairDev *pairs)
+{
+    PairDev &p = pairs[blockIdx.y];
+    if (p.status == 0)
+        mean_shift(p, blockIdx.x);
 }
 
 // grid (maxslots, 2, npairs), block 256: inclusive x-prefix of one needed row
@@ -2468,7 +2468,7 @@ static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, 
     return (size_t)(work - work_base);
 }
 
-// Transposes, summed-area tables and mean shifts of a span of jobs (its job
+// Transposes, summed-area tables and mean shifts (k2_sat2w) of a span of jobs (its job
 // table, fill lists and staged inputs are already on the device, in stream
 // order).  These kernels do not depend on the transform lengths, so one launch
 // covers the chunks of several grids.
@@ -2499,7 +2499,6 @@ static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *>
     if (sp.plain)
         LAUNCH(ctx, "k3_sat", k3_sat, dim3((sp.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS), 0,
                ctx->dpairs);
-    LAUNCH(ctx, "k_mean", k_mean, dim3(2, n), 256, 0, ctx->dpairs);
     if (sonly)
         LAUNCH(ctx, "k2_sat2w", k2_sat2w<true>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
                ctx->dpairs);

@@ -4,7 +4,7 @@
 //
 //   k3_sat    per 32-column band: warp-local column prefix sums of v, v^2,
 //             (v != 0) at the needed rows, per-warp offsets; column totals
-//             (k_mean turns them into mu)
+//             (k2_sat2w turns them into mu)
 //   k2_sat2w  per needed row: add the warp offset, x-prefix -> SAT row
 //   k2_rowfft<L>   rows: (v - mu), zero pad, real FFT of length 2L, [kx][y]
 //   k2_corrcol<Ny> per column kx: FFT of b's column (or the cached spectrum),
@@ -752,16 +752,23 @@ __device__ __forceinline__ void sat2_row_counts(const PairDev &p, int i, int slo
     }
 }
 
-// grid (ceil(maxslots / 8), 2, npairs), block 256: warp k takes slot 8*bx + k.
+// grid (ceil(maxslots / 8), 2, npairs), block 256: warp k takes slot 8*bx + k;
+// an image's first block also makes its mean shift (a launch of its own for two
+// sums took 7 of a single pair's 105 us).  CorrImagesS without a mincor has no
+// value sums and correlates unshifted images: its mu stays 0.
 // NONLY: the form launched for chunks of counts-only jobs (its registers are
 // not sized for the int64 tables).
 template <bool NONLY>
 __global__ void k2_sat2w(PairDev *pairs)
 {
-    const PairDev &p = pairs[blockIdx.z];
+    PairDev &p = pairs[blockIdx.z];
     const int i = blockIdx.y;
     const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (p.status != 0 || slot >= nslots(p, i) || (i == 1 && p.sat_shared))
+    if (p.status != 0)
+        return;
+    if (!NONLY && blockIdx.x == 0 && !p.sat_nonly)
+        mean_shift(p, i);
+    if (slot >= nslots(p, i) || (i == 1 && p.sat_shared))
         return;
     const int len0 = p.need_hi[i][0] - p.need_lo[i][0] + 1;
     const int y = slot < len0 ? p.need_lo[i][0] + slot : p.need_lo[i][1] + slot - len0;

@@ -726,17 +726,20 @@ static int sweep_setup(aln_ctx *ctx, SweepCtx &S, int npairs, const aln_thumbs *
     S.pairs.resize(npairs);
     S.key_base = (++ctx->sweep_serial) << 32;
     // device copies of the thumbnails
-    size_t bytes = 0;
+    auto al512 = [](size_t x) { return (x + 511) & ~(size_t)511; };
+    size_t bytes = 0, abytes = 0;
     for (int k = 0; k < npairs; ++k) {
         const aln_thumbs &T = thumbs[k];
         if (!T.a || T.a_w < 1 || T.a_h < 1 || T.a_stride < T.a_w || !T.b.data ||
             T.b.dtype != ALN_F64 || T.b.w < 1 || T.b.h < 1 || T.b.stride < T.b.w)
             return set_err(ctx, ALN_ERR_ARG, "thumbnail pair %d: bad grid/raster", k);
-        bytes += al256((size_t)T.a_stride * T.a_h * 4);
+        // A's values: FP64 copies back to back, FP32 ones behind them at half
+        // the offsets, so that one launch converts every pair's
+        abytes += al512((size_t)T.a_stride * T.a_h * 8);
         if (!dev)
-            bytes += al256((size_t)T.a_stride * T.a_h * 8) + al256((size_t)T.a_stride * T.a_h) +
-                     al256((size_t)T.b.stride * T.b.h * 8);
+            bytes += al256((size_t)T.a_stride * T.a_h) + al256((size_t)T.b.stride * T.b.h * 8);
     }
+    bytes += (dev ? 0 : abytes) + abytes / 2;
     char *dbuf = nullptr;
     if (bytes) {
         cudaError_t e = cudaMalloc(&dbuf, bytes);
@@ -745,7 +748,9 @@ static int sweep_setup(aln_ctx *ctx, SweepCtx &S, int npairs, const aln_thumbs *
             return set_err(ctx, ALN_ERR_NOMEM, "thumbnails: %s", cudaGetErrorString(e));
         }
     }
-    char *p = dbuf;
+    char *const a64 = dbuf, *const a32 = dbuf + (dev ? 0 : abytes);
+    char *p = a32 + abytes / 2;
+    size_t aoff = 0;   // of this pair's A in the FP64 copies
     int rc = ALN_OK;
     for (int k = 0; k < npairs && rc == ALN_OK; ++k) {
         const aln_thumbs &T = thumbs[k];
@@ -757,37 +762,43 @@ static int sweep_setup(aln_ctx *ctx, SweepCtx &S, int npairs, const aln_thumbs *
         // elements from the first point to the last one
         const size_t na = (size_t)T.a_stride * (T.a_h - 1) + T.a_w;
         const size_t nbr = (size_t)T.b.stride * (T.b.h - 1) + T.b.w;
-        const double *dev_a = T.a;
         tp.dev_mask = T.a_mask;
         tp.dev_b = T.b;
         tp.dev_b.on_device = 1;
-        auto copy = [&](const void *src, size_t n, size_t room, const char *what) -> const void * {
-            if (cudaMemcpyAsync(p, src, n, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
+        auto copy = [&](char *to, const void *src, size_t n, const char *what) {
+            if (cudaMemcpyAsync(to, src, n, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
                 rc = set_err(ctx, ALN_ERR_CUDA, "%s copy", what);
             ctx->h2d_bytes += (long long)n;
-            const void *q = p;
-            p += al256(room);
-            return q;
         };
-        if (!dev) {
-            const size_t room = (size_t)T.a_stride * T.a_h;
-            dev_a = (const double *)copy(T.a, na * 8, room * 8, "thumbnail");
-            if (T.a_mask)
-                tp.dev_mask = (const unsigned char *)copy(T.a_mask, na, room, "mask");
-            tp.dev_b.data = copy(T.b.data, nbr * 8, (size_t)T.b.stride * T.b.h * 8, "thumbnail");
-        }
-        // the splat multiplies in FP32: convert once here instead of per
+        // the splat multiplies in FP32: converted once here instead of per
         // gathered point (FP64 conversions run on the narrow FP64 pipe)
-        tp.dev_af = (const float *)p;
-        LAUNCH(ctx, "k_f64_to_f32", k_f64_to_f32,
-               (unsigned)std::min<size_t>((na + 255) / 256, 1024), 256, 0, dev_a, (float *)p, na);
-        p += al256((size_t)T.a_stride * T.a_h * 4);
+        tp.dev_af = (const float *)(a32 + aoff / 2);
+        if (!dev) {
+            copy(a64 + aoff, T.a, na * 8, "thumbnail");
+            if (T.a_mask) {
+                copy(p, T.a_mask, na, "mask");
+                tp.dev_mask = (const unsigned char *)p;
+            }
+            p += al256((size_t)T.a_stride * T.a_h);
+            copy(p, T.b.data, nbr * 8, "thumbnail");
+            tp.dev_b.data = p;
+            p += al256((size_t)T.b.stride * T.b.h * 8);
+        } else {
+            LAUNCH(ctx, "k_f64_to_f32", k_f64_to_f32,
+                   (unsigned)std::min<size_t>((na + 255) / 256, 1024), 256, 0, T.a,
+                   (float *)(a32 + aoff / 2), na);
+        }
+        aoff += al512((size_t)T.a_stride * T.a_h * 8);
         make_hull(tp, dev ? dev[k].rows : nullptr);
         if (tp.hull.empty())
             rc = set_err(ctx, ALN_ERR_ARG, "thumbnail pair %d: no A points", k);
         tp.best.X = tp.best.Y = tp.best.A = tp.best.R = -999.0;   // CThmScan::Initialize
         tp.own_disc = 0;
     }
+    if (!dev && rc == ALN_OK && abytes)   // (between the pairs: what is there)
+        LAUNCH(ctx, "k_f64_to_f32", k_f64_to_f32,
+               (unsigned)std::min<size_t>((abytes / 8 + 255) / 256, 4096), 256, 0,
+               (const double *)a64, (float *)a32, abytes / 8);
     *dbuf_out = dbuf;
     return rc;
 }
