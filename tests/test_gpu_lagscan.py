@@ -149,3 +149,18 @@ def test_corr_images_r_bound(ctx, orc, data, rule):
     o = orc.corr_images(1, pts[0], a.ravel().astype(np.float64), pts[1],
                         b.ravel().astype(np.float64), lg, mincor, 0.75, *disc)
     check(g, o, 1, (data, rule))
+
+
+@pytest.mark.parametrize("w,h", [(33, 5), (127, 31), (128, 32), (129, 33), (131, 64), (512, 30),
+                                 (513, 97), (640, 36), (1030, 203)])
+@pytest.mark.parametrize("col", [0, 1, 2])
+def test_transposed_solve(ctx, w, h, col):
+    """A wide pair is solved on its transposed images: the same as the pair
+    handed over transposed, at tile edges, odd sizes, starts and strides."""
+    rng = np.random.default_rng(w + h + col)
+    a, b = _pair(rng, w, h)
+    wide = dict(a=_view(a, col, w + 3 * col), b=_view(b, col, w + 3 * col), radius=20)
+    tall = dict(a=np.ascontiguousarray(a.T), b=np.ascontiguousarray(b.T), radius=20)
+    g, t = ctx.corr_patches_batch([wide, tall])
+    assert (g["r"], g["dx"], g["dy"], g["peak_x"], g["peak_y"]) == \
+        (t["r"], t["dy"], t["dx"], t["peak_y"], t["peak_x"])
