@@ -3,13 +3,14 @@
 // CorrImagesF/R/S, CorrPatchToImage, the FFT_2D / IFT_2D / Convolve drop-ins
 // and the C ABI of include/aln_corr.h.
 //
-// The batched pipeline (aln_pipeline.cuh) runs each chunk of jobs sharing a
-// transform grid: k_transpose (wide jobs), k3_sat + k_mean + k2_sat2w
-// (summed-area-table rows the lag window needs, mean shifts), k2_rowfft
-// (row spectra T[kx][y]), k2_corrcol or k2_corrseg (column transforms,
-// spectral product, inverse; the window's lag rows -> Q), k2_lagrow /
-// k2_lagimg / k2_lagp2i (inverse rows, r or S per lag, legality, row argmax),
-// k_final* (argmax, ParabPeakFFT / ParabPeak, S score).  The CThmScan sweep
+// The batched pipeline (aln_pipeline.cuh) runs spans of jobs through
+// k_transpose (wide jobs), k3_sat / k3_satp + k2_sat2w (summed-area-table rows
+// the lag window needs, mean shifts); each chunk of jobs sharing a transform
+// grid through k2_rowfft (row spectra T[kx][y]), k2_corrcol or k2_corrseg
+// (column transforms, spectral product, inverse; the window's lag rows -> Q)
+// and k2_lagrow / k2_lagss / k2_lagimg / k2_lagp2i (inverse rows); then
+// k2_lagscan / k2_imgscan (r per lag, legality, row argmax) and k_final*
+// (argmax, ParabPeakFFT / ParabPeak, S score).  The CThmScan sweep
 // (aln_sweep.cuh) and the request server (aln_server.cuh) drive it.
 //
 // The kernels defined in this file are the shared-memory FFT path: FFT_2D /

@@ -3,9 +3,11 @@
 // the device helpers (load_px, sat slots, lag_r, best_merge).
 //
 //   k3_sat    per 32-column band: warp-local column prefix sums of v, v^2,
-//             (v != 0) at the needed rows, per-warp offsets; column totals
-//             (k2_sat2w turns them into mu)
-//   k2_sat2w  per needed row: add the warp offset, x-prefix -> SAT row
+//             (v != 0) at the needed rows, per-warp offsets, column totals
+//   k3_satp   the same for 8-bit pairs whose sums pack into 64 bits, in bands
+//             of 64 columns copied to shared memory asynchronously
+//   k2_sat2w  per needed row: add the warp offset, x-prefix -> SAT row; the
+//             column totals -> mu
 //   k2_rowfft<L>   rows: (v - mu), zero pad, real FFT of length 2L, [kx][y]
 //   k2_corrcol<Ny> per column kx: FFT of b's column (or the cached spectrum),
 //             FFT of a's column, X2 * conj(X1), inverse FFT, the window's
@@ -15,6 +17,7 @@
 //             summed per column, one inverse
 //   k2_lagrow<L>   per lag row: inverse real FFT -> the lag image
 //   k2_lagscan     per lag row: r per lag, row argmax
+//   k2_imgscan     the same for CorrImagesR (bounded in FP32, FP64 where it counts)
 //   k2_lagimg / k2_lagss / k2_lagp2i, k_final_img / k_makef / k_fpeak / k_final_p2i:
 //             the CorrImages and CorrPatchToImage ends of the pipeline
 #pragma once
@@ -904,7 +907,7 @@ k2_rowfft(PairDev *pairs, const float2 *__restrict__ tw, int only_img, const int
             }
         }
     } else if (dt == ALN_F32) {
-        // the shift is an FP32 number (k_mean), and the FP64 difference of two
+        // the shift is an FP32 number (mean_shift), and the FP64 difference of two
         // FP32 numbers rounds to FP32 as the FP32 difference does: no FP64
         // instruction (they held this kernel's sweep rows at 50 % of that pipe)
         const float mu = (float)p.mu[i];
