@@ -440,6 +440,17 @@ __device__ __forceinline__ int isqrt_ll(long long v)
     return (int)s;
 }
 
+// First statement of the batched pipeline's kernels (launch_dep): wait until
+// the kernel before has ended and its writes are visible, then let the next
+// kernel's blocks take the places that this one's leave free.  Every block
+// waits before it does anything, so a kernel's end means that all kernels
+// before it have ended too.
+__device__ __forceinline__ void grid_dep()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------
 // summed-area tables and mean shift
 // ---------------------------------------------------------------------------
@@ -934,6 +945,7 @@ __device__ double stored_value(const PairDev &p, int xs, int ys, bool raw)
 // grid (npairs), block 256; p.fin bit 2: see stored_value's raw
 __global__ void k_final(PairDev *pairs, ResultDev *res)
 {
+    grid_dep();
     __shared__ double red_r[32];
     __shared__ long long red_k[32];
     __shared__ double near[4];
@@ -1259,6 +1271,48 @@ static void prof_collect(aln_ctx *c)
     do {                                                                             \
         prof_begin(c, name);                                                         \
         kern<<<grid, block, smem, (c)->stream>>>(__VA_ARGS__);                       \
+        prof_end(c);                                                                 \
+    } while (0)
+
+static int sm_count(aln_ctx *ctx)
+{
+    if (!ctx->sms) {
+        cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        ctx->sms = std::max(ctx->sms, 1);
+    }
+    return ctx->sms;
+}
+
+// The same for the batched pipeline's kernels, whose first statement is
+// grid_dep(): the launch may overlap the end of the kernel before it.  A small
+// batch is a chain of dependent launches of 8-17 us each, where a kernel's
+// ramp counts: one 235 x 2048 pair 101 -> 86 us, 3000 uneven pairs in 74 grids
+// 15.7 -> 15.2 ms.  Grids of many waves have nothing to gain from it, and 4096
+// strips ran 0.6 % slower with it (22.92 -> 23.06 ms, their blocks filling
+// first the multiprocessors that were free first): they wait as usual.
+constexpr int DEP_BLOCKS_PER_SM = 64;
+template <class... P, class... A>
+static void launch_dep(aln_ctx *c, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                       A &&...args)
+{
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed =
+        (size_t)grid.x * grid.y * grid.z <= (size_t)DEP_BLOCKS_PER_SM * sm_count(c);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+#define LAUNCH_DEP(c, name, kern, grid, block, smem, ...)                            \
+    do {                                                                             \
+        prof_begin(c, name);                                                         \
+        launch_dep(c, kern, grid, block, smem, __VA_ARGS__);                         \
         prof_end(c);                                                                 \
     } while (0)
 
@@ -2122,15 +2176,6 @@ static size_t carve(PairPlan &pl, char *base, const aln_pair &P)
     return (size_t)(p - base);
 }
 
-static int sm_count(aln_ctx *ctx)
-{
-    if (!ctx->sms) {
-        cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
-        ctx->sms = std::max(ctx->sms, 1);
-    }
-    return ctx->sms;
-}
-
 static int rows_per_cta(int L) { return std::max(1, std::min(16, 4096 / L)); }
 static int cols_per_cta(int Ny) { return std::max(1, std::min(16, 4096 / Ny)); }
 
@@ -2141,8 +2186,8 @@ static void launch_rowfft2(aln_ctx *ctx, int n, int maxh)
     const int thr = rowfft_threads(T), G = thr / T;
     const size_t sm = ((size_t)G * rowfft_pitch<LL>() + 16) * sizeof(float2);
     smem_attr(ctx->device, (const void *)k2_rowfft<LL>, sm);
-    LAUNCH(ctx, "k2_rowfft", k2_rowfft<LL>, dim3((maxh + G - 1) / G, 2, n), thr, sm,
-           ctx->dpairs, ctx->tw, -1, (const int *)nullptr);
+    LAUNCH_DEP(ctx, "k2_rowfft", k2_rowfft<LL>, dim3((maxh + G - 1) / G, 2, n), thr, sm,
+               ctx->dpairs, ctx->tw, -1, (const int *)nullptr);
 }
 
 // spectrum-cache fills: b's rows and columns of the selected jobs -> X2
@@ -2153,8 +2198,8 @@ static void launch_fill_rows(aln_ctx *ctx, int nsel, int maxh)
     const int thr = rowfft_threads(T), G = thr / T;
     const size_t sm = ((size_t)G * rowfft_pitch<LL>() + 16) * sizeof(float2);
     smem_attr(ctx->device, (const void *)k2_rowfft<LL>, sm);
-    LAUNCH(ctx, "k2_rowfft", k2_rowfft<LL>, dim3((maxh + G - 1) / G, 1, nsel), thr, sm,
-           ctx->dpairs, ctx->tw, 1, (const int *)ctx->dsel_cur);
+    LAUNCH_DEP(ctx, "k2_rowfft", k2_rowfft<LL>, dim3((maxh + G - 1) / G, 1, nsel), thr, sm,
+               ctx->dpairs, ctx->tw, 1, (const int *)ctx->dsel_cur);
 }
 
 template <int NY, int RAD>
@@ -2164,8 +2209,8 @@ static void launch_fill_cols_rad(aln_ctx *ctx, int nsel, int L)
     const int thr = std::max(256, T), G = thr / T;
     const size_t sm = (size_t)G * RegFFT<NY, -1, RAD>::SMEM * sizeof(float2);   // k2_colspec's FF
     smem_attr(ctx->device, (const void *)k2_colspec<NY, RAD>, sm);
-    LAUNCH(ctx, "k2_colspec", (k2_colspec<NY, RAD>), dim3((L + 1 + G - 1) / G, nsel), thr, sm,
-           ctx->dpairs, ctx->tw, (const int *)ctx->dsel_cur);
+    LAUNCH_DEP(ctx, "k2_colspec", (k2_colspec<NY, RAD>), dim3((L + 1 + G - 1) / G, nsel), thr, sm,
+               ctx->dpairs, ctx->tw, (const int *)ctx->dsel_cur);
 }
 
 // the cache entry is computed with the radix of the column kernel that reads it
@@ -2197,8 +2242,8 @@ static void launch_corrcol_var(aln_ctx *ctx, int n, int L, int cached)
                       sizeof(float2);
     void (*kern)(PairDev *, const float2 *, int) = k2_corrcol<NY, VAR>;
     smem_attr(ctx->device, (const void *)kern, sm);
-    LAUNCH(ctx, "k2_corrcol", kern, dim3((L + 1 + G - 1) / G, n), thr, sm, ctx->dpairs, ctx->tw,
-           cached);
+    LAUNCH_DEP(ctx, "k2_corrcol", kern, dim3((L + 1 + G - 1) / G, n), thr, sm, ctx->dpairs, ctx->tw,
+               cached);
 }
 
 template <int NY>
@@ -2231,8 +2276,8 @@ static void launch_corrseg(aln_ctx *ctx, int n, int L)
         RegFFT<NS, -1, corrseg_radix<NS>()>::SMEM + (corrseg_regs<NS>() ? 0 : 2 * NS);
     const size_t sm = (size_t)G * per_team * sizeof(float2);
     smem_attr(ctx->device, (const void *)k2_corrseg<NS>, (size_t)GMAX * per_team * sizeof(float2));
-    LAUNCH(ctx, "k2_corrseg", k2_corrseg<NS>, dim3((L + 1 + G - 1) / G, n), G * T, sm,
-           ctx->dpairs, ctx->tw);
+    LAUNCH_DEP(ctx, "k2_corrseg", k2_corrseg<NS>, dim3((L + 1 + G - 1) / G, n), G * T, sm,
+               ctx->dpairs, ctx->tw);
 }
 
 template <int LL>
@@ -2242,8 +2287,8 @@ static void launch_lagrow2(aln_ctx *ctx, int n, int maxWy)
     constexpr int thr = lagrow_threads(T), G = thr / T;
     const size_t sm = (size_t)G * lag_pitch<LL>() * sizeof(float2);
     smem_attr(ctx->device, (const void *)k2_lagrow<LL>, sm);
-    LAUNCH(ctx, "k2_lagrow", k2_lagrow<LL>, dim3((maxWy + G - 1) / G, n), thr, sm,
-           ctx->dpairs, ctx->tw);
+    LAUNCH_DEP(ctx, "k2_lagrow", k2_lagrow<LL>, dim3((maxWy + G - 1) / G, n), thr, sm,
+               ctx->dpairs, ctx->tw);
 }
 
 template <int LL>
@@ -2271,13 +2316,13 @@ static void launch_lagimg2(aln_ctx *ctx, int n, int maxWy, bool both, bool sonly
         const int per = (int)std::max(1LL, std::min(8LL, (long long)groups * n / full));
         const size_t sm = (size_t)G * lag_pitch<LL>() * 2 * sizeof(float2);
         smem_attr(ctx->device, (const void *)k2_lagss<LL>, sm);
-        LAUNCH(ctx, "k2_lagimg", k2_lagss<LL>, dim3((groups + per - 1) / per, n), thr, sm,
-               ctx->dpairs, ctx->tw);
+        LAUNCH_DEP(ctx, "k2_lagimg", k2_lagss<LL>, dim3((groups + per - 1) / per, n), thr, sm,
+                   ctx->dpairs, ctx->tw);
         return;
     }
     const size_t sm = (size_t)G * lag_pitch<LL>() * (both ? 2 : 1) * sizeof(float2);
     smem_attr(ctx->device, (const void *)k2_lagimg<LL>, sm);
-    LAUNCH(ctx, "k2_lagimg", k2_lagimg<LL>, dim3(groups, n), thr, sm, ctx->dpairs, ctx->tw);
+    LAUNCH_DEP(ctx, "k2_lagimg", k2_lagimg<LL>, dim3(groups, n), thr, sm, ctx->dpairs, ctx->tw);
 }
 
 #define ALN_CASES_L(X) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
@@ -2319,9 +2364,9 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "row length %d", L);
         }
         if (mode == JOB_IMAGES_R)
-            LAUNCH(ctx, "k2_lagscan", k2_imgscan,
-                   dim3((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n), 32 * LAGSCAN_ROWS, 0,
-                   ctx->dpairs);
+            LAUNCH_DEP(ctx, "k2_lagscan", k2_imgscan,
+                       dim3((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n), 32 * LAGSCAN_ROWS, 0,
+                       ctx->dpairs);
     } else if (mode == JOB_P2I) {
         switch (L) {
 #define X(v) case v: launch_lagp2i<v>(ctx, n, maxWy); break;
@@ -2485,27 +2530,27 @@ static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *>
                                    (size_t)pl->d.table_w * pl->d.table_h, cudaMemcpyHostToDevice,
                                    ctx->stream));
     if (sp.sw > 0)
-        LAUNCH(ctx, "k_transpose", k_transpose,
-               dim3(sp.t8 ? (sp.sw + 128 * TR_TILES - 1) / (128 * TR_TILES)
-                          : (sp.sw + 32 * TR_TILES - 1) / (32 * TR_TILES),
-                    (sp.sh + 31) / 32, 2 * n),
-               dim3(32, 8), 0, ctx->dpairs);
+        LAUNCH_DEP(ctx, "k_transpose", k_transpose,
+                   dim3(sp.t8 ? (sp.sw + 128 * TR_TILES - 1) / (128 * TR_TILES)
+                              : (sp.sw + 32 * TR_TILES - 1) / (32 * TR_TILES),
+                        (sp.sh + 31) / 32, 2 * n),
+                   dim3(32, 8), 0, ctx->dpairs);
     if (mode == JOB_P2I)
         return ALN_OK;
     if (sp.packed) {
         smem_attr(ctx->device, (const void *)k3_satp, satp_smem());
-        LAUNCH(ctx, "k3_sat", k3_satp, dim3((sp.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
-               satp_smem(), ctx->dpairs);
+        LAUNCH_DEP(ctx, "k3_sat", k3_satp, dim3((sp.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
+                   satp_smem(), ctx->dpairs);
     }
     if (sp.plain)
-        LAUNCH(ctx, "k3_sat", k3_sat, dim3((sp.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS), 0,
-               ctx->dpairs);
+        LAUNCH_DEP(ctx, "k3_sat", k3_sat, dim3((sp.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS), 0,
+                   ctx->dpairs);
     if (sonly)
-        LAUNCH(ctx, "k2_sat2w", k2_sat2w<true>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
-               ctx->dpairs);
+        LAUNCH_DEP(ctx, "k2_sat2w", k2_sat2w<true>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
+                   ctx->dpairs);
     else
-        LAUNCH(ctx, "k2_sat2w", k2_sat2w<false>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
-               ctx->dpairs);
+        LAUNCH_DEP(ctx, "k2_sat2w", k2_sat2w<false>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
+                   ctx->dpairs);
     return ALN_OK;
 }
 
@@ -2513,10 +2558,10 @@ static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *>
 static void launch_peaks(aln_ctx *ctx, const JobSpan &sp)
 {
     ctx->dpairs = ctx->dpairs_base + sp.off;
-    LAUNCH(ctx, "k2_lagscan", k2_lagscan,
-           dim3((sp.maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, sp.n), 32 * LAGSCAN_ROWS, 0,
-           ctx->dpairs);
-    LAUNCH(ctx, "k_final", k_final, sp.n, 256, 0, ctx->dpairs, ctx->dres_base + sp.off);
+    LAUNCH_DEP(ctx, "k2_lagscan", k2_lagscan,
+               dim3((sp.maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, sp.n), 32 * LAGSCAN_ROWS, 0,
+               ctx->dpairs);
+    LAUNCH_DEP(ctx, "k_final", k_final, sp.n, 256, 0, ctx->dpairs, ctx->dres_base + sp.off);
 }
 
 // The chunk's transforms, and the peaks of CorrImages and CorrPatchToImage.
@@ -2581,7 +2626,7 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
                ctx->dpairs);
         LAUNCH(ctx, "k_fpeak", k_fpeak, n, FPK_THREADS, 0, ctx->dpairs, ctx->dres);
     } else if (mode != JOB_PATCHES)
-        LAUNCH(ctx, "k_final_img", k_final_img, n, 256, 0, ctx->dpairs, ctx->dres);
+        LAUNCH_DEP(ctx, "k_final_img", k_final_img, n, 256, 0, ctx->dpairs, ctx->dres);
     CK(cudaGetLastError());
     return ALN_OK;
 }

@@ -426,6 +426,7 @@ __device__ __forceinline__ void sat_cols_packed(const PairDev &p, int i, unsigne
 // bytes of dynamic shared memory.
 __global__ void __launch_bounds__(32 * SAT_WARPS, 2) k3_satp(PairDev *pairs)
 {
+    grid_dep();
     extern __shared__ __align__(16) unsigned char satp_stage[];
     __shared__ unsigned long long shP[64 * SAT_WARPS];
     __shared__ int shN[64 * SAT_WARPS];
@@ -441,6 +442,7 @@ __global__ void __launch_bounds__(32 * SAT_WARPS, 2) k3_satp(PairDev *pairs)
 
 __global__ void k3_sat(PairDev *pairs)
 {
+    grid_dep();
     __shared__ long long shS[32 * SAT_WARPS], shQ[32 * SAT_WARPS];
     __shared__ int shN[32 * SAT_WARPS];
     const PairDev &p = pairs[blockIdx.y >> 1];
@@ -509,6 +511,7 @@ __device__ __forceinline__ void store_bits(char *p, int es, long long idx, unsig
 #define TR_WORDS (3 * 296 + 9 * 32)   // words of a turned uint8 tile
 __global__ void __launch_bounds__(256) k_transpose(PairDev *pairs)
 {
+    grid_dep();
     __shared__ __align__(16) unsigned long long tile[37][32];
     static_assert(sizeof tile >= 2 * TR_WORDS * 4 && sizeof tile >= 32 * 33 * 8, "tile buffers");
     PairDev &p = pairs[blockIdx.z >> 1];
@@ -786,6 +789,7 @@ __device__ __forceinline__ void sat2_row_counts(const PairDev &p, int i, int slo
 template <bool NONLY>
 __global__ void k2_sat2w(PairDev *pairs)
 {
+    grid_dep();
     PairDev &p = pairs[blockIdx.z];
     const int i = blockIdx.y;
     const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -822,6 +826,7 @@ template <int L>
 __global__ void __launch_bounds__(rowfft_threads(rowfft_T<L>()), rowfft_minb<L>())
 k2_rowfft(PairDev *pairs, const float2 *__restrict__ tw, int only_img, const int *sel)
 {
+    grid_dep();
     using F = RowFFT<L>;
     constexpr int V = F::V, T = F::T;
     constexpr int G = rowfft_threads(T) / T;
@@ -1011,6 +1016,7 @@ __global__ void __launch_bounds__(corrcol_threads<NY, VAR>(),
                                                                                  : (VAR >= 2 ? 3 : 2))
 k2_corrcol(PairDev *pairs, const float2 *__restrict__ tw, int use_cached_b)
 {
+    grid_dep();
     constexpr bool PLAIN = VAR == 1, SONLY = VAR >= 2, DIRECT = VAR == 3;
     using FF = RegFFT<NY, -1, corrcol_radix<NY, VAR>()>;
     using FI = RegFFT<NY, +1, corrcol_radix<NY, VAR>()>;
@@ -1179,6 +1185,7 @@ template <int NS>
 __global__ void __launch_bounds__(256, 2)
 k2_corrseg(PairDev *pairs, const float2 *__restrict__ tw)
 {
+    grid_dep();
     using FF = RegFFT<NS, -1, corrseg_radix<NS>()>;
     using FI = RegFFT<NS, +1, corrseg_radix<NS>()>;
     static_assert(FI::SMEM <= FF::SMEM, "the inverse runs in the forward transform's buffer");
@@ -1291,6 +1298,7 @@ template <int NY, int RAD>
 __global__ void __launch_bounds__(NY / RAD >= 256 ? NY / RAD : 256)
 k2_colspec(PairDev *pairs, const float2 *__restrict__ tw, const int *sel)
 {
+    grid_dep();
     using FF = RegFFT<NY, -1, RAD>;
     constexpr int R = FF::R, T = FF::T;
     extern __shared__ float2 smem[];
@@ -1375,6 +1383,7 @@ template <int L>
 __global__ void __launch_bounds__(lagrow_threads(FFTOf<L, +1>::T))
 k2_lagrow(PairDev *pairs, const float2 *__restrict__ tw)
 {
+    grid_dep();
     using F = FFTOf<L, +1>;   // RegFFT, or MixFFT for L = 3 * 2^k, 5 * 2^k
     static_assert(F::SMEM <= lag_pitch<L>(), "the exchange buffer fits the team's row region");
     constexpr int V = F::V, T = F::T;
@@ -1494,6 +1503,7 @@ __device__ __forceinline__ void scan_row_int(const PairDev &p, const LagRow &q, 
 // grid (ceil(max Wy / LAGSCAN_ROWS), npairs), block 32 * LAGSCAN_ROWS
 __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
 {
+    grid_dep();
     const PairDev &p = pairs[blockIdx.y];
     if (p.status != 0 || !(p.fin & 4))
         return;
@@ -1578,6 +1588,7 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
 template <int L>
 __global__ void __launch_bounds__(256, 2) k2_lagimg(PairDev *pairs, const float2 *__restrict__ tw)
 {
+    grid_dep();
     using F = RegFFT<L, +1>;
     static_assert(F::SMEM <= lag_pitch<L>(), "the exchange buffer fits the team's row region");
     constexpr int R = F::R, T = F::T;
@@ -1774,6 +1785,7 @@ __device__ __forceinline__ bool key_better(float a, int ka, float b, int kb)
 template <int L>
 __global__ void __launch_bounds__(256, 3) k2_lagss(PairDev *pairs, const float2 *__restrict__ tw)
 {
+    grid_dep();
     using F = RegFFT<L, +1>;
     static_assert(F::SMEM <= lag_pitch<L>(), "the exchange buffer fits the team's row region");
     constexpr int R = F::R, T = F::T, G = 256 / T, W = T < 32 ? T : 32;
@@ -2093,6 +2105,7 @@ __device__ __forceinline__ void scan_row_img(const PairDev &p, const LagRow &q, 
 
 __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_imgscan(PairDev *pairs)
 {
+    grid_dep();
     const PairDev &p = pairs[blockIdx.y];
     if (p.status != 0)
         return;
@@ -2204,6 +2217,7 @@ __device__ void img_result(PairDev &p, int rx, int ry, double ss, double ss2, co
 // with the sample sd over the whole S image (:3285-3289).
 __global__ void k_final_img(PairDev *pairs, ResultDev *res)
 {
+    grid_dep();
     __shared__ double red_r[32], red_s[32], red_s2[32];
     __shared__ long long red_k[32];
     PairDev &p = pairs[blockIdx.x];

@@ -164,3 +164,17 @@ def test_transposed_solve(ctx, w, h, col):
     g, t = ctx.corr_patches_batch([wide, tall])
     assert (g["r"], g["dx"], g["dy"], g["peak_x"], g["peak_y"]) == \
         (t["r"], t["dy"], t["dx"], t["peak_y"], t["peak_x"])
+
+
+@pytest.mark.parametrize("dtype", ["u8", "u16"])
+@pytest.mark.parametrize("w,h", [(90, 300), (300, 90)])
+def test_overlapped_launches(ctx, w, h, dtype):
+    """Alone, a pair's kernels are launched ahead of the end of the one before
+    them; a batch's grids of many waves wait.  The same numbers bit for bit."""
+    rng = np.random.default_rng(w)
+    dt = np.uint8 if dtype == "u8" else np.uint16
+    kinds = [dict(zip("ab", (_view(t.astype(dt), 0, w) for t in _pair(rng, w, h))), radius=20)
+             for _ in range(8)]
+    alone = [ctx.corr_patches_batch([k])[0] for k in kinds]
+    batch = ctx.corr_patches_batch([kinds[i % 8] for i in range(1600)])
+    assert batch == [alone[i % 8] for i in range(1600)]
