@@ -2035,16 +2035,40 @@ __device__ __forceinline__ float r_bound(float n, float cs, const float4 &A, con
     return fmaxf(num, 0.0f) * (rsqrtf(lo1) * rsqrtf(lo2)) * (1.0f + 1.0e-6f) + 1.0e-6f;
 }
 
+// The same bound for integer pixels, whose box sums are exact.  FP32 rounds n cs
+// and a b, and where an overlap lies far from the image's mean they cancel:
+// 100 grey levels off with a deviation of 0.5, the rounded R is 2e-3 off and
+// more.  So their magnitudes enter, as in r_bound.  FP64 itself rounds n Q and
+// S^2: e64 n^2 is more than that, e64 being 2^-51 times the largest pixel value
+// squared.  (n Q - S^2 of 16-bit pixels may pass 2^64; what is left of it then is
+// less, and bounds R too.)  Infinite where the flat-overlap guard may hold.
+__device__ __forceinline__ float r_bound_int(int n, float cs, const longlong2 &A,
+                                             const longlong2 &B, int m1, int m2, float e64)
+{
+    typedef unsigned long long u64;
+    const float EPS = 4.8e-7f;   // a few FP32 roundings of a term
+    const float f1 = u64_to_float((u64)n * (u64)A.y - (u64)A.x * (u64)A.x);
+    const float f2 = u64_to_float((u64)n * (u64)B.y - (u64)B.x * (u64)B.x);
+    const float fn = __int2float_rn(n), nc = fn * cs;
+    const float ab = i64_to_float(A.x - (long long)n * m1) * i64_to_float(B.x - (long long)n * m2);
+    if (!(f1 * f2 > fn * fn * 1.001e-9f))
+        return __int_as_float(0x7f800000);
+    const float i1 = rsqrtf(f1), i2 = rsqrtf(f2);
+    const float num = fmaxf(nc - ab, 0.0f) + EPS * (fabsf(nc) + fabsf(ab));
+    return num * (i1 * i2) * (1.0f + 1.0e-6f) + fn * fn * e64 * (i1 * i1 + i2 * i2) + 1.0e-6f;
+}
+
 // CorrImagesR's scan of the lag image k2_lagrow wrote: one warp per lag row.
 // R itself is FP64 (RCalc::CalcR, clamped to (-1, 1)), and this GPU computes
 // FP64 two lanes per clock and SM: with R, its box sums, conversions and
 // comparisons in FP64 at every lag the scan took 1063 of 1543 us for 24 pairs
 // of 300 x 421.  So each lag's R is first bounded from above without FP64 --
-// integer images by r_int, others from FP32 copies of their tables -- and the
-// FP64 R, the counts and the exact comparison are made where the bound reaches
-// the best R that any row of the job has found so far (p.reach; what is skipped
-// lies below that one, so the result does not depend on the rows' order): 234
-// us.  grid (ceil(max Wy / LAGSCAN_ROWS), njobs), block 32 * LAGSCAN_ROWS.
+// integer images from their exact sums, others from FP32 copies of the tables
+// -- and the FP64 R, the counts and the exact comparison are made where the
+// bound reaches the best R that any row of the job has found so far (p.reach;
+// what is skipped lies below that one, so the result does not depend on the
+// rows' order): 234 us.  grid (ceil(max Wy / LAGSCAN_ROWS), njobs), block
+// 32 * LAGSCAN_ROWS.
 template <bool INT>
 __device__ __forceinline__ void scan_row_img(const PairDev &p, const LagRow &q, int j, int lo,
                                              int hi, bool check, int *job_reach, double &br,
@@ -2060,6 +2084,7 @@ __device__ __forceinline__ void scan_row_img(const PairDev &p, const LagRow &q, 
     const int key0 = iy * p.wR + p.cx;   // key of lag x: key0 + x
     const float mu1 = (float)p.mu[0], mu2 = (float)p.mu[1];
     const int m1 = INT ? (int)p.mu[0] : 0, m2 = INT ? (int)p.mu[1] : 0;
+    const float e64 = p.dt[0] == ALN_U8 && p.dt[1] == ALN_U8 ? 2.9e-11f : 1.91e-6f;
     float reach = from_ord_float(*(volatile int *)job_reach);   // R below it cannot win
 #pragma unroll 2
     for (int x0 = lo; x0 <= hi; x0 += 32) {
@@ -2071,10 +2096,7 @@ __device__ __forceinline__ void scan_row_img(const PairDev &p, const LagRow &q, 
         if (INT) {
             const longlong2 A = row_box_i(p, q, 0, n, L2 - x, R2 - x);
             const longlong2 B = row_box_i(p, q, 1, n, L2, R2);
-            top = r_int(n, c * invf, A.x, A.y, B.x, B.y, m1, m2);
-            // r_int's FP32 rounding, its flat-overlap guard near the FP64 one, and
-            // R = 0 where the FP64 r falls outside (-1, 1)
-            top = top == 0.0f ? __int_as_float(0x7f800000) : fmaxf(top, 0.0f) + 1.0e-4f;
+            top = r_bound_int(n, c * invf, A, B, m1, m2, e64);
         } else {
             top = r_bound((float)n, c * invf,
                           row_box_f(p.satf[0], q.oT[0], q.oB[0], L2 - x, R2 - x),
@@ -2119,8 +2141,7 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_imgscan(PairDev *pairs)
     legal_span(p, q, y + p.cy, lo, hi);
     double br = -1.0e30;
     int bk = 0x7fffffff;
-    // (r_int's integers hold for every overlap of an 8-bit row, of a 16-bit one
-    // below 2^20 pixels; the rest bound nothing and take the FP64 R at each lag)
+    // (16-bit rows of 2^20 pixels and more take the FP64 R at each lag)
     if (!p.satf[0] && r_int_ok(p, (long long)min(q.w1, q.w2) * q.olh)) {
         scan_row_img<true>(p, q, j, lo, hi, check, &pairs[blockIdx.y].reach, br, bk);
     } else if (p.satf[0]) {

@@ -151,6 +151,40 @@ def test_corr_images_r_bound(ctx, orc, data, rule):
     check(g, o, 1, (data, rule))
 
 
+@pytest.mark.parametrize("kinds", ["u8 u8", "u16 u16", "u8 u16"])
+@pytest.mark.parametrize("away,sd", [(60, 0.4), (100, 0.5), (120, 0.8)])
+def test_corr_images_r_flat_overlaps(ctx, kinds, away, sd):
+    """Integer images whose searched overlaps are nearly flat and far from the
+    image's mean, where FP32 gives R to 1e-3 only: the scan's peak is the largest
+    of the values that the same call gives lag by lag (a box rule that one lag of
+    the oval meets; the correlation is the same numbers), alone and in a batch."""
+    import alignment_projects_gb300 as aln
+    rng = np.random.default_rng(away)
+    h, w, rx, ry = 48, 1024, 128, 10
+    cx = w // 2 + rx   # lags that overlap a's dark left half with b's dark right half
+    lags = [(x, y) for y in range(-ry, ry + 1) for x in range(cx - rx, cx + rx + 1)
+            if (x - cx) ** 2 + (rx / ry) ** 2 * y * y <= rx * rx]
+    for _ in range(3):
+        job = {}
+        for name, dt, dark in zip("ab", kinds.split(), (0, w // 2)):
+            scale = 16 if dt == "u16" else 1
+            v = np.full((h, w), 128.0 + away)
+            v[:, dark:dark + w // 2] -= 2 * away
+            v = np.rint((v + sd * rng.standard_normal((h, w))) * scale)
+            job[name] = _view(np.clip(v, 0, 255 * scale)
+                              .astype(np.uint8 if dt == "u8" else np.uint16), 0, w)
+        job.update(kind=aln.CORR_R, ox=cx, oy=0, rx=rx, ry=ry,
+                   legal=aln.legal(aln.RGN_MIN, 8, 8, 0))
+        each = ctx.corr_images_batch([
+            dict(job, ox=x, oy=y, rx=1, ry=1,
+                 legal=aln.legal(aln.RGN_EXACT, w - x, h - abs(y), 0)) for x, y in lags])
+        assert all(e["status"] == aln.ALN_OK and (e["peak_x"], e["peak_y"]) == q
+                   for e, q in zip(each, lags))
+        best = max(range(len(lags)), key=lambda k: each[k]["r"])
+        for g in ctx.corr_images_batch([job]) + ctx.corr_images_batch([job] * 40):
+            assert (g["r"], (g["peak_x"], g["peak_y"])) == (each[best]["r"], lags[best])
+
+
 @pytest.mark.parametrize("w,h", [(33, 5), (127, 31), (128, 32), (129, 33), (131, 64), (512, 30),
                                  (513, 97), (640, 36), (1030, 203)])
 @pytest.mark.parametrize("col", [0, 1, 2])
