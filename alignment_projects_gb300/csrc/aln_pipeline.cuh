@@ -1514,9 +1514,14 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
     const int y = p.ylo + j, ox = p.ox;
     const long long dy = y - p.oy, in = p.rsqr - dy * dy;   // disc: dx^2 <= in
     // the row's span of the disc, a little wide; the lag's own test is exact
-    // (an FP64 square root per row cost more than the test)
-    const int xr = in < 0 ? -1 : (int)sqrtf(__uint2float_rn((unsigned)min(in, 1ll << 30))) + 2;
-    const int xa = max(p.xlo, ox - xr), xb = xr < 0 ? xa - 1 : min(p.xhi, ox + xr);
+    // (an FP64 square root per row cost more than the test).  From 2^15 px on,
+    // where FP32 is a pixel off and the centre may be far, the whole row
+    int xa = p.xlo, xb = in < 0 ? xa - 1 : p.xhi;
+    if (in >= 0 && in < 1ll << 30) {
+        const int xr = (int)sqrtf(__int2float_rn((int)in)) + 2;
+        xa = max(xa, ox - xr);
+        xb = min(xb, ox + xr);
+    }
     const LagRow q = lag_row(p, y);
     const int key0 = (y < 0 ? y + Ny : y) * Nx;   // storage indices are < 2^26
     const int nmax = min(q.w1, q.w2) * q.olh;     // largest overlap of the row
@@ -1731,7 +1736,12 @@ __global__ void __launch_bounds__(256, 2) k2_lagimg(PairDev *pairs, const float2
 // The lags x of image row iy (lag row y) whose overlap's box and oval are
 // legal, as one interval (empty: lo > hi): the box width is min(w1, w2, x + w1,
 // w2 - x), so widths >= omin are an interval of x, and so is a row of the
-// oval.  Valid when the row has no upper width limit and no table.
+// oval.  Exact when span_exact.
+#define OVAL_SPAN 46340   // squares up to here are ints, as oval_ok's
+__device__ __forceinline__ bool span_exact(const PairDev &p, const LagRow &q)
+{
+    return !q.tbl && q.omax == 0x7fffffff && !(p.oval_on && p.orx > OVAL_SPAN);
+}
 __device__ __forceinline__ void legal_span(const PairDev &p, const LagRow &q, int iy, int &lo,
                                            int &hi)
 {
@@ -1743,7 +1753,7 @@ __device__ __forceinline__ void legal_span(const PairDev &p, const LagRow &q, in
     }
     lo = max(lo, q.omin - q.w1);
     hi = min(hi, q.w2 - q.omin);
-    if (!p.oval_on)
+    if (!p.oval_on || p.orx > OVAL_SPAN)
         return;
     if (iy < p.ocy - p.ory || iy > p.ocy + p.ory) {
         hi = lo - 1;
@@ -1751,7 +1761,7 @@ __device__ __forceinline__ void legal_span(const PairDev &p, const LagRow &q, in
     }
     const int y = iy - p.ocy;
     const double base = p.oasq * y * y;   // oval_ok's terms
-    const int dmax = min(p.orx, 40000);   // (d * d is an int; lags are below 8192)
+    const int dmax = p.orx;
     auto in = [&](int d) { return d <= dmax && !((double)(d * d) + base > p.orx2); };
     int d = min(dmax, (int)sqrtf(fmaxf((float)(p.orx2 - base), 0.f)));
     while (d >= 0 && !in(d))
@@ -1862,7 +1872,7 @@ __global__ void __launch_bounds__(256, 3) k2_lagss(PairDev *pairs, const float2 
         bool slow = false;
         if (live) {
             q = lag_row(p, y);
-            slow = q.tbl || q.omax != 0x7fffffff;
+            slow = !span_exact(p, q);
             if (!slow)
                 legal_span(p, q, iy, xl, xr);
             float fs = 0.f, fe = 0.f, fq = 0.f, fqe = 0.f;
@@ -2136,7 +2146,7 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_imgscan(PairDev *pairs)
         return;
     const int y = p.ylo + j;
     const LagRow q = lag_row(p, y);
-    const bool check = q.tbl || q.omax != 0x7fffffff;
+    const bool check = !span_exact(p, q);
     int lo, hi;
     legal_span(p, q, y + p.cy, lo, hi);
     double br = -1.0e30;

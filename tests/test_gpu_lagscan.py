@@ -185,6 +185,30 @@ def test_corr_images_r_flat_overlaps(ctx, kinds, away, sd):
             assert (g["r"], (g["peak_x"], g["peak_y"])) == (each[best]["r"], lags[best])
 
 
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+def test_far_disc_centre(ctx, orc, dtype):
+    """A disc around a point 40000 px off whose edge crosses the lags: the
+    oracle's peak, for CorrPatches' circle and CorrImages' oval."""
+    import oracle as O
+    from test_gpu_corr import assert_parity
+    from test_gpu_images import aln_legal, check
+    rng = np.random.default_rng(8)
+    a, b = _pair(rng, 60, 70)
+    b[::5, ::3] //= 2   # (equal images: R = 1, which CorrImages takes as 0)
+    a, b = a.astype(dtype), b.astype(dtype)
+    lg = O.legal(O.RGN_MIN, 20, 20, 0)
+    pa, pb = (O.image_to_points(t) for t in (a, b))
+    for ox, oy in ((43000, 0), (-43000, 0), (0, 43000), (5, -43000)):
+        rad = 43000 + 12
+        g = ctx.corr_patches_batch([dict(a=a, b=b, ox=ox, oy=oy, radius=rad,
+                                         legal=aln_legal(lg))])[0]
+        assert_parity(g, orc.corr_patches(*pa, *pb, ox, oy, rad, lg), f"disc {ox} {oy}")
+        for kind in (1, 2):
+            g = ctx.corr_images(kind, a, b, aln_legal(lg), 0.0, 0.75, ox, oy, rad, rad)
+            o = orc.corr_images(kind, *pa, *pb, lg, 0.0, 0.75, ox, oy, rad, rad)
+            check(g, o, kind, f"oval {kind} {ox} {oy}")
+
+
 @pytest.mark.parametrize("w,h", [(33, 5), (127, 31), (128, 32), (129, 33), (131, 64), (512, 30),
                                  (513, 97), (640, 36), (1030, 203)])
 @pytest.mark.parametrize("col", [0, 1, 2])
