@@ -1465,7 +1465,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_dec_sums(DecJob *jobs)
         }
         long long pos = c0;   // first addend not summed yet
         const long long end = min(nb, c0 + SUM_THREADS * SUM_K);
-        while (pos < end) {
+        while (pos < end && !isinf(x)) {   // (an infinite sum takes no more addends >= 0)
             long long X;
             int e;
             sum_split(x, X, e);

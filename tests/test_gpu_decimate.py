@@ -47,3 +47,21 @@ def test_sequential_sums_bitwise(ctx, orc, kind, h, w, lbin):
     ys, xs = np.nonzero(pres)
     assert np.array_equal(np.stack([xs, ys], 1), xy.astype(np.int64))
     assert np.array_equal(vals[ys, xs], v, equal_nan=True)   # bit for bit
+
+
+@pytest.mark.parametrize("value", [1e308, 1e154])   # the sum, the sum of squares overflows
+@pytest.mark.parametrize("at", [300, 4094, 4700])   # in a chunk, over its end, in the next one
+def test_sums_that_overflow(ctx, orc, value, at):
+    """A running sum that reaches infinity stays there, as one thread's would."""
+    h, w = 90, 101
+    img = np.random.default_rng(at).random(h * w) + 0.5
+    img[at:at + 4] = value
+    img[at + 700:at + 704] = value
+    img = img.reshape(h, w)
+    yy, xx = np.mgrid[0:h, 0:w]
+    pts = np.stack([xx.ravel(), yy.ravel()], 1).astype(np.float64)
+    with np.errstate(all="ignore"):
+        _, v = orc.decimate_normalize(pts, img.ravel(), w, h, 1)
+    vals, pres, _ = ctx.decimate([img], 1)[0]
+    assert pres.all()
+    assert np.array_equal(vals.ravel(), v, equal_nan=True)
