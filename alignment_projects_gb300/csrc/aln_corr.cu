@@ -1685,10 +1685,12 @@ static bool spec_room(aln_ctx *ctx, size_t bytes)
 }
 
 // A device buffer for a new cache entry of `bytes`, evicting entries not used
-// by the current chunk (least recently used first) while the cache is at its
+// by the current span (least recently used first) while the cache is at its
 // cap or the device is short of free memory.  Buffers are reused on the
 // context's stream, so a kernel still reading an evicted entry finishes
-// before the buffer is filled again.  Returns NULL when nothing fits.
+// before the buffer is filled again.  The current span's entries stay: its
+// kernels are launched after all of its chunks are prepared, too late for
+// cudaFree to wait for them.  Returns NULL when nothing fits.
 static float2 *spec_alloc(aln_ctx *ctx, size_t bytes)
 {
     auto f = ctx->spec_free.find(bytes);
@@ -1706,7 +1708,7 @@ static float2 *spec_alloc(aln_ctx *ctx, size_t bytes)
             continue;
         }
         if (ctx->spec_lru.empty() || ctx->spec_lru.begin()->first >= ctx->spec_tick)
-            return nullptr;   // every entry is in use by the current chunk
+            return nullptr;   // every entry is in use by the current span
         auto lru = ctx->spec.find(ctx->spec_lru.begin()->second);
         float2 *b = lru->second.X2;
         const size_t lb = lru->second.bytes;
@@ -2438,7 +2440,6 @@ static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, 
     cl.fill_maxh = 1;
     char *work = work_base;
     const bool reg_path = register_path(cl.Nx, cl.Ny);
-    ++ctx->spec_tick;
     for (int k = 0; k < n; ++k) {
         PairPlan &pl = *chunk[k];
         work += carve(pl, work, *pl.src);
@@ -3030,6 +3031,7 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
             js.off = off;
             char *work = ctx->ws + nstage * max_stage;
             std::vector<std::vector<PairPlan *> *> chunks;
+            ++ctx->spec_tick;   // the span's cache entries stay until it is launched
             for (auto &chunk : span) {
                 ChunkLaunch cl;
                 work += prep_chunk(ctx, chunk, off, work, ctx->htab + off, fills, cl);

@@ -188,7 +188,8 @@ int aln_ctx_set_split_grids(aln_ctx *ctx, int on);
  * it off and releases it; SIZE_MAX: bounded by free device memory alone).
  * The cache also never grows into the last (workspace limit + 2 GiB) of
  * free device memory.  Least recently used entries are evicted first
- * (entries the running chunk reads are kept). */
+ * (entries that the jobs being launched together read are kept; a job that
+ * finds no room goes uncached). */
 int aln_ctx_set_spectrum_cache(aln_ctx *ctx, size_t bytes);
 
 /* CorrPatches column segmenting for this context: 0 = the cost model

@@ -493,6 +493,43 @@ def test_spectrum_cache_same_numbers(ctx):
     assert c2["spec_fills"] == 2 and c2["spec_hits"] == 12
 
 
+def test_spectrum_cache_small_cap_mixed_grids(ctx):
+    """Keyed jobs on several grids whose spectra do not fit the cache together:
+    nothing that the batch itself reads is evicted (its grids are launched
+    together), and the results are the uncached ones, call after call."""
+    import alignment_projects_gb300 as aln
+    rng = np.random.default_rng(11)
+    pairs = []
+    for k, n in enumerate([40, 90, 200, 300, 40, 200, 90, 300]):
+        b = rng.integers(0, 256, (n, n)).astype(np.uint8)
+        a = np.roll(b, (2, -1), (0, 1))
+        pairs.append(dict(a=a, b=b, radius=12, b_key=1000 + k,
+                          legal=aln.legal(aln.RGN_MIN, 16, 16, 0)))
+    ctx.set_segmenting(-1)
+    ctx.set_spectrum_cache(0)
+    plain = ctx.corr_patches_batch(pairs)
+    ctx.set_spectrum_cache(1 << 30)
+    keyless = [dict(p, b_key=0) for p in pairs]
+    assert ctx.corr_patches_batch(keyless) == ctx.corr_patches_batch(pairs) == plain
+    cap = ctx.counters()["spec_bytes"] // 2
+    try:
+        for order in (1, -1, 1):
+            ctx.set_spectrum_cache(0)
+            ctx.set_spectrum_cache(cap)
+            ctx.profile_reset()
+            assert ctx.corr_patches_batch(pairs[::order])[::order] == plain
+            c = ctx.counters()
+            assert c["spec_fills"] >= 2 and c["spec_evictions"] == 0
+            assert c["spec_bytes"] <= cap
+            # a later call evicts what an earlier one left
+            assert ctx.corr_patches_batch(pairs[3:4] + pairs[7:]) == plain[3:4] + plain[7:]
+            assert ctx.corr_patches_batch(pairs) == plain
+            assert ctx.counters()["spec_evictions"] > 0
+    finally:
+        ctx.set_segmenting(0)
+        ctx.set_spectrum_cache(8 << 30)
+
+
 def test_spectrum_cache_images_and_off(ctx):
     """CorrImages jobs with a keyed b, and the cache switched off and on."""
     import alignment_projects_gb300 as aln
