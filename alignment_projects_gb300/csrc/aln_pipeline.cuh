@@ -683,7 +683,7 @@ __device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, 
         for (int k = 0; k < K; ++k) {
             s[k] = q[k] = 0;
             if (c + k < w) {
-                const typename SP::type a = r[c + k], b = __ldg(o + c + k);
+                const typename SP::type a = r[c + k], b = o[c + k];
                 s[k] = a.x + b.x;
                 q[k] = a.y + b.y;
             }
@@ -727,7 +727,7 @@ __device__ __forceinline__ void sat2_row_packed(const PairDev &p, int i, int slo
             const int c = c0 + 64 * k + 2 * lane;
             e[k] = make_ulonglong2(0, 0);
             if (c < sp) {
-                const ulonglong2 a = r[c >> 1], b = __ldg(o + (c >> 1));
+                const ulonglong2 a = r[c >> 1], b = o[c >> 1];
                 e[k].x = a.x + b.x;
                 e[k].y = c + 1 < w ? a.y + b.y : 0;
             }
@@ -1473,7 +1473,7 @@ __device__ __forceinline__ void scan_row_int(const PairDev &p, const LagRow &q, 
         const int x = min(x0 + lane, xb);
         const int L2 = max(0, x), R2 = max(min(q.w2 - 1, x + q.w1 - 1), L2);
         const int olw = R2 - L2 + 1, n = olw * q.olh;
-        const float cs = __ldg(row + x) * invf;
+        const float cs = row[x] * invf;
         float r;
         if (KIND == 0) {
             const u64 a = row_box_p((const u64 *)t1, q.oT[0], q.oB[0], L2 - x, R2 - x);
@@ -1566,7 +1566,7 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
     for (int x = xa + lane; x <= xb; x += 32) {
         const long long dx = x - ox;
         double rv;
-        if (dx * dx <= in && lag_row_r(p, q, x, __ldg(row + x) * invf, rv))
+        if (dx * dx <= in && lag_row_r(p, q, x, row[x] * invf, rv))
             best_merge(br, bk, rv, key0 + (x < 0 ? x + Nx : x));
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -2101,7 +2101,7 @@ __device__ __forceinline__ void scan_row_img(const PairDev &p, const LagRow &q, 
         const int x = min(x0 + lane, hi);
         const int L2 = max(0, x), R2 = max(min(q.w2 - 1, x + q.w1 - 1), L2);
         const int n = (R2 - L2 + 1) * q.olh;
-        const float c = __ldg(row + x);
+        const float c = row[x];
         float top;
         if (INT) {
             const longlong2 A = row_box_i(p, q, 0, n, L2 - x, R2 - x);

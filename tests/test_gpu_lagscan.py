@@ -236,3 +236,23 @@ def test_overlapped_launches(ctx, w, h, dtype):
     alone = [ctx.corr_patches_batch([k])[0] for k in kinds]
     batch = ctx.corr_patches_batch([kinds[i % 8] for i in range(1600)])
     assert batch == [alone[i % 8] for i in range(1600)]
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32, np.float64])
+@pytest.mark.parametrize("kind", [1, 2])   # CORR_R, CORR_S
+def test_overlapped_image_launches(ctx, dtype, kind):
+    """The same for CorrImages' kernels, with and without a count rule and a
+    mincor."""
+    import alignment_projects_gb300 as aln
+    rng = np.random.default_rng(kind)
+    jobs = []
+    for k in range(8):
+        a, b = _pair(rng, 70, 60, zeros=0.2)
+        b[::4, ::3] //= 2
+        jobs.append(dict(kind=kind, a=_view(a.astype(dtype), 0, 70), b=_view(b.astype(dtype), 0, 70),
+                         mincor=0.05 * (k // 4),
+                         legal=aln.legal(aln.RGN_MIN, 20, 20, 0, aln.CNT_GT if k % 2 else 0, 300)))
+    alone = [ctx.corr_images_batch([j])[0] for j in jobs]
+    assert all(g["status"] == aln.ALN_OK for g in alone)
+    batch = ctx.corr_images_batch([jobs[i % 8] for i in range(1600)])
+    assert batch == [alone[i % 8] for i in range(1600)]
