@@ -2398,6 +2398,35 @@ struct JobSpan {
     int sw = 0, sh = 0;                // largest caller-frame image of transposed jobs
     int t8 = 1;                        // every transposed job is uint8 (128-byte tiles)
     int packed = 0, plain = 0;         // jobs with packed / other summed-area tables
+    void add(const PairDev &d)
+    {
+        ++n;
+        for (int i = 0; i < 2; ++i) {
+            maxw = std::max(maxw, d.w[i]);
+            maxh = std::max(maxh, d.h[i]);
+            int ns = 0;
+            for (int q = 0; q < 2; ++q)
+                if (d.need_hi[i][q] >= d.need_lo[i][q])
+                    ns += d.need_hi[i][q] - d.need_lo[i][q] + 1;
+            maxslots = std::max(maxslots, ns);
+            if (d.transposed) {
+                sw = std::max(sw, d.h[i]);
+                sh = std::max(sh, d.w[i]);
+                t8 &= d.dt[i] == ALN_U8;
+            }
+        }
+        maxWy = std::max(maxWy, d.yhi - d.ylo + 1);
+        ++(d.sat_packed ? packed : plain);
+    }
+    // blocks of the launches that cover the whole span (launch_tables,
+    // launch_peaks), each sized for the largest job; one of the column walk's,
+    // with 512 threads and their shared memory, takes as long as four to pass
+    long long blocks() const
+    {
+        const long long walk = (packed ? (maxw + 63) / 64 : 0) + (plain ? (maxw + 31) / 32 : 0);
+        const long long turn = (long long)((sw + 127) / 128) * ((sh + 31) / 32);
+        return n * (2 * (turn + 4 * walk + (maxslots + 7) / 8) + (maxWy + 7) / 8);
+    }
     void add(const JobSpan &o)
     {
         n += o.n;
@@ -2427,16 +2456,13 @@ static bool register_path(int Nx, int Ny)
     return Nx / 2 >= 8 && Nx / 2 <= 4096 && Ny >= 8 && Ny <= 8192;
 }
 
-// Host side of a chunk: carve each job's workspace (the chunk's work buffer
-// is reused by every chunk, in stream order), resolve spectrum-cache keys,
-// write the job table entries hd[0..n).
-static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, char *work_base,
+// Host side of a chunk of the sizes cl.s: carve each job's workspace (the
+// chunk's work buffer is reused by every span, in stream order), resolve
+// spectrum-cache keys, write the job table entries hd[0..n).
+static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, char *work_base,
                          PairDev *hd, std::vector<int> &fills, ChunkLaunch &cl)
 {
     const int n = (int)chunk.size();
-    JobSpan &sp = cl.s;
-    sp.off = off;
-    sp.n = n;
     cl.Nx = chunk[0]->d.Nx;
     cl.Ny = chunk[0]->d.Ny;
     cl.fill_off = (int)fills.size();
@@ -2470,21 +2496,6 @@ static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, 
                 }
             }
         }
-        for (int i = 0; i < 2; ++i) {
-            sp.maxw = std::max(sp.maxw, pl.d.w[i]);
-            sp.maxh = std::max(sp.maxh, pl.d.h[i]);
-            int ns = 0;
-            for (int q = 0; q < 2; ++q)
-                if (pl.d.need_hi[i][q] >= pl.d.need_lo[i][q])
-                    ns += pl.d.need_hi[i][q] - pl.d.need_lo[i][q] + 1;
-            sp.maxslots = std::max(sp.maxslots, ns);
-            if (pl.d.transposed) {
-                sp.sw = std::max(sp.sw, pl.d.h[i]);
-                sp.sh = std::max(sp.sh, pl.d.w[i]);
-                sp.t8 &= pl.d.dt[i] == ALN_U8;
-            }
-        }
-        sp.maxWy = std::max(sp.maxWy, pl.d.yhi - pl.d.ylo + 1);
         pl.d.sat_int = (pl.d.dt[0] == ALN_U8 || pl.d.dt[0] == ALN_U16 ? 1 : 0) |
                        (pl.d.dt[1] == ALN_U8 || pl.d.dt[1] == ALN_U16 ? 2 : 0);
         // a sweep correlates one thumbnail b at many angles, one job after the
@@ -2504,7 +2515,6 @@ static size_t prep_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, int off, 
         if ((pl.d.mode == JOB_PATCHES || pl.d.mode == JOB_IMAGES_R) && reg_path)
             pl.d.fin |= 4;
         pl.d.reach = ord_float(pl.d.mincor > 0.0 ? (float)pl.d.mincor - 1.0e-4f : -2.0f);
-        ++(pl.d.sat_packed ? sp.packed : sp.plain);
         hd[k] = pl.d;
     }
     cl.nfill = (int)fills.size() - cl.fill_off;
@@ -2932,8 +2942,16 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
     // has a chunk per grid, and each of its small launches filled the chip for a
     // part of its time only (3000 uneven pairs: 74 chunks in 9 spans, 629 -> 323
     // launches, 18.4 -> 16.0 ms).
-    // A quarter, so that the host prepares the next span while this one runs.
+    // A quarter, and a chunk's 4096 jobs, so that the host prepares the next span
+    // while this one runs (16000 pairs of 16^2 on one grid: 4.2 ms in spans of a
+    // chunk, 5.2 in one).  Its launches are sized for the largest job, and a
+    // block that finds nothing to do costs 1-2 ns, a chunk's own launches about
+    // 20 us: a chunk joins where it adds at most SPAN_PAD such blocks (those 16000
+    // pairs and one of 2000^2: 13.2 ms without this rule, 4.0 apart; 200 pairs of
+    // 100 x 90 and a strip of 235 x 2048: 205 us in one span, 223 apart).
+    constexpr long long SPAN_PAD = 16384;
     std::vector<std::vector<std::vector<std::vector<PairPlan *>>>> wspans(windows.size());
+    std::vector<JobSpan> sizes;   // of all chunks in launch order
     const size_t span_cap = ctx->ws_budget / 4;
     size_t max_stage = 0, max_work = 0;
     for (size_t w = 0; w < windows.size(); ++w) {
@@ -2949,36 +2967,45 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
             sb += pl->in_bytes[0] + pl->in_bytes[1] + 16;
         }
         max_stage = std::max(max_stage, sb);
-        size_t span_bytes = 0, span_jobs = 0;
-        auto put = [&](std::vector<PairPlan *> &chunk, size_t wb) {
+        size_t span_bytes = 0;
+        JobSpan span;   // sizes of the last one
+        auto put = [&](std::vector<PairPlan *> &chunk, size_t wb, JobSpan &cs) {
             auto &spans = wspans[w];
+            JobSpan both = span;
+            both.add(cs);
             const bool more = !spans.empty() && chunk[0]->d.mode == JOB_PATCHES &&
                               spans.back()[0][0]->d.mode == JOB_PATCHES &&
-                              span_bytes + wb <= span_cap && span_jobs + chunk.size() <= 16384;
+                              span_bytes + wb <= span_cap && both.n <= 4096 &&
+                              both.blocks() <= span.blocks() + cs.blocks() + SPAN_PAD;
             if (!more) {
                 spans.emplace_back();
-                span_bytes = span_jobs = 0;
+                span_bytes = 0;
+                both = cs;
             }
+            span = both;
+            sizes.push_back(cs);
             spans.back().push_back(std::move(chunk));
             span_bytes += wb;
-            span_jobs += spans.back().back().size();
             max_work = std::max(max_work, span_bytes);
             chunk.clear();
+            cs = JobSpan();
         };
         for (auto &g : groups) {
             std::vector<PairPlan *> chunk;
             size_t wb = 0;
+            JobSpan cs;
             for (PairPlan *pl : g.second) {
                 const size_t wk = pl->ws_bytes - pl->in_bytes[0] - pl->in_bytes[1];
                 if (!chunk.empty() && (wb + wk > ctx->ws_budget || chunk.size() >= 4096)) {
-                    put(chunk, wb);
+                    put(chunk, wb, cs);
                     wb = 0;
                 }
                 chunk.push_back(pl);
+                cs.add(pl->d);
                 wb += wk;
             }
             if (!chunk.empty())
-                put(chunk, wb);
+                put(chunk, wb, cs);
         }
     }
     max_stage = al256(max_stage);
@@ -3041,7 +3068,9 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
             ++ctx->spec_tick;   // the span's cache entries stay until it is launched
             for (auto &chunk : span) {
                 ChunkLaunch cl;
-                work += prep_chunk(ctx, chunk, off, work, ctx->htab + off, fills, cl);
+                cl.s = sizes[cls.size()];
+                cl.s.off = off;
+                work += prep_chunk(ctx, chunk, work, ctx->htab + off, fills, cl);
                 off += cl.s.n;
                 js.add(cl.s);
                 cls.push_back(cl);

@@ -493,6 +493,27 @@ def test_spectrum_cache_same_numbers(ctx):
     assert c2["spec_fills"] == 2 and c2["spec_hits"] == 12
 
 
+@pytest.mark.parametrize("small,large,together", [(600, 1, False), (12, 3, True)])
+def test_shared_launches(ctx, small, large, together):
+    """The launches that do not depend on the transform lengths are shared by
+    grids while that pays: not where hundreds of small jobs would each get the
+    blocks of a large one.  The same numbers either way."""
+    rng = np.random.default_rng(small)
+    groups = []
+    for n, side in ((small, 16), (large, 700)):
+        b = rng.integers(0, 256, (side, side)).astype(np.uint8)
+        a = np.roll(b, (1, 2), (0, 1))
+        groups.append([dict(a=a, b=b, radius=8)] * n)
+
+    def run(pairs):
+        ctx.corr_patches_batch(pairs)   # (plans its classes)
+        ctx.profile_reset()
+        return ctx.corr_patches_batch(pairs), ctx.counters()["launches"]
+    (got0, n0), (got1, n1), (got, n) = run(groups[0]), run(groups[1]), run(groups[1] + groups[0])
+    assert got == got1 + got0
+    assert n < n0 + n1 if together else n == n0 + n1
+
+
 def test_spectrum_cache_small_cap_mixed_grids(ctx):
     """Keyed jobs on several grids whose spectra do not fit the cache together:
     nothing that the batch itself reads is evicted (its grids are launched
