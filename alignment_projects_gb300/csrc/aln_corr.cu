@@ -1312,6 +1312,23 @@ static void launch_dep(aln_ctx *c, void (*kern)(P...), dim3 grid, dim3 block, si
     cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// Whether a lag scan of so many blocks, each eight rows of `lags` lags, is
+// launched ahead.  Not with long rows on about one block per multiprocessor: the
+// blocks would gather on the multiprocessors that are free first, and the scan
+// takes as long as the fullest of them.  Launched ahead and not, all lags: one
+// FP32 pair of 600 x 500 (125 blocks) 277-347 and 200 us, six of 300^2 (450) 331
+// and 285, one of uint16 600^2 152 and 137, of uint8 800^2 144 and 131,
+// CorrImagesR of one uint8 pair 600^2 165 and 143, of three 141 and 129; but of
+// seven (560 blocks) 225 and 235, of one of 300 x 421 (80) 101 and 112, eight
+// strips of 129 lags 105.5 and 107.3, two uint8 600^2 within 200 px 88 and 92.
+// (An FP64 lag takes about as long as five FP32 ones: FP32 1000 x 100 153 and
+// 140.)
+static bool scan_ahead(aln_ctx *ctx, long long blocks, int lags, bool fp64)
+{
+    const int sms = sm_count(ctx);
+    return lags * (fp64 ? 5 : 1) <= 512 || 5 * blocks < 3 * sms || blocks > 3 * sms;
+}
+
 #define LAUNCH_DEP(c, name, kern, grid, block, smem, ...)                            \
     do {                                                                             \
         prof_begin(c, name);                                                         \
@@ -2335,8 +2352,8 @@ static void launch_lagimg2(aln_ctx *ctx, int n, int maxWy, bool both, bool sonly
 
 // register-FFT pipeline for one chunk: rows (both images), fused columns,
 // lag rows.  L = Nx/2 in [16, 4096], Ny in [16, 8192].
-static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int maxWy,
-                               int mode = JOB_PATCHES, bool both = false, bool sonly = false,
+static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int maxWx,
+                               int maxWy, int mode = JOB_PATCHES, bool both = false, bool sonly = false,
                                bool seg = false, bool cached = false)
 {
     switch (L) {
@@ -2368,10 +2385,11 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
 #undef X
         default: return set_err(ctx, ALN_ERR_UNSUPPORTED, "row length %d", L);
         }
-        if (mode == JOB_IMAGES_R)
-            LAUNCH_DEP(ctx, "k2_lagscan", k2_imgscan,
-                       dim3((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n), 32 * LAGSCAN_ROWS, 0,
-                       ctx->dpairs);
+        const dim3 grid((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n);
+        if (mode == JOB_IMAGES_R && scan_ahead(ctx, (long long)grid.x * n, maxWx, false))
+            LAUNCH_DEP(ctx, "k2_lagscan", k2_imgscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
+        else if (mode == JOB_IMAGES_R)
+            LAUNCH(ctx, "k2_lagscan", k2_imgscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
     } else if (mode == JOB_P2I) {
         switch (L) {
 #define X(v) case v: launch_lagp2i<v>(ctx, n, maxWy); break;
@@ -2394,10 +2412,11 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
 // in the batch's job table.
 struct JobSpan {
     int off = 0, n = 0;                // jobs [off, off + n) of the batch table
-    int maxw = 1, maxh = 1, maxslots = 1, maxWy = 1;
+    int maxw = 1, maxh = 1, maxslots = 1, maxWx = 1, maxWy = 1;
     int sw = 0, sh = 0;                // largest caller-frame image of transposed jobs
     int t8 = 1;                        // every transposed job is uint8 (128-byte tiles)
     int packed = 0, plain = 0;         // jobs with packed / other summed-area tables
+    int fp64 = 0;                      // jobs with FP64 ones
     void add(const PairDev &d)
     {
         ++n;
@@ -2415,8 +2434,10 @@ struct JobSpan {
                 t8 &= d.dt[i] == ALN_U8;
             }
         }
+        maxWx = std::max(maxWx, d.xhi - d.xlo + 1);
         maxWy = std::max(maxWy, d.yhi - d.ylo + 1);
         ++(d.sat_packed ? packed : plain);
+        fp64 += d.dt[0] > ALN_U16 || d.dt[1] > ALN_U16;
     }
     // blocks of the launches that cover the whole span (launch_tables,
     // launch_peaks), each sized for the largest job; one of the column walk's,
@@ -2433,12 +2454,14 @@ struct JobSpan {
         maxw = std::max(maxw, o.maxw);
         maxh = std::max(maxh, o.maxh);
         maxslots = std::max(maxslots, o.maxslots);
+        maxWx = std::max(maxWx, o.maxWx);
         maxWy = std::max(maxWy, o.maxWy);
         sw = std::max(sw, o.sw);
         sh = std::max(sh, o.sh);
         t8 &= o.t8;
         packed += o.packed;
         plain += o.plain;
+        fp64 += o.fp64;
     }
 };
 
@@ -2576,9 +2599,11 @@ static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *>
 static void launch_peaks(aln_ctx *ctx, const JobSpan &sp)
 {
     ctx->dpairs = ctx->dpairs_base + sp.off;
-    LAUNCH_DEP(ctx, "k2_lagscan", k2_lagscan,
-               dim3((sp.maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, sp.n), 32 * LAGSCAN_ROWS, 0,
-               ctx->dpairs);
+    const dim3 grid((sp.maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, sp.n);
+    if (scan_ahead(ctx, (long long)grid.x * sp.n, sp.maxWx, sp.fp64 != 0))
+        LAUNCH_DEP(ctx, "k2_lagscan", k2_lagscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
+    else
+        LAUNCH(ctx, "k2_lagscan", k2_lagscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
     LAUNCH_DEP(ctx, "k_final", k_final, sp.n, 256, 0, ctx->dpairs, ctx->dres_base + sp.off);
 }
 
@@ -2606,8 +2631,9 @@ static int launch_chunk(aln_ctx *ctx, std::vector<PairPlan *> &chunk, const Chun
         }
     }
     if (register_path(Nx, Ny)) {
-        if (int rc = launch_fft_pipeline(ctx, L, Ny, n, cl.s.maxh, cl.s.maxWy, mode, cl.both != 0,
-                                         cl.sonly != 0, cl.seg != 0, cl.cached != 0))
+        if (int rc = launch_fft_pipeline(ctx, L, Ny, n, cl.s.maxh, cl.s.maxWx, cl.s.maxWy, mode,
+                                         cl.both != 0, cl.sonly != 0, cl.seg != 0,
+                                         cl.cached != 0))
             return rc;
     } else if (mode != JOB_PATCHES) {
         return set_err(ctx, ALN_ERR_UNSUPPORTED, "CorrImages FFT size %d x %d", Nx, Ny);

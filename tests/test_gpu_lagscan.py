@@ -256,3 +256,18 @@ def test_overlapped_image_launches(ctx, dtype, kind):
     assert all(g["status"] == aln.ALN_OK for g in alone)
     batch = ctx.corr_images_batch([jobs[i % 8] for i in range(1600)])
     assert batch == [alone[i % 8] for i in range(1600)]
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+@pytest.mark.parametrize("images", [False, True])
+def test_long_scans_alone_and_batched(ctx, dtype, images):
+    """A pair over all lags, whose scan waits for its lag image or is launched
+    ahead by how many blocks there are: the same numbers alone and in a batch."""
+    import alignment_projects_gb300 as aln
+    rng = np.random.default_rng(7)
+    job = dict(zip("ab", (_view(t.astype(dtype), 0, 400) for t in _pair(rng, 400, 430))),
+               legal=aln.legal(aln.RGN_MIN, 40, 40, 0), **(dict(kind=1) if images else {}))
+    call = ctx.corr_images_batch if images else ctx.corr_patches_batch
+    alone = call([job])
+    for n in (3, 9):
+        assert call([job] * n) == alone * n
