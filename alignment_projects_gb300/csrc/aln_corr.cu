@@ -446,8 +446,8 @@ __device__ __forceinline__ int isqrt_ll(long long v)
 // waits before it does anything, so a kernel's end means that all kernels
 // before it have ended too -- and a kernel's first block starts after all of
 // them but the one just before it.  What that one writes is read with plain
-// loads: __ldg is for data that stays as it is while the kernel runs (twiddles,
-// callers' images, and what older kernels of the chain wrote).
+// loads or ld_chain: __ldg is for data that stays as it is while the kernel runs
+// (twiddles, callers' images, and what older kernels of the chain wrote).
 __device__ __forceinline__ void grid_dep()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -2579,13 +2579,9 @@ static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *>
         LAUNCH_DEP(ctx, "k3_sat", k3_satp, dim3((sp.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
                    satp_smem(), ctx->dpairs);
     }
-    // k3_sat reads its images by __ldg (plain loads would wait for the stores of
-    // the rows before: 2 % of a 16-bit batch), so it starts after a transpose's end
-    const dim3 sat_grid((sp.maxw + 31) / 32, 2 * n), sat_block(32, SAT_WARPS);
-    if (sp.plain && sp.sw > 0)
-        LAUNCH(ctx, "k3_sat", k3_sat, sat_grid, sat_block, 0, ctx->dpairs);
-    else if (sp.plain)
-        LAUNCH_DEP(ctx, "k3_sat", k3_sat, sat_grid, sat_block, 0, ctx->dpairs);
+    if (sp.plain)
+        LAUNCH_DEP(ctx, "k3_sat", k3_sat, dim3((sp.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS), 0,
+                   ctx->dpairs);
     if (sonly)
         LAUNCH_DEP(ctx, "k2_sat2w", k2_sat2w<true>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
                    ctx->dpairs);

@@ -38,6 +38,54 @@ __device__ __forceinline__ void fresh(const float2 *__restrict__ &tw)
     asm volatile("" : "+l"(tw));
 }
 
+// Loads of what an earlier kernel of the chain wrote (grid_dep) and this one
+// only reads: coherent, which __ldg is not, but as free to move -- a plain load
+// waits for the stores before it (k3_sat's images by plain loads: 3000 uneven
+// pairs 15.68 -> 15.98 ms).  Their addresses come out of the job's descriptor,
+// which is read after the wait.
+__device__ __forceinline__ unsigned ld_chain(const uint8_t *a)
+{
+    unsigned v;
+    asm("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ unsigned ld_chain(const uint16_t *a)
+{
+    unsigned short v;
+    asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ float ld_chain(const float *a)
+{
+    float v;
+    asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ double ld_chain(const double *a)
+{
+    double v;
+    asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ double2 ld_chain(const double2 *a)
+{
+    double2 v;
+    asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ longlong2 ld_chain(const longlong2 *a)
+{
+    longlong2 v;
+    asm("ld.global.v2.s64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(a));
+    return v;
+}
+__device__ __forceinline__ ulonglong2 ld_chain(const ulonglong2 *a)
+{
+    ulonglong2 v;
+    asm("ld.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(a));
+    return v;
+}
+
 // asynchronous copies, global -> shared without registers
 __device__ __forceinline__ void cp_async8(void *dst_shared, const void *src_global)
 {
@@ -203,7 +251,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
                 stop = min(stop, max(lo1, y));
 #pragma unroll 8
             for (; y < stop; ++y) {
-                const AC v = (AC)__ldg(&col[y * st]);
+                const AC v = (AC)ld_chain(&col[y * st]);
                 if (SQ) {
                     s += v;
                     q += v * v;
@@ -218,7 +266,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
             const int rend = min(y1 - 1, first ? hi0 : hi1);
             const long long base = first ? (long long)(y - lo0) : (long long)(len0 + y - lo1);
             for (long long o = base * p.sp[i] + c; y <= rend; ++y, o += p.sp[i]) {
-                const AC v = (AC)__ldg(&col[y * st]);
+                const AC v = (AC)ld_chain(&col[y * st]);
                 if (SQ) {
                     s += v;
                     q += v * v;
@@ -683,7 +731,7 @@ __device__ __forceinline__ void sat2_row_any(const PairDev &p, int i, int slot, 
         for (int k = 0; k < K; ++k) {
             s[k] = q[k] = 0;
             if (c + k < w) {
-                const typename SP::type a = r[c + k], b = o[c + k];
+                const typename SP::type a = r[c + k], b = ld_chain(o + c + k);
                 s[k] = a.x + b.x;
                 q[k] = a.y + b.y;
             }
@@ -727,7 +775,7 @@ __device__ __forceinline__ void sat2_row_packed(const PairDev &p, int i, int slo
             const int c = c0 + 64 * k + 2 * lane;
             e[k] = make_ulonglong2(0, 0);
             if (c < sp) {
-                const ulonglong2 a = r[c >> 1], b = o[c >> 1];
+                const ulonglong2 a = r[c >> 1], b = ld_chain(o + (c >> 1));
                 e[k].x = a.x + b.x;
                 e[k].y = c + 1 < w ? a.y + b.y : 0;
             }
@@ -1473,7 +1521,7 @@ __device__ __forceinline__ void scan_row_int(const PairDev &p, const LagRow &q, 
         const int x = min(x0 + lane, xb);
         const int L2 = max(0, x), R2 = max(min(q.w2 - 1, x + q.w1 - 1), L2);
         const int olw = R2 - L2 + 1, n = olw * q.olh;
-        const float cs = row[x] * invf;
+        const float cs = ld_chain(row + x) * invf;
         float r;
         if (KIND == 0) {
             const u64 a = row_box_p((const u64 *)t1, q.oT[0], q.oB[0], L2 - x, R2 - x);
@@ -1566,7 +1614,7 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
     for (int x = xa + lane; x <= xb; x += 32) {
         const long long dx = x - ox;
         double rv;
-        if (dx * dx <= in && lag_row_r(p, q, x, row[x] * invf, rv))
+        if (dx * dx <= in && lag_row_r(p, q, x, ld_chain(row + x) * invf, rv))
             best_merge(br, bk, rv, key0 + (x < 0 ? x + Nx : x));
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -2101,7 +2149,7 @@ __device__ __forceinline__ void scan_row_img(const PairDev &p, const LagRow &q, 
         const int x = min(x0 + lane, hi);
         const int L2 = max(0, x), R2 = max(min(q.w2 - 1, x + q.w1 - 1), L2);
         const int n = (R2 - L2 + 1) * q.olh;
-        const float c = row[x];
+        const float c = ld_chain(row + x);
         float top;
         if (INT) {
             const longlong2 A = row_box_i(p, q, 0, n, L2 - x, R2 - x);
