@@ -1345,6 +1345,19 @@ __device__ __forceinline__ double sum_join(long long X, int e)
                                                       (X & ((1ll << 52) - 1)));
 }
 
+// The first n of V, or their squares, added one after another (an absent bin
+// holds +0.0, which leaves any sum as it is).
+__device__ __forceinline__ double sum_in_order(const double *__restrict__ V, int n, bool sq)
+{
+    double x = 0.0;
+#pragma unroll 16
+    for (int k = 0; k < n; ++k) {
+        const double v = __ldg(V + k);
+        x = __dadd_rn(x, sq ? __dmul_rn(v, v) : v);
+    }
+    return x;
+}
+
 // grid (n, 2), block SUM_THREADS: chain 0 sums the present bins' values,
 // chain 1 their squares.
 __global__ void __launch_bounds__(SUM_THREADS) k_dec_sums(DecJob *jobs)
@@ -1360,19 +1373,12 @@ __global__ void __launch_bounds__(SUM_THREADS) k_dec_sums(DecJob *jobs)
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const double *__restrict__ V = J.vals;
     const unsigned char *__restrict__ P = J.pres;
-    // (an absent bin holds +0.0, which leaves any sum as it is)
     double x = 0.0;
     int np = 0;
     // the first bins, where every other one doubles the sum, by one thread
     const int first = (int)min(nb, (long long)SUM_FIRST);
-    if (tid == 0) {
-#pragma unroll 16
-        for (int k = 0; k < first; ++k) {
-            const double v = __ldg(V + k);
-            x = __dadd_rn(x, sq ? __dmul_rn(v, v) : v);
-        }
-        sh_x = x;
-    }
+    if (tid == 0)
+        sh_x = sum_in_order(V, first, sq);
     // this thread's addends of the chunk from k on (V is 16-byte aligned)
     auto fetch = [&](long long k, double *v) {
         if (k + SUM_K <= nb) {
@@ -1549,11 +1555,25 @@ __global__ void __launch_bounds__(SUM_THREADS) k_dec_sums(DecJob *jobs)
 // the reference's operation order (no contraction), then (v - avg) / sd for
 // every present bin.  Across the chip: the FP64 divisions of a
 // full-resolution crop would keep one SM busy for milliseconds.
-__global__ void k_normalize(DecJob *jobs)
+// small: no image has more than SUM_FIRST bins, and each one's block makes the
+// sums itself (8^2 thumbnails 65 -> 59 us, 16^2 86 -> 83: k_dec_sums is a launch
+// that adds them one after another too).
+__global__ void __launch_bounds__(256) k_normalize(DecJob *jobs, bool small)
 {
-    __shared__ double sh_avg, sh_sd;
+    __shared__ double sh_avg, sh_sd, sh_sum[2];
     DecJob &J = jobs[blockIdx.y];
     const long long nb = (long long)J.ow * J.oh;
+    if (small) {
+        static_assert(SUM_FIRST <= 256, "a thread per bin");
+        if (threadIdx.x == 0 || threadIdx.x == 32)
+            sh_sum[threadIdx.x >> 5] = sum_in_order(J.vals, (int)nb, threadIdx.x != 0);
+        const int np = __syncthreads_count(threadIdx.x < nb && J.pres[threadIdx.x]);
+        if (threadIdx.x == 0) {
+            J.sums[0] = sh_sum[0];
+            J.sums[1] = sh_sum[1];
+            J.np = np;
+        }
+    }
     if (threadIdx.x == 0) {
         double avg = J.sums[0], sd = 0.0;
         const int n = J.np;
@@ -1657,9 +1677,12 @@ static int decimate_device(aln_ctx *ctx, int n, const aln_image *in,
                0, dj, lbin);
         if (normalize) {
             const long long mb = (long long)mw * mh;
-            LAUNCH(ctx, "k_dec_sums", k_dec_sums, dim3(n, 2), SUM_THREADS, 0, dj);
+            const bool small = mb <= SUM_FIRST;
+            if (!small)
+                LAUNCH(ctx, "k_dec_sums", k_dec_sums, dim3(n, 2), SUM_THREADS, 0, dj);
             LAUNCH(ctx, "k_normalize", k_normalize,
-                   dim3((unsigned)std::min<long long>((mb + 1023) / 1024, 256), n), 256, 0, dj);
+                   dim3((unsigned)std::min<long long>((mb + 1023) / 1024, 256), n), 256, 0, dj,
+                   small);
         }
         if (rows) {
             LAUNCH(ctx, "k_dec_rows", k_dec_rows, dim3((mh + 7) / 8, n), 256, 0, dj);

@@ -65,3 +65,25 @@ def test_sums_that_overflow(ctx, orc, value, at):
     vals, pres, _ = ctx.decimate([img], 1)[0]
     assert pres.all()
     assert np.array_equal(vals.ravel(), v, equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [1, 16])
+@pytest.mark.parametrize("kind", ["u8", "f64+", "f32-", "late"])
+@pytest.mark.parametrize("h,w,lbin", [(2, 1, 1), (8, 8, 1), (16, 16, 1), (16, 17, 1), (32, 32, 16),
+                                      (40, 36, 3)])
+def test_small_thumbnails(ctx, orc, kind, h, w, lbin, n):
+    """Up to 256 bins the sums are made where the bins are normalised: bit for
+    bit, alone and beside a larger image, whose sums have a kernel of their own."""
+    rng = np.random.default_rng(h * w)
+    imgs = [_image(kind, h, w, rng) for _ in range(n)] + [_image(kind, 40, 50, rng)]
+    yy, xx = np.mgrid[0:h, 0:w]
+    pts = np.stack([xx.ravel(), yy.ravel()], 1).astype(np.float64)
+    alone, beside = ctx.decimate(imgs[:n], lbin), ctx.decimate(imgs, lbin)
+    for img, (vals, pres, sd), (vals2, pres2, sd2) in zip(imgs, alone, beside):
+        with np.errstate(all="ignore"):
+            xy, v = orc.decimate_normalize(pts, img.ravel().astype(np.float64), w, h, lbin)
+        ys, xs = np.nonzero(pres)
+        assert np.array_equal(np.stack([xs, ys], 1), xy.astype(np.int64))
+        assert np.array_equal(vals[ys, xs], v, equal_nan=True)
+        assert np.array_equal(vals, vals2, equal_nan=True) and np.array_equal(pres, pres2)
+        assert sd == sd2
