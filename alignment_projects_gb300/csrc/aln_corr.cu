@@ -2579,9 +2579,14 @@ static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *>
         LAUNCH_DEP(ctx, "k3_sat", k3_satp, dim3((sp.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
                    satp_smem(), ctx->dpairs);
     }
-    if (sp.plain)
-        LAUNCH_DEP(ctx, "k3_sat", k3_sat, dim3((sp.maxw + 31) / 32, 2 * n), dim3(32, SAT_WARPS), 0,
-                   ctx->dpairs);
+    // k3_sat reads its images by __ldg, so it starts after a transpose's end
+    // (by plain loads 3000 uneven pairs took 15.98 ms, not 15.68; by ld_chain the
+    // walk of 205 rasters of 180^2 took 58 us, not 44)
+    const dim3 sat_grid((sp.maxw + 31) / 32, 2 * n), sat_block(32, SAT_WARPS);
+    if (sp.plain && sp.sw > 0)
+        LAUNCH(ctx, "k3_sat", k3_sat, sat_grid, sat_block, 0, ctx->dpairs);
+    else if (sp.plain)
+        LAUNCH_DEP(ctx, "k3_sat", k3_sat, sat_grid, sat_block, 0, ctx->dpairs);
     if (sonly)
         LAUNCH_DEP(ctx, "k2_sat2w", k2_sat2w<true>, dim3((sp.maxslots + 7) / 8, 2, n), 256, 0,
                    ctx->dpairs);

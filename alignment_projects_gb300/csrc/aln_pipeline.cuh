@@ -39,32 +39,13 @@ __device__ __forceinline__ void fresh(const float2 *__restrict__ &tw)
 }
 
 // Loads of what an earlier kernel of the chain wrote (grid_dep) and this one
-// only reads: coherent, which __ldg is not, but as free to move -- a plain load
-// waits for the stores before it (k3_sat's images by plain loads: 3000 uneven
-// pairs 15.68 -> 15.98 ms).  Their addresses come out of the job's descriptor,
-// which is read after the wait.
-__device__ __forceinline__ unsigned ld_chain(const uint8_t *a)
-{
-    unsigned v;
-    asm("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(a));
-    return v;
-}
-__device__ __forceinline__ unsigned ld_chain(const uint16_t *a)
-{
-    unsigned short v;
-    asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(a));
-    return v;
-}
+// only reads: coherent, which __ldg is not, but free to move, where a plain load
+// waits for the stores before it.  Their addresses come out of the job's
+// descriptor, which is read after the wait.
 __device__ __forceinline__ float ld_chain(const float *a)
 {
     float v;
     asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(a));
-    return v;
-}
-__device__ __forceinline__ double ld_chain(const double *a)
-{
-    double v;
-    asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(a));
     return v;
 }
 __device__ __forceinline__ double2 ld_chain(const double2 *a)
@@ -251,7 +232,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
                 stop = min(stop, max(lo1, y));
 #pragma unroll 8
             for (; y < stop; ++y) {
-                const AC v = (AC)ld_chain(&col[y * st]);
+                const AC v = (AC)__ldg(&col[y * st]);
                 if (SQ) {
                     s += v;
                     q += v * v;
@@ -266,7 +247,7 @@ __device__ __forceinline__ void sat_cols(const PairDev &p, int i, TA *shS, TA *s
             const int rend = min(y1 - 1, first ? hi0 : hi1);
             const long long base = first ? (long long)(y - lo0) : (long long)(len0 + y - lo1);
             for (long long o = base * p.sp[i] + c; y <= rend; ++y, o += p.sp[i]) {
-                const AC v = (AC)ld_chain(&col[y * st]);
+                const AC v = (AC)__ldg(&col[y * st]);
                 if (SQ) {
                     s += v;
                     q += v * v;
