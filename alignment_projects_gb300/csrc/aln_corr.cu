@@ -130,10 +130,10 @@ __device__ __forceinline__ double div_sqrt2(double num, double d1, double d2)
 }
 
 // CLinCorr::GetCorr's terms for integer pixels (0_GEN/Correlation.cpp:
-// 705-757).  The normalisation terms n*Q - S^2 >= 0 are exact in unsigned
-// 64-bit arithmetic (valid while n*Q < 2^64: always for 8-bit pixels, for
-// 16-bit ones while n < 2^20), and the shifted sums S - n mu are exact
-// integers; the rest is FP32 -- the cross sum cs comes from the FP32 FFT, so
+// 705-757).  The normalisation terms n*Q - S^2 = n^2 var are exact integers, in
+// unsigned 64-bit arithmetic while below 2^64 (8-bit pixels: n < 2^25; 16-bit
+// ones, var < 2^30: n <= 2^17) and in 128-bit from there on (int_spread), and
+// so are the shifted sums S - n mu; the rest is FP32 -- the cross sum cs comes from the FP32 FFT, so
 // FP32 here adds an error of the same order (~1e-7 in r), and this GPU's
 // FP64 pipe is narrow (FP64 arithmetic bounded the lag kernel).  The
 // flat-overlap guard d1 d2 < n^2 1e-9 is evaluated in FP32 too.
@@ -158,15 +158,32 @@ __device__ __forceinline__ float i64_to_float(long long v)
     return v < 0 ? -f : f;
 }
 
+// n q - s^2 >= 0 (s, q >= 0); wide: it may pass 2^64
+__device__ __forceinline__ float int_spread(unsigned long long n, unsigned long long s,
+                                            unsigned long long q, bool wide)
+{
+    const unsigned long long a = n * q, b = s * s;
+    const float f = u64_to_float(a - b);
+    if (!wide)
+        return f;
+    const unsigned hi = (unsigned)(__umul64hi(n, q) - __umul64hi(s, s)) - (a < b);
+    return fmaf(__uint2float_rn(hi), 18446744073709551616.0f, f);   // (hi = 0: f)
+}
+
+// overlaps from which n q - s^2 may pass 2^64
+__device__ __forceinline__ bool int_wide(const PairDev &p, long long n)
+{
+    return n > (p.dt[0] == ALN_U8 && p.dt[1] == ALN_U8 ? 1ll << 25 : 1ll << 17);
+}
+
 // n: the overlap's pixels (a box of an FFT raster: < 2^26); m1, m2: the
 // integer mean shifts.  (The 32-bit form of the sums is r_int32.)
 __device__ __forceinline__ float r_int(int n, float cs, long long s1, long long q1, long long s2,
-                                       long long q2, int m1, int m2)
+                                       long long q2, int m1, int m2, bool wide)
 {
     typedef unsigned long long u64;
-    const u64 un = (u64)n;
-    const u64 d1 = un * (u64)q1 - (u64)s1 * (u64)s1, d2 = un * (u64)q2 - (u64)s2 * (u64)s2;
-    const float f1 = u64_to_float(d1), f2 = u64_to_float(d2), fn = __int2float_rn(n);
+    const float f1 = int_spread((u64)n, (u64)s1, (u64)q1, wide);
+    const float f2 = int_spread((u64)n, (u64)s2, (u64)q2, wide), fn = __int2float_rn(n);
     const float num = fmaf(fn, cs,
                            -(i64_to_float(s1 - (long long)n * m1) *
                              i64_to_float(s2 - (long long)n * m2)));
@@ -188,7 +205,7 @@ __device__ __forceinline__ float r_int32(int n, float cs, int s1, unsigned long 
     return f1 * f2 < fn * fn * 1.0e-9f ? 0.0f : num * (rsqrtf(f1) * rsqrtf(f2));
 }
 
-// the overlap sizes for which r_int is exact on this pair's pixel types
+// the overlap sizes for which this pair takes r_int
 __device__ __forceinline__ bool r_int_ok(const PairDev &p, long long n)
 {
     if ((p.sat_int & 3) != 3)
@@ -378,7 +395,8 @@ __device__ __forceinline__ bool lag_row_r(const PairDev &p, const LagRow &q, int
     if (r_int_ok(p, (long long)olw * olh)) {
         const longlong2 a = row_box_i(p, q, 0, olw * olh, L1, R1);
         const longlong2 b = row_box_i(p, q, 1, olw * olh, L2, R2);
-        r = (double)r_int(olw * olh, cs, a.x, a.y, b.x, b.y, (int)p.mu[0], (int)p.mu[1]);
+        r = (double)r_int(olw * olh, cs, a.x, a.y, b.x, b.y, (int)p.mu[0], (int)p.mu[1],
+                          int_wide(p, olw * olh));
         return true;
     }
     const double n = (double)(olw * olh);

@@ -1480,7 +1480,9 @@ k2_lagrow(PairDev *pairs, const float2 *__restrict__ tw)
 
 // The lags xa + lane, xa + lane + 32, ... <= xb of one row of an integer pair:
 // the best FP32 r and its storage index.  KIND: 0 packed tables, 1 int64
-// pairs with sums below 2^31, 2 int64 pairs; CHECK: a legality table or a
+// pairs with sums below 2^31, 2 int64 pairs, 3 those whose overlaps may be
+// int_wide (uint16 600^2 over all lags: 137 us as KIND 2, 138 as 3); CHECK: a
+// legality table or a
 // count rule is looked up too.  The body has no branch and reads past the
 // row's end at xb again, so that the unrolled loop's loads are in flight
 // together: with a branch per lag the scan waited for them one lag at a time.
@@ -1513,7 +1515,7 @@ __device__ __forceinline__ void scan_row_int(const PairDev &p, const LagRow &q, 
             const longlong2 a = row_box2((const longlong2 *)t1, q.oT[0], q.oB[0], L2 - x, R2 - x);
             const longlong2 b = row_box2((const longlong2 *)t2, q.oT[1], q.oB[1], L2, R2);
             r = KIND == 1 ? r_int32(n, cs, (int)a.x, a.y, (int)b.x, b.y, m1, m2)
-                          : r_int(n, cs, a.x, a.y, b.x, b.y, m1, m2);
+                          : r_int(n, cs, a.x, a.y, b.x, b.y, m1, m2, KIND == 3);
         }
         const int dx = x - ox;
         bool ok = olw >= q.omin && olw <= q.omax && (long long)dx * dx <= in;
@@ -1567,9 +1569,11 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
             else
                 scan_row_int<0, false>(p, q, xa, xb, y, in, key0, br, bk);
         } else if (check) {
-            scan_row_int<2, true>(p, q, xa, xb, y, in, key0, br, bk);
+            scan_row_int<3, true>(p, q, xa, xb, y, in, key0, br, bk);
         } else if (narrow) {
             scan_row_int<1, false>(p, q, xa, xb, y, in, key0, br, bk);
+        } else if (int_wide(p, nmax)) {
+            scan_row_int<3, false>(p, q, xa, xb, y, in, key0, br, bk);
         } else {
             scan_row_int<2, false>(p, q, xa, xb, y, in, key0, br, bk);
         }

@@ -590,3 +590,25 @@ def test_tiny_integer_patches(ctx, orc, dt, w, h):
         B, VB = oracle.image_to_points(p["b"])
         o = orc.corr_patches(A, VA, B, VB, 0, 0, 4096, oracle.legal(oracle.RGN_MIN, m, m, 0))
         assert_parity(g, o, f"{dt.__name__} {w}x{h}")
+
+
+@pytest.mark.parametrize("w,h,radius", [(300, 300, 4096), (700, 650, 24), (600, 420, 4096)])
+def test_full_range_16_bit(ctx, orc, w, h, radius):
+    """16-bit pixels over their whole range: n sum v^2 - (sum v)^2 of a large
+    overlap passes 2^64."""
+    import oracle
+    import alignment_projects_gb300 as aln
+    rng = np.random.default_rng(w)
+    big = np.where(rng.random((h + 8, w + 8)) < 0.5, 0, 65535) - 0.2 * rng.integers(
+        0, 65536, (h + 8, w + 8))
+    a, b = (np.clip(t, 0, 65535).astype(np.uint16) for t in (big[3:3 + h, 3:3 + w],
+                                                             big[1:1 + h, 4:4 + w]))
+    m = min(w, h) // 3
+    g = ctx.corr_patches_batch([dict(a=a, b=b, radius=radius,
+                                     legal=aln.legal(aln.RGN_MIN, m, m, 0))])[0]
+    A, VA = oracle.image_to_points(a)
+    B, VB = oracle.image_to_points(b)
+    o = orc.corr_patches(A, VA, B, VB, 0, 0, radius, oracle.legal(oracle.RGN_MIN, m, m, 0))
+    assert_parity(g, o, f"{w}x{h}")
+    i = ctx.corr_images(1, a, b, aln.legal(aln.RGN_MIN, m, m, 0))
+    assert abs(i["r"] - g["r"]) < 1e-5 and (i["peak_x"], i["peak_y"]) == (g["peak_x"], g["peak_y"])
