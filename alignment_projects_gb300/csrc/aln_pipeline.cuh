@@ -1,6 +1,6 @@
 // aln_pipeline.cuh -- the batched CorrPatches kernels built on the
 // register-resident FFT (aln_fft_reg.cuh).  Included by aln_corr.cu, after
-// the device helpers (load_px, sat slots, lag_r, best_merge).
+// the device helpers (load_px, sat slots, lag rows, r_int, best_merge).
 //
 //   k3_sat    per 32-column band: warp-local column prefix sums of v, v^2,
 //             (v != 0) at the needed rows, per-warp offsets, column totals

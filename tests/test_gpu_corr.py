@@ -612,3 +612,43 @@ def test_full_range_16_bit(ctx, orc, w, h, radius):
     assert_parity(g, o, f"{w}x{h}")
     i = ctx.corr_images(1, a, b, aln.legal(aln.RGN_MIN, m, m, 0))
     assert abs(i["r"] - g["r"]) < 1e-5 and (i["peak_x"], i["peak_y"]) == (g["peak_x"], g["peak_y"])
+
+
+def test_staging_windows(ctx):
+    """Host batches from 128 MB are copied window by window while the one before
+    computes: page-locked and pageable, 8 and 16 bits, tall, wide and small
+    images of their own in submission order mixed -- the numbers of the same
+    pairs on the device."""
+    import torch
+    rng = np.random.default_rng(21)
+    noise = {np.uint8: rng.integers(0, 256, (2300, 1400)).astype(np.uint8),
+             np.uint16: rng.integers(0, 4096, (2300, 1400)).astype(np.uint16)}
+    host, dev = [], []
+    for k in range(210):
+        dt = np.uint16 if k % 7 == 3 else np.uint8
+        w, h = (235, 2048) if k % 5 else (301, 260)
+        y, x = (int(v) for v in rng.integers(8, 150, 2))
+        ty, tx = (int(v) for v in rng.integers(-6, 7, 2))
+        src = noise[dt]
+        a, b = src[y:y + h, x:x + w], src[y + ty:y + ty + h, x + tx:x + tx + w]
+        if k % 11 == 4:
+            a, b = a.T, b.T
+        a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
+        job = dict(radius=20)
+        dev.append(dict(job, a=_cuda(a), b=_cuda(b)))
+        if k % 3:   # page-locked, the others pageable
+            a, b = (torch.from_numpy(t.view(np.uint8)).pin_memory().numpy().view(dt)
+                    for t in (a, b))
+        host.append(dict(job, a=a, b=b))
+    assert sum(j["a"].nbytes + j["b"].nbytes for j in host) > 128 << 20
+    want = ctx.corr_patches_batch(dev)
+    assert all(g["status"] == 0 and g["r"] > 0.99 for g in want)
+    for _ in range(3):
+        assert ctx.corr_patches_batch(host) == want
+
+
+def _cuda(t):
+    import torch
+    if t.dtype == np.uint16:
+        return torch.from_numpy(t.view(np.int16)).cuda().view(torch.uint16)
+    return torch.from_numpy(t).cuda()
