@@ -2356,7 +2356,7 @@ static void launch_lagimg2(aln_ctx *ctx, int n, int maxWy, bool both, bool sonly
         const int per = (int)std::max(1LL, std::min(8LL, (long long)groups * n / full));
         const size_t sm = (size_t)G * lag_pitch<LL>() * 2 * sizeof(float2);
         smem_attr(ctx->device, (const void *)k2_lagss<LL>, sm);
-        LAUNCH_DEP(ctx, "k2_lagimg", k2_lagss<LL>, dim3((groups + per - 1) / per, n), thr, sm,
+        LAUNCH_DEP(ctx, "k2_lagss", k2_lagss<LL>, dim3((groups + per - 1) / per, n), thr, sm,
                    ctx->dpairs, ctx->tw);
         return;
     }
@@ -2405,9 +2405,9 @@ static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int
         }
         const dim3 grid((maxWy + LAGSCAN_ROWS - 1) / LAGSCAN_ROWS, n);
         if (mode == JOB_IMAGES_R && scan_ahead(ctx, (long long)grid.x * n, maxWx, false))
-            LAUNCH_DEP(ctx, "k2_lagscan", k2_imgscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
+            LAUNCH_DEP(ctx, "k2_imgscan", k2_imgscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
         else if (mode == JOB_IMAGES_R)
-            LAUNCH(ctx, "k2_lagscan", k2_imgscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
+            LAUNCH(ctx, "k2_imgscan", k2_imgscan, grid, 32 * LAGSCAN_ROWS, 0, ctx->dpairs);
     } else if (mode == JOB_P2I) {
         switch (L) {
 #define X(v) case v: launch_lagp2i<v>(ctx, n, maxWy); break;
@@ -2594,7 +2594,7 @@ static int launch_tables(aln_ctx *ctx, const std::vector<std::vector<PairPlan *>
         return ALN_OK;
     if (sp.packed) {
         smem_attr(ctx->device, (const void *)k3_satp, satp_smem());
-        LAUNCH_DEP(ctx, "k3_sat", k3_satp, dim3((sp.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
+        LAUNCH_DEP(ctx, "k3_satp", k3_satp, dim3((sp.maxw + 63) / 64, 2 * n), dim3(32, SAT_WARPS),
                    satp_smem(), ctx->dpairs);
     }
     // k3_sat reads its images by __ldg, so it starts after a transpose's end
