@@ -2371,8 +2371,8 @@ static void launch_lagimg2(aln_ctx *ctx, int n, int maxWy, bool both, bool sonly
 // register-FFT pipeline for one chunk: rows (both images), fused columns,
 // lag rows.  L = Nx/2 in [16, 4096], Ny in [16, 8192].
 static int launch_fft_pipeline(aln_ctx *ctx, int L, int Ny, int n, int maxh, int maxWx,
-                               int maxWy, int mode = JOB_PATCHES, bool both = false, bool sonly = false,
-                               bool seg = false, bool cached = false)
+                               int maxWy, int mode = JOB_PATCHES, bool both = false,
+                               bool sonly = false, bool seg = false, bool cached = false)
 {
     switch (L) {
 #define X(v) case v: launch_rowfft2<v>(ctx, n, maxh); break;
@@ -2988,11 +2988,11 @@ static int batch_impl(aln_ctx *ctx, int npairs, const aln_pair *pairs, const Img
     // part of its time only (3000 uneven pairs: 74 chunks in 9 spans, 629 -> 323
     // launches, 18.4 -> 16.0 ms).
     // A quarter, and a chunk's 4096 jobs, so that the host prepares the next span
-    // while this one runs (16000 pairs of 16^2 on one grid: 4.2 ms in spans of a
+    // while this one runs (16000 pairs of 16^2 on one grid: 3.9 ms in spans of a
     // chunk, 5.2 in one).  Its launches are sized for the largest job, and a
     // block that finds nothing to do costs 1-2 ns, a chunk's own launches about
     // 20 us: a chunk joins where it adds at most SPAN_PAD such blocks (those 16000
-    // pairs and one of 2000^2: 13.2 ms without this rule, 4.0 apart; 200 pairs of
+    // pairs and one of 2000^2: 13.2 ms without this rule, 3.9 apart; 200 pairs of
     // 100 x 90 and a strip of 235 x 2048: 205 us in one span, 223 apart).
     constexpr long long SPAN_PAD = 16384;
     std::vector<std::vector<std::vector<std::vector<PairPlan *>>>> wspans(windows.size());

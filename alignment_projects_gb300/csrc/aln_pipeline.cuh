@@ -1545,8 +1545,8 @@ __global__ void __launch_bounds__(32 * LAGSCAN_ROWS) k2_lagscan(PairDev *pairs)
     const int y = p.ylo + j, ox = p.ox;
     const long long dy = y - p.oy, in = p.rsqr - dy * dy;   // disc: dx^2 <= in
     // the row's span of the disc, a little wide; the lag's own test is exact
-    // (an FP64 square root per row cost more than the test).  From 2^15 px on,
-    // where FP32 is a pixel off and the centre may be far, the whole row
+    // (an FP64 square root per row cost more than the test).  Where the span
+    // reaches 2^15 px to each side, the whole row: the centre may be far off
     int xa = p.xlo, xb = in < 0 ? xa - 1 : p.xhi;
     if (in >= 0 && in < 1ll << 30) {
         const int xr = (int)sqrtf(__int2float_rn((int)in)) + 2;

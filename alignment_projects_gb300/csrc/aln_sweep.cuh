@@ -1346,13 +1346,13 @@ __device__ __forceinline__ double sum_join(long long X, int e)
 }
 
 // The first n of V, or their squares, added one after another (an absent bin
-// holds +0.0, which leaves any sum as it is).
-__device__ __forceinline__ double sum_in_order(const double *__restrict__ V, int n, bool sq)
+// holds +0.0, which leaves any sum as it is).  Plain loads: k_normalize writes V.
+__device__ __forceinline__ double sum_in_order(const double *V, int n, bool sq)
 {
     double x = 0.0;
 #pragma unroll 16
     for (int k = 0; k < n; ++k) {
-        const double v = __ldg(V + k);
+        const double v = V[k];
         x = __dadd_rn(x, sq ? __dmul_rn(v, v) : v);
     }
     return x;
