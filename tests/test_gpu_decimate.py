@@ -87,3 +87,18 @@ def test_small_thumbnails(ctx, orc, kind, h, w, lbin, n):
         assert np.array_equal(vals[ys, xs], v, equal_nan=True)
         assert np.array_equal(vals, vals2, equal_nan=True) and np.array_equal(pres, pres2)
         assert sd == sd2
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("at", [3, 5000])   # among the first bins, in a later chunk
+def test_sums_of_infinities(ctx, orc, value, at):
+    h, w = 90, 101
+    img = np.random.default_rng(at).random(h * w).astype(np.float32)
+    img[at] = value
+    img = img.reshape(h, w)
+    yy, xx = np.mgrid[0:h, 0:w]
+    pts = np.stack([xx.ravel(), yy.ravel()], 1).astype(np.float64)
+    with np.errstate(all="ignore"):
+        _, v = orc.decimate_normalize(pts, img.ravel().astype(np.float64), w, h, 1)
+    vals, pres, _ = ctx.decimate([img], 1)[0]
+    assert pres.all() and np.array_equal(vals.ravel(), v, equal_nan=True)

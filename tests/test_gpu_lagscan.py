@@ -151,11 +151,11 @@ def test_corr_images_r_bound(ctx, orc, data, rule):
     check(g, o, 1, (data, rule))
 
 
-@pytest.mark.parametrize("kinds", ["u8 u8", "u16 u16", "u8 u16"])
+@pytest.mark.parametrize("kinds", ["u8 u8", "u16 u16", "u8 u16", "f32 f32", "f64 f64", "u8 f32"])
 @pytest.mark.parametrize("away,sd", [(60, 0.4), (100, 0.5), (120, 0.8)])
 def test_corr_images_r_flat_overlaps(ctx, kinds, away, sd):
-    """Integer images whose searched overlaps are nearly flat and far from the
-    image's mean, where FP32 gives R to 1e-3 only: the scan's peak is the largest
+    """Images whose searched overlaps are nearly flat and far from the image's
+    mean, where FP32 gives R to 1e-3 only: the scan's peak is the largest
     of the values that the same call gives lag by lag (a box rule that one lag of
     the oval meets; the correlation is the same numbers), alone and in a batch."""
     import alignment_projects_gb300 as aln
@@ -171,8 +171,8 @@ def test_corr_images_r_flat_overlaps(ctx, kinds, away, sd):
             v = np.full((h, w), 128.0 + away)
             v[:, dark:dark + w // 2] -= 2 * away
             v = np.rint((v + sd * rng.standard_normal((h, w))) * scale)
-            job[name] = _view(np.clip(v, 0, 255 * scale)
-                              .astype(np.uint8 if dt == "u8" else np.uint16), 0, w)
+            job[name] = _view(np.clip(v, 0, 255 * scale).astype(
+                dict(u8=np.uint8, u16=np.uint16, f32=np.float32, f64=np.float64)[dt]), 0, w)
         job.update(kind=aln.CORR_R, ox=cx, oy=0, rx=rx, ry=ry,
                    legal=aln.legal(aln.RGN_MIN, 8, 8, 0))
         each = ctx.corr_images_batch([
@@ -271,3 +271,23 @@ def test_long_scans_alone_and_batched(ctx, dtype, images):
     alone = call([job])
     for n in (3, 9):
         assert call([job] * n) == alone * n
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_images_with_infinities(ctx, orc, dtype, value):
+    """A pixel that is no number spoils every lag: R is 0 at all of them, as the
+    oracle has it, and S and CorrPatches find no peak."""
+    import oracle as O
+    from test_gpu_images import aln_legal, check
+    a, b = (t.astype(dtype) for t in _pair(np.random.default_rng(4), 50, 41))
+    a[20, 30] = value
+    lg = O.legal(O.RGN_MIN, 10, 10, 0)
+    pa, pb = (O.image_to_points(t) for t in (a, b))
+    with np.errstate(all="ignore"):
+        o = orc.corr_images(1, *pa, *pb, lg)
+    job = dict(a=a, b=b, legal=aln_legal(lg))
+    for g in ctx.corr_images_batch([dict(job, kind=1)] * 3):
+        check(g, o, 1, (dtype, value))
+    none = ctx.corr_images_batch([dict(job, kind=2)]) + ctx.corr_patches_batch([job])
+    assert all(g["status"] == 1 and g["r"] == 0 for g in none)
